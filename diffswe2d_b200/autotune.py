@@ -47,9 +47,13 @@ def _cache_file() -> Path:
     return Path(base) / "diffswe2d_b200" / "autotune.json"
 
 
+#: generation of the step kernels: choices timed with other kernels are not used
+KERNELS = 2
+
+
 def _device_key(device) -> str:
     props = torch.cuda.get_device_properties(torch.device(device))
-    return f"{props.name}/{props.multi_processor_count}"
+    return f"{props.name}/{props.multi_processor_count}/{KERNELS}"
 
 
 def _load(device) -> dict:

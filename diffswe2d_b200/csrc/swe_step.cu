@@ -14,11 +14,14 @@
 // The global reduction between the two stages is why the step is two
 // launches: dt depends on every face of the grid.
 //
-// Each block owns a TX x TY tile.  It stages the tile and a two-cell halo
-// (ghost cells of add_ghost_cells, src/boundary.py:150-413, evaluated on the
-// fly at the domain edge) in shared memory as per-cell primitives, then
-// computes per-cell face-side values in both directions, then the HLL face
-// fluxes, then each cell's tendency.  All arithmetic is FP32 on the CUDA
+// Two forms of the IEEE stages give the same bits.  In the tile form
+// (stage_kernel, small and medium grids) each block owns a TX x TY tile: it
+// stages the tile and a two-cell halo (ghost cells of add_ghost_cells,
+// src/boundary.py:150-413, evaluated on the fly at the domain edge) in
+// shared memory as per-cell primitives, then computes per-cell face-side
+// values in both directions, then the HLL face fluxes, then each cell's
+// tendency.  In the sweep form (sweep_kernel, large grids and ensembles)
+// each warp walks down a strip of columns.  All arithmetic is FP32 on the CUDA
 // cores (swe_math.cuh) in the reference's operation order.
 #include <cuda_runtime.h>
 
@@ -129,6 +132,7 @@ __global__ void __launch_bounds__(NT) stage_kernel(const StepArgs a) {
     __shared__ Side s_yp[TY + 2][TX], s_ym[TY + 2][TX];
     __shared__ FaceFlux s_fx[TY][TX + 1], s_fy[TY + 1][TX];
 
+    chain_start();
     const SweConsts& kc = a.kc;
     const int tid = threadIdx.x;
     const int b = blockIdx.z;
@@ -256,6 +260,11 @@ __global__ void __launch_bounds__(NT) stage_kernel(const StepArgs a) {
         a.tend[o + plane] = r.r1;
         a.tend[o + 2 * plane] = r.r2;
     } else {
+        if (a.k2_out != nullptr) {
+            a.k2_out[o] = r.r0;
+            a.k2_out[o + plane] = r.r1;
+            a.k2_out[o + 2 * plane] = r.r2;
+        }
         const State u{a.U[o], a.U[o + plane], a.U[o + 2 * plane]};
         const State c{u.h + dt * r.r0, u.hu + dt * r.r1, u.hv + dt * r.r2};
         State upd = clean_and_limit(u, c, kc, a.positivity != 0);
@@ -485,6 +494,32 @@ __global__ void ensemble_init_kernel(EnsCtl* ctl, int count, EnsGlobal* g) {
 // swe_tune_sweep_rows; the ensemble carries one value per scenario).
 int g_sweep_rows = SW_ROWS;
 
+// Tile height of a launch while the knob is at its default.  A warp walks
+// r + 4 rows one after another, so a stage takes about
+// (r + 4) (1 + W(r) / 2500) row times, W(r) the launch's warps: the first
+// term is one warp's chain (a small grid: short tiles), the second the
+// chip's rate once warps queue (a large grid: the 4 halo rows want tall
+// tiles).  Against the best of twelve heights, measured from 40 x 40 to
+// 4096 x 4096 in both arithmetics, the height this picks is within 6 %; 64
+// rows everywhere took 467 us a step at 64 x 96 (29 us at one row), 516 at
+// 244 x 393 (45 at 1) and 789 at 4096^2 in the tolerance mode (754 at 32).
+int sweep_rows_for(int B, int ny, int nx) {
+    if (g_sweep_rows != SW_ROWS) return g_sweep_rows;
+    const double strips = (double)((nx + SW_OUT - 1) / SW_OUT) * B;
+    int best = SW_ROWS;
+    double best_cost = INFINITY;
+    for (int r : {1, 2, 3, 4, 6, 8, 12, 16, 24, 32, SW_ROWS}) {
+        const int tiles = (ny + r - 1) / r;
+        if (tiles > 65535) continue;  // grid.y
+        const double cost = (r + 4) * (1.0 + strips * tiles / 2500.0);
+        if (cost < best_cost) {
+            best_cost = cost;
+            best = r;
+        }
+    }
+    return best;
+}
+
 bool fill_common(StepArgs& a, const float* U, const float* bed, int B, int bedB, int ny, int nx,
                  const swe_params* p, const float* level, int levelB) {
     if (!U || !bed || !level || !valid_params(p)) return false;
@@ -512,7 +547,7 @@ bool fill_common(StepArgs& a, const float* U, const float* bed, int B, int bedB,
     a.friction = p->apply_friction;
     a.friction_model = p->friction_model;
     a.kc = make_consts(*p);
-    a.rows = g_sweep_rows;
+    a.rows = sweep_rows_for(B, ny, nx);
     return true;
 }
 
@@ -531,14 +566,22 @@ dim3 sweep_grid_of(const StepArgs& a) {
     return dim3((strips + SW_WARPS - 1) / SW_WARPS, (a.ny + a.rows - 1) / a.rows, a.B);
 }
 
-// Kernel form of the two stages: the row sweep (default) or the
-// shared-memory tile form (SWE_STEP_KERNEL=tiled), read once per process.
-bool use_tiled_kernels() {
-    static const bool tiled = [] {
+// Kernel form of the IEEE stages.  The shared-memory tile evaluates a cell
+// per thread (no serial chain, fewer halo cells than short sweep tiles) and
+// is the faster form up to about 1.5 million cells; above that the row sweep
+// with tall tiles is (a step, tile / best sweep: 244 x 393 36 / 45 us,
+// 4 x 244 x 393 78 / 97, 1021 x 1019 168 / 189, 1200^2 221 / 235, 2048^2
+// 605 / 570, 4096^2 2341 / 1968).  SWE_STEP_KERNEL=tiled or =sweep fixes the
+// form, read once per process.  Both give the same bits.
+constexpr long long kTiledMaxCells = 3ll << 19;
+
+bool use_tiled_kernels(const StepArgs& a) {
+    static const int form = [] {
         const char* v = getenv("SWE_STEP_KERNEL");
-        return v != nullptr && strcmp(v, "tiled") == 0;
+        return v == nullptr ? 0 : strcmp(v, "tiled") == 0 ? 1 : strcmp(v, "sweep") == 0 ? 2 : 0;
     }();
-    return tiled;
+    if (form != 0) return form == 1;
+    return (long long)a.B * a.ny * a.nx <= kTiledMaxCells;
 }
 
 }  // namespace
@@ -567,10 +610,10 @@ extern "C" int swe_spatial_operator_f32(const float* U, const float* bed, int B,
     if (cudaMemsetAsync(red, 0, SWE_RED_WORDS * sizeof(uint32_t), s) != cudaSuccess) return SWE_ECUDA;
     // the stage-1 kernel of the step computes exactly this (tendency + maxima)
     if (p->arithmetic == SWE_ARITH_FAST) return fast_launch_stages(1, a, sweep_grid_of(a), s);
-    if (use_tiled_kernels()) stage_kernel<1><<<grid_of(a), NT, 0, s>>>(a);
-    else if (launch_chained(sweep_kernel<1, 0>, sweep_grid_of(a), dim3(SW_WARPS * 32), s, a) != cudaSuccess)
-        return SWE_ECUDA;
-    return cudaGetLastError() == cudaSuccess ? SWE_OK : SWE_ECUDA;
+    const cudaError_t e =
+        use_tiled_kernels(a) ? launch_chained(stage_kernel<1>, grid_of(a), dim3(NT), s, a)
+                             : launch_chained(sweep_kernel<1, 0>, sweep_grid_of(a), dim3(SW_WARPS * 32), s, a);
+    return e == cudaSuccess && cudaGetLastError() == cudaSuccess ? SWE_OK : SWE_ECUDA;
 }
 
 namespace swe {
@@ -605,8 +648,7 @@ int launch_step(int stage, const float* U, const float* bed, int bedB, const flo
     a.k2_out = k2_out;
     cudaStream_t s = (cudaStream_t)stream;
     const bool fast = p->arithmetic == SWE_ARITH_FAST;
-    const bool tiled = !fast && use_tiled_kernels();
-    if (k2_out && tiled) return SWE_EARG;  // the tiled IEEE kernels do not write k2
+    const bool tiled = !fast && use_tiled_kernels(a);
     const dim3 g = tiled ? grid_of(a) : sweep_grid_of(a);
     // A clocked step's reduction words are cleared by swe_clock_f32.
     if ((stage & 1) && !clk && cudaMemsetAsync(red, 0, SWE_RED_WORDS * sizeof(uint32_t), s) != cudaSuccess)
@@ -615,12 +657,12 @@ int launch_step(int stage, const float* U, const float* bed, int bedB, const flo
     const dim3 th(SW_WARPS * 32);
     cudaError_t e = cudaSuccess;
     if (stage & 1) {
-        if (tiled) stage_kernel<1><<<g, NT, 0, s>>>(a);
+        if (tiled) e = launch_chained(stage_kernel<1>, g, dim3(NT), s, a);
         else e = launch_chained(sweep_kernel<1, 0>, g, th, s, a);
     }
     if ((stage & 2) && e == cudaSuccess) {
         if (tiled) {
-            stage_kernel<2><<<g, NT, 0, s>>>(a);
+            e = launch_chained(stage_kernel<2>, g, dim3(NT), s, a);
         } else if (!a.friction) {
             e = launch_chained(sweep_kernel<2, 0>, g, th, s, a);
         } else if (a.friction_model == 0) {

@@ -290,7 +290,6 @@ int swe_step_clocked_f32(int stage, const float* U, const float* bed, int bedB, 
  * k2 = rhs(P) at the predictor P (solver.py:641) into k2_out [B,3,ny,nx],
  * as the step computes it, for an adjoint pass that then need not
  * re-evaluate it.  Steps the clock marks inactive leave k2_out untouched.
- * SWE_EARG with the tiled IEEE kernels (SWE_STEP_KERNEL=tiled).
  */
 int swe_step_clocked_k2_f32(int stage, const float* U, const float* bed, int bedB, const float* n,
                             int nB, int B, int ny, int nx, const swe_params* p, const float* level,
@@ -463,7 +462,8 @@ int swe_ensemble_results_f32(const void* workspace, int count, swe_ensemble_resu
 int swe_load_kernels(void);
 
 /* Output rows per tile of the single-grid sweep kernels (process-wide
- * tuning knob, default 64; set it between launches, not during them). */
+ * tuning knob; set it between launches, not during them).  At its default,
+ * 64, each launch takes the height that suits its grid, at most 64. */
 int swe_tune_sweep_rows(int rows);
 
 /* The current value of that knob (CUDA graphs keep the value they were
