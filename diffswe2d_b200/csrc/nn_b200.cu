@@ -1,18 +1,18 @@
 // nn_b200.cu -- training and inference kernels of the warm-start network.
 //
 // The matrix products run on the 5th-generation tensor cores: one CTA of
-// 128 threads computes a 128 x BN tile of A B^T (bf16 operands, fp32
-// accumulator in tensor memory).  Operands are staged global -> shared
-// memory by all threads in the canonical no-swizzle K-major layout that
-// tcgen05.mma reads through shared-memory matrix descriptors, two stages
-// deep; one elected thread issues the MMAs and commits them to an mbarrier
-// per stage; the epilogue reads the accumulator with tcgen05.ld (each warp
-// its 32 lanes) and applies bias and activation.  Every mbarrier wait is
-// bounded in time: a wait inside the K loop gives up after the launch's
-// limit (wait_ns), after which the CTA records error bit 1, stops issuing,
-// waits for its issued MMAs to drain (a fixed, separate bound of 2 s),
-// frees its tensor memory and returns.  If the drain bound also runs out,
-// the CTA still frees its tensor memory (every allocation must be freed
+// nine warps computes a 128 x bn tile of A B^T (bf16 operands, fp32
+// accumulator in tensor memory).  Eight warps stage the operands global ->
+// shared memory by cp.async in the 128-byte-swizzled K-major layout that
+// tcgen05.mma reads through shared-memory matrix descriptors, up to eight
+// stages deep; one thread of the ninth issues the MMAs and commits them to
+// the stage's mbarrier; the epilogue reads the accumulator with tcgen05.ld
+// (each warp its 32 lanes) and applies bias and activation.  Every mbarrier
+// wait is bounded in time: a wait inside the K loop gives up after the
+// launch's limit (wait_ns), after which the CTA records error bit 1, stops
+// issuing, waits for its issued MMAs to drain (a fixed, separate bound of
+// 2 s), frees its tensor memory and returns.  If the drain bound also runs
+// out, the CTA still frees its tensor memory (every allocation must be freed
 // before the CTA exits) and records error bit 2: MMAs may then have been
 // running when it was freed, and the context should not be trusted.
 //
@@ -30,23 +30,30 @@ namespace {
 
 constexpr int BM = 128;       // tile rows (UMMA M)
 constexpr int BK = 64;        // K elements per stage
-constexpr int BN_MAX = 128;   // tile columns (UMMA N), multiple of 16
-constexpr int NT = 128;       // threads per CTA
-constexpr int A_BYTES = BM * BK * 2;      // 16 KB
-constexpr int B_BYTES = BN_MAX * BK * 2;  // 16 KB
-constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
-// Two stages use 64 KB; the allocation is 96 KB so that the operand reads
-// of every descriptor stay inside it by a wide margin.
-constexpr int SMEM_BYTES = 96 * 1024;
+constexpr int BN_MAX = 128;   // tile columns (UMMA N): 16, 32, 64 or 128
+constexpr int LOADERS = 8;    // warps that stage operands
+constexpr int NT = 32 * (LOADERS + 1);
+constexpr int STAGES_MAX = 8;
+// A K-major operand tile: one 128-byte row (64 bf16) per matrix row, its
+// sixteen-byte chunk c stored at position c ^ (row & 7) (the 128-byte
+// swizzle; the tile starts on a 1,024-byte boundary).
+__host__ __device__ constexpr int tile_bytes(int rows) { return rows * BK * 2; }
 // Bound of the final wait for the CTA's own MMAs before its tensor memory is
 // freed (independent of the launch's wait limit, so that a short limit
 // never frees tensor memory under MMAs that are still running).
 constexpr unsigned long long DRAIN_LIMIT_NS = 2000000000ull;  // 2 s
 
+// Dynamic shared memory of a launch: up to eight stages of the narrower
+// tiles, four of the widest.
+constexpr int SMEM_ALIGN = 1024;
+constexpr int SMEM_MAX = STAGES_MAX * (tile_bytes(BM) + tile_bytes(64));
+static_assert(SMEM_MAX + SMEM_ALIGN + 1024 <= 227 * 1024 && 4 * (tile_bytes(BM) + tile_bytes(BN_MAX)) <= SMEM_MAX, "");
+
 struct GemmArgs {
     const uint16_t* A;
     const uint16_t* B;
     int M, N, K, lda, ldb, kchunk;  // kchunk: K per blockIdx.z (multiple of BK)
+    int bn, stages;                 // tile columns, pipeline stages
     const float* bias;
     int act, ldc;
     float* out_f32;
@@ -67,12 +74,13 @@ __device__ __forceinline__ unsigned long long global_ns() {
     return t;
 }
 
-// Shared-memory matrix descriptor, no swizzle, K-major: 8-row x 16-byte core
-// matrices; lbo = byte distance between the two core matrices along K of
-// one MMA, sbo = byte distance between 8-row groups; version 1 (bits 46-47).
-__device__ __forceinline__ uint64_t smem_desc(uint32_t addr, uint32_t lbo, uint32_t sbo) {
-    return (uint64_t)((addr >> 4) & 0x3FFFu) | ((uint64_t)((lbo >> 4) & 0x3FFFu) << 16) |
-           ((uint64_t)((sbo >> 4) & 0x3FFFu) << 32) | (1ull << 46);
+// Shared-memory matrix descriptor of a K-major tile in the 128-byte swizzle:
+// 1,024 bytes between 8-row groups (bits 32-45; the leading offset, bits
+// 16-29, is not used by this layout), version 1 (bits 46-47), layout 2
+// (bits 61-63).  A K step of 16 elements is 32 bytes further on.
+__device__ __forceinline__ uint64_t smem_desc(uint32_t addr) {
+    return (uint64_t)((addr >> 4) & 0x3FFFu) | (1ull << 16) | ((uint64_t)(1024 >> 4) << 32) | (1ull << 46) |
+           (2ull << 61);
 }
 
 // Instruction descriptor of kind::f16: fp32 accumulator (bits 4-5 = 1),
@@ -83,8 +91,12 @@ __device__ __forceinline__ uint32_t instr_desc(int n) {
            ((uint32_t)(BM >> 4) << 24);
 }
 
-__device__ __forceinline__ void mbar_init(uint32_t bar) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar));
+__device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count));
+}
+
+__device__ __forceinline__ void mbar_arrive(uint32_t bar) {
+    asm volatile("{\n\t.reg .b64 t;\n\tmbarrier.arrive.shared::cta.b64 t, [%0];\n\t}" ::"r"(bar) : "memory");
 }
 
 __device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity) {
@@ -100,14 +112,33 @@ __device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity) {
 }
 
 // Wait for the phase `parity` of an mbarrier, giving up once `limit`
-// nanoseconds have passed (the time is checked before every probe, so a
-// limit of 0 gives up at once).
-__device__ bool mbar_wait(uint32_t bar, uint32_t parity, unsigned long long limit) {
+// nanoseconds have passed (a limit of 0 gives up at once).  The clock is
+// read only after a first run of probes: a read of globaltimer costs more
+// than a K block (0.9 us a block with the clock read before every probe).
+__device__ __noinline__ bool mbar_wait_slow(uint32_t bar, uint32_t parity, unsigned long long limit) {
+    for (int i = 0; i < 256; ++i)
+        if (mbar_try(bar, parity)) return true;
     const unsigned long long t0 = global_ns();
     while (global_ns() - t0 < limit) {
         if (mbar_try(bar, parity)) return true;
     }
     return false;
+}
+
+__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, unsigned long long limit) {
+    if (limit == 0) return false;
+    return mbar_try(bar, parity) || mbar_wait_slow(bar, parity, limit);
+}
+
+// One lane of a converged warp.
+__device__ __forceinline__ bool elect_one() {
+    uint32_t p;
+    asm volatile(
+        "{\n\t.reg .pred q;\n\t"
+        "elect.sync _|q, 0xffffffff;\n\t"
+        "selp.u32 %0, 1, 0, q;\n\t}"
+        : "=r"(p));
+    return p != 0;
 }
 
 __device__ __forceinline__ void mma_bf16(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc,
@@ -124,15 +155,24 @@ __device__ __forceinline__ void mma_commit(uint32_t bar) {
                  ::"r"(bar) : "memory");
 }
 
-__device__ __forceinline__ void tmem_ld8(uint32_t taddr, float (&v)[8]) {
-    uint32_t r[8];
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]),
-                   "=r"(r[6]), "=r"(r[7])
-                 : "r"(taddr));
+__device__ __forceinline__ void tmem_ld16(uint32_t taddr, float (&v)[16]) {
+    uint32_t r[16];
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, "
+        "[%16];"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
+          "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]),
+          "=r"(r[14]), "=r"(r[15])
+        : "r"(taddr));
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-    for (int i = 0; i < 8; ++i) v[i] = __uint_as_float(r[i]);
+    for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
+}
+
+// 16 bytes global -> shared, zero-filled where !ok (src is then not read).
+__device__ __forceinline__ void cp16(uint32_t dst, const uint16_t* src, bool ok) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(ok ? 16 : 0)
+                 : "memory");
 }
 
 __device__ __forceinline__ float gelu(float x) {
@@ -155,97 +195,185 @@ __device__ __forceinline__ void epilogue_store(const GemmArgs& g, int r, int c, 
     if (g.out_bf16) g.out_bf16[o] = __bfloat16_as_ushort(__float2bfloat16_rn(y));
 }
 
+// Whether four values at o, o + 1, ... of p can be written by one 16-byte
+// store (o a multiple of 4 with ldc, checked here with the base's alignment).
+__device__ __forceinline__ bool vec4_ok(const void* p, int ldc, int bytes) {
+    return (((uintptr_t)p & (uintptr_t)(4 * bytes - 1)) | (uintptr_t)(ldc & 3)) == 0;
+}
+
+// 16 consecutive accumulators of row r from column c on.
+__device__ __forceinline__ void epilogue16(const GemmArgs& g, int r, int c, const float (&v)[16], bool vec) {
+    if (g.partial) {
+        float* p = g.partial + ((size_t)blockIdx.z * g.M + r) * g.N + c;
+        if (vec && c + 16 <= g.N) {
+#pragma unroll
+            for (int i = 0; i < 16; i += 4)
+                *reinterpret_cast<float4*>(p + i) = make_float4(v[i], v[i + 1], v[i + 2], v[i + 3]);
+        } else {
+#pragma unroll
+            for (int i = 0; i < 16; ++i)
+                if (c + i < g.N) p[i] = v[i];
+        }
+        return;
+    }
+    if (!vec || c + 16 > g.N) {
+#pragma unroll
+        for (int i = 0; i < 16; ++i)
+            if (c + i < g.N) epilogue_store(g, r, c + i, v[i]);
+        return;
+    }
+    const size_t o = (size_t)r * g.ldc + c;
+#pragma unroll
+    for (int i = 0; i < 16; i += 4) {
+        float pre[4], y[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            pre[e] = v[i + e] + (g.bias ? g.bias[c + i + e] : 0.0f);
+            y[e] = g.act == NN_ACT_GELU ? gelu(pre[e]) : pre[e];
+        }
+        if (g.pre_f32) *reinterpret_cast<float4*>(g.pre_f32 + o + i) = make_float4(pre[0], pre[1], pre[2], pre[3]);
+        if (g.out_f32) *reinterpret_cast<float4*>(g.out_f32 + o + i) = make_float4(y[0], y[1], y[2], y[3]);
+        if (g.out_bf16) {
+            ushort4 b;
+            b.x = __bfloat16_as_ushort(__float2bfloat16_rn(y[0]));
+            b.y = __bfloat16_as_ushort(__float2bfloat16_rn(y[1]));
+            b.z = __bfloat16_as_ushort(__float2bfloat16_rn(y[2]));
+            b.w = __bfloat16_as_ushort(__float2bfloat16_rn(y[3]));
+            *reinterpret_cast<ushort4*>(g.out_bf16 + o + i) = b;
+        }
+    }
+}
+
+// Stage columns [k0, k0 + BK) of `rows` rows from row0 on (rows at or past
+// `limit` and columns at or past kend read as zero), the share of part `part`
+// of `parts` warps: eight lanes per row, one 16-byte chunk each.  A row stays
+// within 128 bytes of shared memory: with the chunks of a row spread over the
+// tile (the unswizzled layout) each 32-byte sector that arrives is split
+// (17,920 x 64 x 384: 22.5 us against 16.5 at otherwise the same code).
+__device__ __forceinline__ void stage_tile(uint32_t smem, const uint16_t* base, int ld, int row0, int limit,
+                                           int rows, int k0, int kend, int part, int parts) {
+    const int lane = threadIdx.x & 31, kc = lane & 7;
+    const int k = k0 + kc * 8;
+    const bool kin = k < kend;
+    const int r0 = part * 4 + (lane >> 3);
+    const uint16_t* src = base + (size_t)(row0 + r0) * ld + k;
+    const size_t step = (size_t)(4 * parts) * ld;
+    const int left = limit - row0;
+#pragma unroll 4
+    for (int r = r0; r < rows; r += 4 * parts, src += step) {
+        const bool ok = kin && r < left;
+        cp16(smem + r * 128 + ((kc ^ (r & 7)) << 4), ok ? src : base, ok);
+    }
+}
+
+// The network's products are small (a CTA walks up to 70 K blocks of 18 to
+// 33 KB), so what bounds this kernel is how many blocks' loads are in flight.
+// Each loader warp has a stage of its own (two or more share one where K is
+// short): it copies the stage, waits for the copies, makes them visible to
+// the tensor core and only then goes on, so that the eight stages' latencies
+// overlap without one warp's proxy fence waiting for another's copies.  The
+// tile is narrowed until the grid fills the chip.  The K order of every
+// element's sum does not depend on any of this, so neither do its bits.
+// Measured against 128 threads that load a stage, issue its MMAs and only
+// then load the next: 256 x 96 x 4480 226 -> 20 us, the 17 products of a
+// training step of 256 runs 764 -> 160 us.
 __global__ void __launch_bounds__(NT, 1) gemm_kernel(const GemmArgs g) {
-    extern __shared__ __align__(1024) uint8_t smem[];
-    __shared__ uint64_t s_bar[2];
+    extern __shared__ uint8_t smem[];
+    __shared__ uint64_t s_full[STAGES_MAX], s_free[STAGES_MAX];
     __shared__ uint32_t s_tmem;
-    __shared__ int s_ok;
+    __shared__ volatile int s_ok;
+    __shared__ int s_drained;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int m0 = blockIdx.x * BM;
-    const int bn = min(BN_MAX, ((g.N + 15) / 16) * 16);
-    const int n0 = blockIdx.y * BN_MAX;
+    const int bn = g.bn, S = g.stages;
+    const int n0 = blockIdx.y * bn;
     const int kbeg = blockIdx.z * g.kchunk;
     const int kend = min(g.K, kbeg + g.kchunk);
     const int nkb = kend > kbeg ? (kend - kbeg + BK - 1) / BK : 0;
     uint32_t ncols = 32;
     while ((int)ncols < bn) ncols <<= 1;
 
-    if (warp == 0) {  // tensor memory for the accumulator (one full warp)
+    const int parts = LOADERS / S;  // loader warps per stage (S is a power of two)
+    if (warp == LOADERS) {          // tensor memory for the accumulator (one full warp)
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
                      ::"r"(smem_u32(&s_tmem)), "r"(ncols));
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
     }
     if (tid == 0) {
-        mbar_init(smem_u32(&s_bar[0]));
-        mbar_init(smem_u32(&s_bar[1]));
+        for (int i = 0; i < S; ++i) {
+            mbar_init(smem_u32(&s_full[i]), (uint32_t)parts);
+            mbar_init(smem_u32(&s_free[i]), 1u);
+        }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         s_ok = 1;
+        s_drained = 1;
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = s_tmem;
-    const uint32_t idesc = instr_desc(bn);
-    uint32_t phase[2] = {0u, 0u};
-    int issued = 0;  // MMA groups committed
+    const uint32_t base = (smem_u32(smem) + 1023u) & ~1023u;
+    const int stage_bytes = tile_bytes(BM) + tile_bytes(bn);
+    const uint32_t full0 = smem_u32(&s_full[0]), free0 = smem_u32(&s_free[0]);
+    const int log_s = 31 - __clz(S);
 
-    for (int kb = 0; kb < nkb; ++kb) {
-        const int s = kb & 1;
-        uint8_t* sA = smem + s * STAGE_BYTES;
-        uint8_t* sB = sA + A_BYTES;
-        if (kb >= 2) {  // the MMAs that read this stage two blocks ago are done
-            if (tid == 0) {
-                if (!mbar_wait(smem_u32(&s_bar[s]), phase[s], g.wait_ns)) s_ok = 0;
+    // Stage kb % S holds block kb; its loads complete phase kb / S of the
+    // stage's "full" barrier, its MMAs phase kb / S of its "free" barrier.
+    if (warp < LOADERS) {
+        const int st = warp / parts, part = warp - st * parts;
+        const uint32_t sA = base + st * stage_bytes, sB = sA + tile_bytes(BM);
+        const uint32_t full = full0 + 8 * st, freed = free0 + 8 * st;
+        for (int kb = st; kb < nkb; kb += S) {
+            if (kb >= S && !mbar_wait(freed, (uint32_t)(((kb >> log_s) - 1) & 1), g.wait_ns)) {
+                s_ok = 0;
+                break;
             }
-            phase[s] ^= 1u;
-            __syncthreads();
             if (!s_ok) break;
+            const int k0 = kbeg + kb * BK;
+            stage_tile(sA, g.A, g.lda, m0, g.M, BM, k0, kend, part, parts);
+            stage_tile(sB, g.B, g.ldb, n0, g.N, bn, k0, kend, part, parts);
+            asm volatile("cp.async.wait_all;" ::: "memory");
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) mbar_arrive(full);
         }
-        const int k0 = kbeg + kb * BK;
-        // A rows: thread t stages row m0 + t, 8 chunks of 8 K-elements.
-        {
-            const int r = m0 + tid;
-#pragma unroll
-            for (int kc = 0; kc < BK / 8; ++kc) {
-                const int k = k0 + kc * 8;
-                uint4 v = make_uint4(0u, 0u, 0u, 0u);
-                if (r < g.M && k < kend) v = *reinterpret_cast<const uint4*>(g.A + (size_t)r * g.lda + k);
-                *reinterpret_cast<uint4*>(sA + kc * (BM * 16) + tid * 16) = v;
-            }
-        }
-        if (tid < bn) {
-            const int r = n0 + tid;
-#pragma unroll
-            for (int kc = 0; kc < BK / 8; ++kc) {
-                const int k = k0 + kc * 8;
-                uint4 v = make_uint4(0u, 0u, 0u, 0u);
-                if (r < g.N && k < kend) v = *reinterpret_cast<const uint4*>(g.B + (size_t)r * g.ldb + k);
-                *reinterpret_cast<uint4*>(sB + kc * (bn * 16) + tid * 16) = v;
-            }
-        }
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        __syncthreads();
-        if (tid == 0) {
+    } else {
+        // The whole warp walks the K loop (uniform control flow and operands;
+        // one thread in a divergent branch took 1,150 cycles a block, twice
+        // the loads' share) and one elected lane issues.
+        const uint32_t idesc = instr_desc(bn);
+        const uint64_t descA = smem_desc(base), descB = smem_desc(base + tile_bytes(BM));
+        const uint32_t stage_step = (uint32_t)stage_bytes >> 4;  // in descriptor address units
+        const bool issuer = elect_one();
+        const int ktail = (kend - kbeg) - (nkb - 1) * BK;  // columns of the last block
+        bool good = true;
+        int kb = 0;
+        for (; kb < nkb; ++kb) {
+            const int st = kb & (S - 1);
+            // the first two blocks' waits are for loads alone
+            good = mbar_wait(full0 + 8 * st, (uint32_t)((kb >> log_s) & 1), kb < 2 ? DRAIN_LIMIT_NS : g.wait_ns);
+            if (!__all_sync(0xffffffffu, good)) break;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            const uint32_t a0 = smem_u32(sA), b0 = smem_u32(sB);
+            const uint64_t ad = descA + st * stage_step, bd = descB + st * stage_step;
+            if (issuer) {
+                if (kb + 1 < nkb || ktail == BK) {
 #pragma unroll
-            for (int t = 0; t < BK / 16; ++t) {
-                const uint64_t ad = smem_desc(a0 + t * 2 * (BM * 16), BM * 16, 128);
-                const uint64_t bd = smem_desc(b0 + t * 2 * (bn * 16), bn * 16, 128);
-                mma_bf16(tmem, ad, bd, idesc, (kb > 0 || t > 0) ? 1u : 0u);
+                    for (int t = 0; t < BK / 16; ++t)
+                        mma_bf16(tmem, ad + 2 * t, bd + 2 * t, idesc, (kb > 0 || t > 0) ? 1u : 0u);
+                } else {
+                    for (int t = 0; t * 16 < ktail; ++t)
+                        mma_bf16(tmem, ad + 2 * t, bd + 2 * t, idesc, (kb > 0 || t > 0) ? 1u : 0u);
+                }
+                mma_commit(free0 + 8 * st);
             }
-            mma_commit(smem_u32(&s_bar[s]));
+            __syncwarp();
         }
-        issued = kb + 1;
-    }
-
-    // Wait for the last commit (it covers every MMA this thread issued).
-    __shared__ int s_drained;
-    if (tid == 0) s_drained = 1;
-    if (issued > 0) {
-        const int s = (issued - 1) & 1;
-        if (tid == 0) {
-            if (!mbar_wait(smem_u32(&s_bar[s]), phase[s], DRAIN_LIMIT_NS)) s_drained = 0;
+        if (kb < nkb) s_ok = 0;
+        // Wait for the last commit (it covers every MMA issued).
+        if (kb > 0) {
+            const int last = kb - 1;
+            if (!mbar_wait(free0 + 8 * (last & (S - 1)), (uint32_t)((last >> log_s) & 1), DRAIN_LIMIT_NS))
+                s_drained = 0;
         }
     }
     __syncthreads();
@@ -253,31 +381,28 @@ __global__ void __launch_bounds__(NT, 1) gemm_kernel(const GemmArgs g) {
     const bool ok = s_ok != 0 && s_drained != 0;
     if (!ok) {
         if (tid == 0 && g.err) atomicOr(g.err, (s_ok ? 0u : 1u) | (s_drained ? 0u : 2u));
-    } else {
-        const int r = m0 + warp * 32 + lane;
-        const uint32_t lane_addr = tmem + ((uint32_t)(warp * 32) << 16);
-        for (int c0 = 0; c0 < bn; c0 += 8) {
-            float v[8];
-            if (issued > 0) {
-                tmem_ld8(lane_addr + (uint32_t)c0, v);
+    } else if (warp < LOADERS) {
+        // warps w and w + 4 share the rows of TMEM lanes 32 (w % 4) ..
+        const int r = m0 + (warp & 3) * 32 + lane;
+        const uint32_t lane_addr = tmem + ((uint32_t)((warp & 3) * 32) << 16);
+        const bool vec = g.partial ? vec4_ok(g.partial, g.N, 4)
+                                   : vec4_ok(g.out_f32, g.ldc, 4) && vec4_ok(g.pre_f32, g.ldc, 4) &&
+                                         vec4_ok(g.out_bf16, g.ldc, 2);
+        for (int c0 = (warp >> 2) * 16; c0 < bn && n0 + c0 < g.N; c0 += 32) {
+            float v[16];
+            if (nkb > 0) {
+                tmem_ld16(lane_addr + (uint32_t)c0, v);
             } else {
 #pragma unroll
-                for (int i = 0; i < 8; ++i) v[i] = 0.0f;
+                for (int i = 0; i < 16; ++i) v[i] = 0.0f;
             }
-            if (r < g.M) {
-#pragma unroll
-                for (int i = 0; i < 8; ++i) {
-                    const int c = n0 + c0 + i;
-                    if (c >= g.N) continue;
-                    if (g.partial) g.partial[((size_t)blockIdx.z * g.M + r) * g.N + c] = v[i];
-                    else epilogue_store(g, r, c, v[i]);
-                }
-            }
+            if (r < g.M) epilogue16(g, r, n0 + c0, v, vec);
         }
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
-    if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(ncols));
+    if (warp == LOADERS)
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(ncols));
 }
 
 // Split-K: sum the partial tiles in z order, then the epilogue.
@@ -468,7 +593,7 @@ extern "C" int nn_gemm_bf16(const uint16_t* A, int lda, const uint16_t* B, int l
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return SWE_ECUDA;
     if (!g_smem_set[dev]) {
         if (cudaFuncSetAttribute(gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 SMEM_BYTES) != cudaSuccess)
+                                 SMEM_MAX + SMEM_ALIGN) != cudaSuccess)
             return SWE_ECUDA;
         g_smem_set[dev] = true;
     }
@@ -495,8 +620,16 @@ extern "C" int nn_gemm_bf16(const uint16_t* A, int lda, const uint16_t* B, int l
     g.err = err;
     g.wait_ns = (unsigned long long)wait_ns;
     cudaStream_t s = (cudaStream_t)stream;
-    const dim3 grid((M + BM - 1) / BM, (N + BN_MAX - 1) / BN_MAX, zs);
-    gemm_kernel<<<grid, NT, SMEM_BYTES, s>>>(g);
+    // Tile columns: the widest tile (A is read once per column tile) whose
+    // grid still has a CTA for each SM, or the narrowest.
+    int bn = BN_MAX;
+    const long long mz = (long long)((M + BM - 1) / BM) * zs;
+    while (bn > 16 && (bn / 2 >= N || mz * ((N + bn - 1) / bn) < 148)) bn /= 2;
+    g.bn = bn;
+    g.stages = 1;  // a power of two, no more than the K blocks need
+    while (g.stages < per && g.stages < (bn == BN_MAX ? 4 : STAGES_MAX)) g.stages *= 2;
+    const dim3 grid((M + BM - 1) / BM, (N + bn - 1) / bn, zs);
+    gemm_kernel<<<grid, NT, g.stages * (tile_bytes(BM) + tile_bytes(bn)) + SMEM_ALIGN, s>>>(g);
     if (zs > 1) splitk_epilogue_kernel<<<grid_for((long long)M * N, 256), 256, 0, s>>>(g, zs);
     return cudaGetLastError() == cudaSuccess ? SWE_OK : SWE_ECUDA;
 }

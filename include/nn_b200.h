@@ -35,8 +35,8 @@ extern "C" {
  * partial sums go to `workspace` (ksplit * M * N floats) and a second kernel
  * adds them in a fixed order and applies the epilogue.
  * Every wait of a CTA for its tensor-core work inside the K loop gives up
- * after wait_ns nanoseconds (>= 0; the time is checked before each probe,
- * so 0 gives up at once; NN_GEMM_WAIT_NS is the normal limit); the CTA then
+ * after wait_ns nanoseconds (>= 0; counted after a short run of probes; 0
+ * gives up at once; NN_GEMM_WAIT_NS is the normal limit); the CTA then
  * stops, waits up to 2 s for the MMAs it issued, frees its tensor memory and
  * returns without writing its tile.  err (one word, may be NULL) receives
  * bit 1 when a wait gave up and bit 2 when the MMAs had still not completed
