@@ -135,6 +135,25 @@ class SweEnsembleResult(ctypes.Structure):
         ("time", ctypes.c_double),
     ]
 
+
+class NnLayer(ctypes.Structure):
+    """nn_layer of include/nn_b200.h."""
+    _fields_ = [
+        ("conv", ctypes.c_int32),
+        ("cin", ctypes.c_int32),
+        ("cout", ctypes.c_int32),
+        ("k", ctypes.c_int32),
+        ("stride", ctypes.c_int32),
+        ("pad", ctypes.c_int32),
+        ("lin", ctypes.c_int32),
+        ("lout", ctypes.c_int32),
+        ("kpad", ctypes.c_int32),
+        ("reserved", ctypes.c_int32),
+        ("w", ctypes.c_int64),
+        ("b", ctypes.c_int64),
+    ]
+
+
 _P = ctypes.c_void_p
 _I = ctypes.c_int
 _F = ctypes.c_float
@@ -200,6 +219,10 @@ _SIGNATURES = {
     "nn_cast_bf16": [_P, _I, _I, _I, _P, _I, _P, _I, _P],
     "nn_mse": [_P, _P, _I, _I, _P, _P, _P],
     "nn_adam": [_P, _P, _P, _P, ctypes.c_longlong, _F, _F, _F, _F, _I, _P],
+    "nn_adam_bf16": [_P, _P, _P, _P, ctypes.c_longlong, _F, _F, _F, _F, _I, _P, _P],
+    "nn_net_forward": [ctypes.POINTER(NnLayer), _I, _P, _P, _P, _F, _I, _P, _P, ctypes.c_longlong, _P,
+                       _P],
+    "nn_net_backward": [ctypes.POINTER(NnLayer), _I, _P, _P, _I, _P, _P, ctypes.c_longlong, _P, _P],
 }
 
 _lib = None
@@ -220,6 +243,8 @@ def lib() -> ctypes.CDLL:
             fn.restype = ctypes.c_int
         handle.swe_ensemble_workspace_bytes.argtypes = [_I]
         handle.swe_ensemble_workspace_bytes.restype = ctypes.c_longlong
+        handle.nn_net_workspace_bytes.argtypes = [ctypes.POINTER(NnLayer), _I, _I, _I]
+        handle.nn_net_workspace_bytes.restype = ctypes.c_longlong
         _lib = handle
     return _lib
 

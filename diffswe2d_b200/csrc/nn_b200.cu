@@ -22,6 +22,9 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <algorithm>
+#include <atomic>
+
 #include "../../include/nn_b200.h"
 #include "../../include/swe_b200.h"
 
@@ -34,10 +37,12 @@ constexpr int BN_MAX = 128;   // tile columns (UMMA N): 16, 32, 64 or 128
 constexpr int LOADERS = 8;    // warps that stage operands
 constexpr int NT = 32 * (LOADERS + 1);
 constexpr int STAGES_MAX = 8;
-// A K-major operand tile: one 128-byte row (64 bf16) per matrix row, its
-// sixteen-byte chunk c stored at position c ^ (row & 7) (the 128-byte
-// swizzle; the tile starts on a 1,024-byte boundary).
+// Operand tiles are stored in lines of 128 bytes (64 bf16), the sixteen-byte
+// chunk c of line i at position c ^ (i & 7) (the 128-byte swizzle; a tile
+// starts on a 1,024-byte boundary).  K-major: a line per row of the tile, BK
+// elements of K.  MN-major: blocks of 64 rows, each BK lines (one per K).
 __host__ __device__ constexpr int tile_bytes(int rows) { return rows * BK * 2; }
+__host__ __device__ constexpr int mn_tile_bytes(int rows) { return (rows < 64 ? 64 : rows) * BK * 2; }
 // Bound of the final wait for the CTA's own MMAs before its tensor memory is
 // freed (independent of the launch's wait limit, so that a short limit
 // never frees tensor memory under MMAs that are still running).
@@ -49,17 +54,31 @@ constexpr int SMEM_ALIGN = 1024;
 constexpr int SMEM_MAX = STAGES_MAX * (tile_bytes(BM) + tile_bytes(64));
 static_assert(SMEM_MAX + SMEM_ALIGN + 1024 <= 227 * 1024 && 4 * (tile_bytes(BM) + tile_bytes(BN_MAX)) <= SMEM_MAX, "");
 
+// A GEMM operand in memory: lines of `cols` contiguous elements.  K-major: a
+// line is a row of the product's operand (M or N index), its elements run
+// along K.  MN-major: a line is one K index, its elements run along M or N.
+// With lout > 0 the lines are the patches of a 1-D convolution read in place
+// (line n * lout + l is elements [off + l * ld, ...) of sample n, whose
+// `batch` elements are followed by the next sample's; elements outside the
+// sample are zero padding).
+struct Operand {
+    const uint16_t* p;
+    int ld, lines, cols;
+    int lout, batch, off;
+};
+
 struct GemmArgs {
-    const uint16_t* A;
-    const uint16_t* B;
-    int M, N, K, lda, ldb, kchunk;  // kchunk: K per blockIdx.z (multiple of BK)
-    int bn, stages;                 // tile columns, pipeline stages
+    Operand A, B;
+    int M, N, K, kchunk;  // kchunk: K per blockIdx.z (multiple of BK)
+    int bn, stages;       // tile columns, pipeline stages
     const float* bias;
     int act, ldc;
     float* out_f32;
     uint16_t* out_bf16;
     float* pre_f32;
-    float* partial;  // split K: [z][M][N]
+    const float* adj_pre;  // activation adjoint: acc *= gelu'(adj_pre[r, c]) (ldc)
+    float* colpart;        // then: column sums of each row tile [gridDim.x][N]
+    float* partial;        // split K: [z][M][N]
     uint32_t* err;
     unsigned long long wait_ns;  // limit of each wait inside the K loop
 };
@@ -74,21 +93,24 @@ __device__ __forceinline__ unsigned long long global_ns() {
     return t;
 }
 
-// Shared-memory matrix descriptor of a K-major tile in the 128-byte swizzle:
-// 1,024 bytes between 8-row groups (bits 32-45; the leading offset, bits
-// 16-29, is not used by this layout), version 1 (bits 46-47), layout 2
-// (bits 61-63).  A K step of 16 elements is 32 bytes further on.
-__device__ __forceinline__ uint64_t smem_desc(uint32_t addr) {
-    return (uint64_t)((addr >> 4) & 0x3FFFu) | (1ull << 16) | ((uint64_t)(1024 >> 4) << 32) | (1ull << 46) |
-           (2ull << 61);
+// Shared-memory matrix descriptor in the 128-byte swizzle: address, leading
+// offset (bits 16-29: MN-major, bytes between two blocks of 64 rows; not
+// used K-major), stride offset (bits 32-45: 1,024 bytes between groups of
+// eight lines), version 1 (bits 46-47), layout 2 (bits 61-63).  A K step of
+// 16 elements is 32 bytes further on K-major, 16 lines MN-major.
+__device__ __forceinline__ uint64_t smem_desc(uint32_t addr, bool mn) {
+    return (uint64_t)((addr >> 4) & 0x3FFFu) | ((uint64_t)(mn ? (64 * BK * 2) >> 4 : 1) << 16) |
+           ((uint64_t)(1024 >> 4) << 32) | (1ull << 46) | (2ull << 61);
 }
+template <bool MN>
+__host__ __device__ constexpr uint32_t k_step() { return MN ? (16 * 128) >> 4 : 32 >> 4; }
 
 // Instruction descriptor of kind::f16: fp32 accumulator (bits 4-5 = 1),
-// A and B bf16 (bits 7-9, 10-12 = 1), both K-major, N >> 3 at bit 17,
-// M >> 4 at bit 24.
-__device__ __forceinline__ uint32_t instr_desc(int n) {
-    return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) |
-           ((uint32_t)(BM >> 4) << 24);
+// A and B bf16 (bits 7-9, 10-12 = 1), A / B MN-major (bits 15, 16),
+// N >> 3 at bit 17, M >> 4 at bit 24.
+__device__ __forceinline__ uint32_t instr_desc(int n, bool a_mn, bool b_mn) {
+    return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)a_mn << 15) | ((uint32_t)b_mn << 16) |
+           ((uint32_t)(n >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
 }
 
 __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
@@ -201,6 +223,37 @@ __device__ __forceinline__ bool vec4_ok(const void* p, int ldc, int bytes) {
     return (((uintptr_t)p & (uintptr_t)(4 * bytes - 1)) | (uintptr_t)(ldc & 3)) == 0;
 }
 
+// Sums over the warp's lanes of 16 values per lane: lane l returns the sum of
+// value l >> 1 (a fixed order: halves exchanged at distances 16, 8, 4, 2, 1).
+__device__ __forceinline__ float column_sum16(const float (&v)[16]) {
+    const int lane = threadIdx.x & 31;
+    float a[8], b[4], c[2], d;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        const bool up = (lane & 16) != 0;
+        const float keep = up ? v[i + 8] : v[i], give = up ? v[i] : v[i + 8];
+        a[i] = keep + __shfl_xor_sync(0xffffffffu, give, 16);
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const bool up = (lane & 8) != 0;
+        const float keep = up ? a[i + 4] : a[i], give = up ? a[i] : a[i + 4];
+        b[i] = keep + __shfl_xor_sync(0xffffffffu, give, 8);
+    }
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+        const bool up = (lane & 4) != 0;
+        const float keep = up ? b[i + 2] : b[i], give = up ? b[i] : b[i + 2];
+        c[i] = keep + __shfl_xor_sync(0xffffffffu, give, 4);
+    }
+    {
+        const bool up = (lane & 2) != 0;
+        const float keep = up ? c[1] : c[0], give = up ? c[0] : c[1];
+        d = keep + __shfl_xor_sync(0xffffffffu, give, 2);
+    }
+    return d + __shfl_xor_sync(0xffffffffu, d, 1);
+}
+
 // 16 consecutive accumulators of row r from column c on.
 __device__ __forceinline__ void epilogue16(const GemmArgs& g, int r, int c, const float (&v)[16], bool vec) {
     if (g.partial) {
@@ -244,25 +297,42 @@ __device__ __forceinline__ void epilogue16(const GemmArgs& g, int r, int c, cons
     }
 }
 
-// Stage columns [k0, k0 + BK) of `rows` rows from row0 on (rows at or past
-// `limit` and columns at or past kend read as zero), the share of part `part`
-// of `parts` warps: eight lanes per row, one 16-byte chunk each.  A row stays
-// within 128 bytes of shared memory: with the chunks of a row spread over the
-// tile (the unswizzled layout) each 32-byte sector that arrives is split
+// Stage block [k0, k0 + BK) of a tile of `rows` rows from row0 on (what lies
+// outside the operand or at or past kend reads as zero), the share of part
+// `part` of `parts` warps: eight lanes per line, one 16-byte chunk each.  A
+// line stays within 128 bytes of shared memory: with its chunks spread over
+// the tile (the unswizzled layout) each 32-byte sector that arrives is split
 // (17,920 x 64 x 384: 22.5 us against 16.5 at otherwise the same code).
-__device__ __forceinline__ void stage_tile(uint32_t smem, const uint16_t* base, int ld, int row0, int limit,
-                                           int rows, int k0, int kend, int part, int parts) {
-    const int lane = threadIdx.x & 31, kc = lane & 7;
-    const int k = k0 + kc * 8;
-    const bool kin = k < kend;
-    const int r0 = part * 4 + (lane >> 3);
-    const uint16_t* src = base + (size_t)(row0 + r0) * ld + k;
-    const size_t step = (size_t)(4 * parts) * ld;
-    const int left = limit - row0;
+template <bool MN>
+__device__ __forceinline__ void stage_tile(uint32_t smem, const Operand& o, int row0, int rows, int k0,
+                                           int kend, int part, int parts) {
+    const int lane = threadIdx.x & 31, c = lane & 7;
+    const int nlines = MN ? BK : rows;
+    const int line0 = MN ? k0 : row0;
+    const int left = (MN ? min(kend, o.lines) : o.lines) - line0;  // lines that exist
+    const int i0 = part * 4 + (lane >> 3), step = 4 * parts;
+    for (int blk = 0; blk < (MN ? rows : 1); blk += 64) {
+        if (MN && blk + c * 8 >= rows) break;  // never read by the MMA
+        const int col = (MN ? row0 + blk : k0) + c * 8;
+        const bool cin = col < (MN ? o.cols : kend);
+        const uint32_t dst = smem + (MN ? blk * (BK * 2) : 0);
+        if (o.lout == 0) {
+            const uint16_t* src = o.p + (size_t)(line0 + i0) * o.ld + col;
+            const size_t inc = (size_t)step * o.ld;
 #pragma unroll 4
-    for (int r = r0; r < rows; r += 4 * parts, src += step) {
-        const bool ok = kin && r < left;
-        cp16(smem + r * 128 + ((kc ^ (r & 7)) << 4), ok ? src : base, ok);
+            for (int i = i0; i < nlines; i += step, src += inc) {
+                const bool ok = cin && i < left;
+                cp16(dst + i * 128 + ((c ^ (i & 7)) << 4), ok ? src : o.p, ok);
+            }
+        } else {
+            int n = (line0 + i0) / o.lout, l = (line0 + i0) - n * o.lout;
+            for (int i = i0; i < nlines; i += step) {
+                const int e = o.off + l * o.ld + col;
+                const bool ok = cin && i < left && (unsigned)e < (unsigned)o.batch;
+                cp16(dst + i * 128 + ((c ^ (i & 7)) << 4), ok ? o.p + (size_t)n * o.batch + e : o.p, ok);
+                for (l += step; l >= o.lout; l -= o.lout) ++n;
+            }
+        }
     }
 }
 
@@ -277,12 +347,14 @@ __device__ __forceinline__ void stage_tile(uint32_t smem, const uint16_t* base, 
 // Measured against 128 threads that load a stage, issue its MMAs and only
 // then load the next: 256 x 96 x 4480 226 -> 20 us, the 17 products of a
 // training step of 256 runs 764 -> 160 us.
+template <bool A_MN, bool B_MN>
 __global__ void __launch_bounds__(NT, 1) gemm_kernel(const GemmArgs g) {
     extern __shared__ uint8_t smem[];
     __shared__ uint64_t s_full[STAGES_MAX], s_free[STAGES_MAX];
     __shared__ uint32_t s_tmem;
     __shared__ volatile int s_ok;
     __shared__ int s_drained;
+    __shared__ float s_col[4][BN_MAX];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int m0 = blockIdx.x * BM;
     const int bn = g.bn, S = g.stages;
@@ -313,7 +385,7 @@ __global__ void __launch_bounds__(NT, 1) gemm_kernel(const GemmArgs g) {
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = s_tmem;
     const uint32_t base = (smem_u32(smem) + 1023u) & ~1023u;
-    const int stage_bytes = tile_bytes(BM) + tile_bytes(bn);
+    const int stage_bytes = tile_bytes(BM) + (B_MN ? mn_tile_bytes(bn) : tile_bytes(bn));
     const uint32_t full0 = smem_u32(&s_full[0]), free0 = smem_u32(&s_free[0]);
     const int log_s = 31 - __clz(S);
 
@@ -330,8 +402,8 @@ __global__ void __launch_bounds__(NT, 1) gemm_kernel(const GemmArgs g) {
             }
             if (!s_ok) break;
             const int k0 = kbeg + kb * BK;
-            stage_tile(sA, g.A, g.lda, m0, g.M, BM, k0, kend, part, parts);
-            stage_tile(sB, g.B, g.ldb, n0, g.N, bn, k0, kend, part, parts);
+            stage_tile<A_MN>(sA, g.A, m0, BM, k0, kend, part, parts);
+            stage_tile<B_MN>(sB, g.B, n0, bn, k0, kend, part, parts);
             asm volatile("cp.async.wait_all;" ::: "memory");
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             __syncwarp();
@@ -341,8 +413,8 @@ __global__ void __launch_bounds__(NT, 1) gemm_kernel(const GemmArgs g) {
         // The whole warp walks the K loop (uniform control flow and operands;
         // one thread in a divergent branch took 1,150 cycles a block, twice
         // the loads' share) and one elected lane issues.
-        const uint32_t idesc = instr_desc(bn);
-        const uint64_t descA = smem_desc(base), descB = smem_desc(base + tile_bytes(BM));
+        const uint32_t idesc = instr_desc(bn, A_MN, B_MN);
+        const uint64_t descA = smem_desc(base, A_MN), descB = smem_desc(base + tile_bytes(BM), B_MN);
         const uint32_t stage_step = (uint32_t)stage_bytes >> 4;  // in descriptor address units
         const bool issuer = elect_one();
         const int ktail = (kend - kbeg) - (nkb - 1) * BK;  // columns of the last block
@@ -359,10 +431,12 @@ __global__ void __launch_bounds__(NT, 1) gemm_kernel(const GemmArgs g) {
                 if (kb + 1 < nkb || ktail == BK) {
 #pragma unroll
                     for (int t = 0; t < BK / 16; ++t)
-                        mma_bf16(tmem, ad + 2 * t, bd + 2 * t, idesc, (kb > 0 || t > 0) ? 1u : 0u);
+                        mma_bf16(tmem, ad + k_step<A_MN>() * t, bd + k_step<B_MN>() * t, idesc,
+                                 (kb > 0 || t > 0) ? 1u : 0u);
                 } else {
                     for (int t = 0; t * 16 < ktail; ++t)
-                        mma_bf16(tmem, ad + 2 * t, bd + 2 * t, idesc, (kb > 0 || t > 0) ? 1u : 0u);
+                        mma_bf16(tmem, ad + k_step<A_MN>() * t, bd + k_step<B_MN>() * t, idesc,
+                                 (kb > 0 || t > 0) ? 1u : 0u);
                 }
                 mma_commit(free0 + 8 * st);
             }
@@ -396,11 +470,23 @@ __global__ void __launch_bounds__(NT, 1) gemm_kernel(const GemmArgs g) {
 #pragma unroll
                 for (int i = 0; i < 16; ++i) v[i] = 0.0f;
             }
+            if (g.adj_pre) {
+#pragma unroll
+                for (int i = 0; i < 16; ++i) {
+                    const bool in = r < g.M && n0 + c0 + i < g.N;
+                    v[i] = in ? v[i] * gelu_grad(g.adj_pre[(size_t)r * g.ldc + n0 + c0 + i]) : 0.0f;
+                }
+                const float sum = column_sum16(v);
+                if ((lane & 1) == 0) s_col[warp & 3][c0 + (lane >> 1)] = sum;
+            }
             if (r < g.M) epilogue16(g, r, n0 + c0, v, vec);
         }
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
+    if (ok && g.adj_pre && tid < bn && n0 + tid < g.N)  // the four row quarters, in order
+        g.colpart[(size_t)blockIdx.x * g.N + n0 + tid] =
+            ((s_col[0][tid] + s_col[1][tid]) + s_col[2][tid]) + s_col[3][tid];
     if (warp == LOADERS)
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(ncols));
 }
@@ -552,8 +638,9 @@ __global__ void mse_kernel(const float* pred, const float* target, int M, int N,
     if (threadIdx.x == 0 && loss) loss[0] = s[0] * inv;
 }
 
+// p_bf16, if given, receives the updated parameters rounded to bf16.
 __global__ void adam_kernel(float* p, const float* g, float* m, float* v, long long count, float lr,
-                            float b1, float b2, float eps, float c1, float c2) {
+                            float b1, float b2, float eps, float c1, float c2, uint16_t* p_bf16) {
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < count;
          i += (long long)gridDim.x * blockDim.x) {
         const float gi = g[i];
@@ -561,7 +648,9 @@ __global__ void adam_kernel(float* p, const float* g, float* m, float* v, long l
         const float vi = b2 * v[i] + (1.0f - b2) * gi * gi;
         m[i] = mi;
         v[i] = vi;
-        p[i] -= lr * (mi / c1) / (sqrtf(vi / c2) + eps);
+        const float pi = p[i] - lr * (mi / c1) / (sqrtf(vi / c2) + eps);
+        p[i] = pi;
+        if (p_bf16) p_bf16[i] = f_to_bf16(pi);
     }
 }
 
@@ -571,7 +660,260 @@ int grid_for(long long n, int threads) {
     return (int)(b > 148LL * 16 ? 148LL * 16 : b);
 }
 
-bool g_smem_set[64] = {false};
+// ------------------------------------------------------ network kernels
+// im2col of the fp32 network input, eight columns (one 16-byte store) per
+// thread (one element per thread, 64-bit index divisions: 22 us for the
+// first layer of 256 records; this form 8 us).
+__global__ void im2col8_kernel(const float* __restrict__ x, int Nb, int Lin, int Cin, int sn, int sl, int sc,
+                               int k, int stride, int pad, int Lout, float scale, uint16_t* cols, int ldcols) {
+    const unsigned per = (unsigned)ldcols / 8, total = (unsigned)Nb * Lout * per;
+    const unsigned t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= total) return;
+    const unsigned row = t / per;
+    const int c0 = (int)(t - row * per) * 8;
+    const int n = (int)(row / (unsigned)Lout), l0 = (int)(row - (unsigned)n * Lout) * stride - pad;
+    int kk = c0 / Cin, ci = c0 - kk * Cin;
+    uint16_t v[8];
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+        const int l = l0 + kk;
+        float f = 0.0f;
+        if (kk < k && l >= 0 && l < Lin) f = x[(size_t)n * sn + (size_t)l * sl + (size_t)ci * sc] * scale;
+        v[e] = f_to_bf16(f);
+        if (++ci == Cin) {
+            ci = 0;
+            ++kk;
+        }
+    }
+    uint4 q;
+    q.x = v[0] | (uint32_t)v[1] << 16;
+    q.y = v[2] | (uint32_t)v[3] << 16;
+    q.z = v[4] | (uint32_t)v[5] << 16;
+    q.w = v[6] | (uint32_t)v[7] << 16;
+    *reinterpret_cast<uint4*>(cols + (size_t)row * ldcols + c0) = q;
+}
+
+constexpr int ADJ_ROWS = 128;  // rows per block of the kernel below
+
+// Adjoint of a layer's activation over [rows, C], four channels per thread:
+// the adjoint of the activation is src itself (k == 0) or gathered from the
+// next convolution's patches (the sum of nn_col2im, in its order); times
+// gelu'(pre) if pre is given; written as bf16, with the column sums of each
+// block's rows (the bias gradient's partial sums).  One pass in place of
+// col2im, activation adjoint, transpose and column sums, with three fp32
+// arrays written and read back (first convolution of 256 records: 120 us in
+// four kernels, 12 us here; memory bound, 32 MB).
+__global__ void __launch_bounds__(256) adjoint_rows_kernel(const float* __restrict__ src, int ld, int rows, int C,
+                                                           int Lin, int k, int stride, int pad, int Lout,
+                                                           const float* __restrict__ pre, uint16_t* d_bf16,
+                                                           float* colpart) {
+    __shared__ float4 s_sum[256];
+    const int tpr = C / 4, rpp = 256 / tpr;  // threads per row, rows per pass
+    const int t = threadIdx.x, g = t / tpr, c = (t - g * tpr) * 4;
+    float4 sum = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    const int row0 = blockIdx.x * ADJ_ROWS, row1 = min(rows, row0 + ADJ_ROWS);
+    for (int r = row0 + g; r < row1; r += rpp) {
+        float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        if (k == 0) {
+            v = *reinterpret_cast<const float4*>(src + (size_t)r * ld + c);
+        } else {
+            const int n = r / Lin, l = r - n * Lin;
+            for (int kk = (l + pad) % stride; kk < k; kk += stride) {  // kk = l + pad - lo * stride
+                const int lo = (l + pad - kk) / stride;
+                if (l + pad < kk || lo >= Lout) continue;
+                const float4 q =
+                    *reinterpret_cast<const float4*>(src + ((size_t)n * Lout + lo) * ld + (size_t)kk * C + c);
+                v.x += q.x;
+                v.y += q.y;
+                v.z += q.z;
+                v.w += q.w;
+            }
+        }
+        const size_t o = (size_t)r * C + c;
+        if (pre) {
+            const float4 q = *reinterpret_cast<const float4*>(pre + o);
+            v.x *= gelu_grad(q.x);
+            v.y *= gelu_grad(q.y);
+            v.z *= gelu_grad(q.z);
+            v.w *= gelu_grad(q.w);
+        }
+        ushort4 b;
+        b.x = f_to_bf16(v.x);
+        b.y = f_to_bf16(v.y);
+        b.z = f_to_bf16(v.z);
+        b.w = f_to_bf16(v.w);
+        *reinterpret_cast<ushort4*>(d_bf16 + o) = b;
+        sum.x += v.x;
+        sum.y += v.y;
+        sum.z += v.z;
+        sum.w += v.w;
+    }
+    s_sum[t] = sum;
+    __syncthreads();
+    if (t < tpr) {
+        for (int q = 1; q < rpp; ++q) {
+            const float4 v = s_sum[q * tpr + t];
+            sum.x += v.x;
+            sum.y += v.y;
+            sum.z += v.z;
+            sum.w += v.w;
+        }
+        *reinterpret_cast<float4*>(colpart + (size_t)blockIdx.x * C + c) = sum;
+    }
+}
+
+// Bias gradients of all layers: out[c] = sum of part[t][c], t < T, a warp per
+// column (lanes stride over t, then a fixed tree).
+constexpr int MAX_LAYERS = 8;
+struct BiasArgs {
+    const float* part[MAX_LAYERS];
+    float* out[MAX_LAYERS];
+    int T[MAX_LAYERS], n[MAX_LAYERS];
+    int layers;
+};
+
+__global__ void bias_reduce_kernel(const BiasArgs a) {
+    int c = (int)(blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)), i = 0;
+    while (i < a.layers && c >= a.n[i]) c -= a.n[i++];
+    if (i == a.layers) return;
+    const float* p = a.part[i] + c;
+    float v = 0.0f;
+    for (int t = threadIdx.x & 31; t < a.T[i]; t += 32) v += p[(size_t)t * a.n[i]];
+    for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
+    if ((threadIdx.x & 31) == 0) a.out[i][c] = v;
+}
+
+// Dynamic shared memory limit raised once per device and kernel.
+template <bool A_MN, bool B_MN>
+int allow_smem() {
+    static std::atomic<uint64_t> set{0};
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return SWE_ECUDA;
+    if (set.load(std::memory_order_acquire) >> dev & 1) return SWE_OK;
+    if (cudaFuncSetAttribute(gemm_kernel<A_MN, B_MN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             SMEM_MAX + SMEM_ALIGN) != cudaSuccess)
+        return SWE_ECUDA;
+    set.fetch_or(1ull << dev, std::memory_order_release);
+    return SWE_OK;
+}
+
+// Launch the product of g's operands (everything but the launch shape is
+// set), K split over ksplit CTAs at most.
+template <bool A_MN, bool B_MN>
+int launch_gemm(GemmArgs g, int ksplit, float* workspace, cudaStream_t s) {
+    const int rc = allow_smem<A_MN, B_MN>();
+    if (rc != SWE_OK) return rc;
+    // K per split, a multiple of BK
+    const int kblocks = (g.K + BK - 1) / BK;
+    const int per = (kblocks + ksplit - 1) / ksplit;
+    g.kchunk = per * BK;
+    const int zs = (kblocks + per - 1) / per;
+    g.partial = zs > 1 ? workspace : nullptr;
+    // Tile columns: the widest tile (A is read once per column tile) whose
+    // grid still has a CTA for each SM, or the narrowest.
+    int bn = BN_MAX;
+    const long long mz = (long long)((g.M + BM - 1) / BM) * zs;
+    while (bn > 16 && (bn / 2 >= g.N || mz * ((g.N + bn - 1) / bn) < 148)) bn /= 2;
+    g.bn = bn;
+    const int stage = tile_bytes(BM) + (B_MN ? mn_tile_bytes(bn) : tile_bytes(bn));
+    g.stages = 1;  // a power of two, no more than the K blocks need
+    while (g.stages < per && g.stages < (bn == BN_MAX ? 4 : STAGES_MAX)) g.stages *= 2;
+    const dim3 grid((g.M + BM - 1) / BM, (g.N + bn - 1) / bn, zs);
+    gemm_kernel<A_MN, B_MN><<<grid, NT, g.stages * stage + SMEM_ALIGN, s>>>(g);
+    if (zs > 1) splitk_epilogue_kernel<<<grid_for((long long)g.M * g.N, 256), 256, 0, s>>>(g, zs);
+    return cudaGetLastError() == cudaSuccess ? SWE_OK : SWE_ECUDA;
+}
+
+Operand lines(const uint16_t* p, int ld, int n, int cols) { return Operand{p, ld, n, cols, 0, 0, 0}; }
+
+// ------------------------------------------------------------- the network
+int round_up(int x, int m) { return (x + m - 1) / m * m; }
+size_t align256(size_t x) { return (x + 255) / 256 * 256; }
+int rows_of(const nn_layer& l, int nb) { return l.conv ? nb * l.lout : nb; }
+int split_of(int K) { return K / 2048 < 1 ? 1 : (K / 2048 > 128 ? 128 : K / 2048); }
+
+// The layer list that the functions below accept: convolutions (the first
+// one on the fp32 input, the others in place on the previous layer's NLC
+// activations), then dense layers.
+bool valid_layers(const nn_layer* L, int n, int nb) {
+    if (!L || n < 2 || n > MAX_LAYERS || nb < 1 || !L[0].conv || L[n - 1].conv) return false;
+    for (int i = 0; i < n; ++i) {
+        const nn_layer& l = L[i];
+        if (l.cin < 1 || l.cout < 1 || l.kpad < 16 || l.kpad % 16 || l.w < 0 || l.b < 0 || l.w % 8) return false;
+        if (l.conv) {
+            if (i > 0 && !L[i - 1].conv) return false;
+            if (l.k < 1 || l.stride < 1 || l.pad < 0 || l.lin < 1 ||
+                l.lout != (l.lin + 2 * l.pad - l.k) / l.stride + 1 || l.lout < 1 || l.kpad < l.k * l.cin)
+                return false;
+            if (i > 0 && (l.cin != L[i - 1].cout || l.lin != L[i - 1].lout || l.kpad != l.k * l.cin)) return false;
+        } else if (l.kpad != l.cin || l.cin != (L[i - 1].conv ? L[i - 1].cout * L[i - 1].lout : L[i - 1].cout)) {
+            return false;
+        }
+        // rows of 16-byte chunks, whole four-channel groups, 32-bit indices
+        if (i + 1 < n && l.cout % 16) return false;
+        if (i + 1 < n && L[i + 1].conv && (l.cout > 1024 || 256 % (l.cout / 4))) return false;
+        if ((long long)rows_of(l, nb) * (l.kpad > l.cout ? l.kpad : l.cout) >= (1ll << 31)) return false;
+    }
+    return true;
+}
+
+// Workspace of one batch size: forward buffers, then the backward ones.
+struct NetBuffers {
+    uint16_t* cols;                 // first layer's patches
+    float* pre[MAX_LAYERS];         // pre-activations
+    uint16_t* act[MAX_LAYERS];      // activations (not of the last layer)
+    uint16_t* d[MAX_LAYERS];        // adjoints of the pre-activations
+    float* dcols;                   // adjoint of a convolution's patches
+    float* colpart[MAX_LAYERS];     // column sums of d, per row tile
+    float* split;                   // partial products
+    size_t bytes;
+};
+
+int column_tiles(const nn_layer* L, int n, int i, int nb) {
+    // the last layer and the inputs of convolutions: adjoint_rows_kernel; the
+    // others: the row tiles of the product that makes them
+    const int rows = rows_of(L[i], nb);
+    if (i == n - 1 || L[i + 1].conv) return (rows + ADJ_ROWS - 1) / ADJ_ROWS;
+    return (nb + BM - 1) / BM * (rows / nb);
+}
+
+NetBuffers carve(void* ws, const nn_layer* L, int n, int nb, bool training) {
+    NetBuffers b{};
+    size_t at = 0;
+    auto take = [&](size_t bytes) {
+        void* p = static_cast<char*>(ws) + at;
+        at += align256(bytes);
+        return p;
+    };
+    b.cols = (uint16_t*)take((size_t)nb * L[0].lout * L[0].kpad * 2);
+    for (int i = 0; i < n; ++i) {
+        const size_t e = (size_t)rows_of(L[i], nb) * L[i].cout;
+        b.pre[i] = (float*)take(e * 4);
+        if (i + 1 < n) b.act[i] = (uint16_t*)take(e * 2);
+    }
+    if (training) {
+        size_t dc = 0, sp = 0;
+        for (int i = 0; i < n; ++i) {
+            const int rows = rows_of(L[i], nb), Mp = round_up(rows, 64);
+            b.d[i] = (uint16_t*)take((size_t)rows * L[i].cout * 2);
+            b.colpart[i] = (float*)take((size_t)column_tiles(L, n, i, nb) * L[i].cout * 4);
+            if (i > 0 && L[i].conv) dc = std::max(dc, (size_t)rows * L[i].kpad * 4);
+            if (split_of(Mp) > 1) sp = std::max(sp, (size_t)split_of(Mp) * L[i].cout * L[i].kpad * 4);
+        }
+        b.dcols = (float*)take(dc);
+        b.split = (float*)take(sp);
+    }
+    b.bytes = at;
+    return b;
+}
+
+// Layer i's input as lines of its data rows.
+Operand layer_input(const nn_layer* L, const NetBuffers& b, int i, int nb) {
+    const nn_layer& l = L[i];
+    if (i == 0) return lines(b.cols, l.kpad, nb * l.lout, l.kpad);
+    if (!l.conv) return lines(b.act[i - 1], l.cin, nb, l.cin);
+    return Operand{b.act[i - 1], l.stride * l.cin, nb * l.lout, l.kpad, l.lout, l.lin * l.cin, -l.pad * l.cin};
+}
 
 }  // namespace
 }  // namespace nn
@@ -589,48 +931,130 @@ extern "C" int nn_gemm_bf16(const uint16_t* A, int lda, const uint16_t* B, int l
     if (act != NN_ACT_NONE && act != NN_ACT_GELU) return SWE_EARG;
     if (!out_f32 && !out_bf16 && !pre_f32) return SWE_EARG;
     if (ldc < N || ksplit < 1 || ksplit > 1024 || (ksplit > 1 && !workspace)) return SWE_EARG;
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return SWE_ECUDA;
-    if (!g_smem_set[dev]) {
-        if (cudaFuncSetAttribute(gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 SMEM_MAX + SMEM_ALIGN) != cudaSuccess)
-            return SWE_ECUDA;
-        g_smem_set[dev] = true;
-    }
     GemmArgs g{};
-    g.A = A;
-    g.B = B;
+    g.A = lines(A, lda, M, K);
+    g.B = lines(B, ldb, N, K);
     g.M = M;
     g.N = N;
     g.K = K;
-    g.lda = lda;
-    g.ldb = ldb;
-    // K per split, a multiple of BK
-    const int kblocks = (K + BK - 1) / BK;
-    const int per = (kblocks + ksplit - 1) / ksplit;
-    g.kchunk = per * BK;
-    const int zs = (kblocks + per - 1) / per;
     g.bias = bias;
     g.act = act;
     g.ldc = ldc;
     g.out_f32 = out_f32;
     g.out_bf16 = out_bf16;
     g.pre_f32 = pre_f32;
-    g.partial = zs > 1 ? workspace : nullptr;
     g.err = err;
     g.wait_ns = (unsigned long long)wait_ns;
+    return launch_gemm<false, false>(g, ksplit, workspace, (cudaStream_t)stream);
+}
+
+extern "C" long long nn_net_workspace_bytes(const nn_layer* layers, int nlayers, int nb, int training) {
+    if (!valid_layers(layers, nlayers, nb)) return -1;
+    return (long long)carve(nullptr, layers, nlayers, nb, training != 0).bytes;
+}
+
+extern "C" int nn_net_forward(const nn_layer* layers, int nlayers, const float* params,
+                              const uint16_t* params_bf16, const float* x, float in_scale, int nb,
+                              void* workspace, float* out, long long wait_ns, uint32_t* err, void* stream) {
+    if (!valid_layers(layers, nlayers, nb) || !params || !params_bf16 || !x || !workspace || !out || wait_ns < 0)
+        return SWE_EARG;
+    if (((uintptr_t)workspace & 255u) || ((uintptr_t)params_bf16 & 15u)) return SWE_EARG;
     cudaStream_t s = (cudaStream_t)stream;
-    // Tile columns: the widest tile (A is read once per column tile) whose
-    // grid still has a CTA for each SM, or the narrowest.
-    int bn = BN_MAX;
-    const long long mz = (long long)((M + BM - 1) / BM) * zs;
-    while (bn > 16 && (bn / 2 >= N || mz * ((N + bn - 1) / bn) < 148)) bn /= 2;
-    g.bn = bn;
-    g.stages = 1;  // a power of two, no more than the K blocks need
-    while (g.stages < per && g.stages < (bn == BN_MAX ? 4 : STAGES_MAX)) g.stages *= 2;
-    const dim3 grid((M + BM - 1) / BM, (N + bn - 1) / bn, zs);
-    gemm_kernel<<<grid, NT, g.stages * (tile_bytes(BM) + tile_bytes(bn)) + SMEM_ALIGN, s>>>(g);
-    if (zs > 1) splitk_epilogue_kernel<<<grid_for((long long)M * N, 256), 256, 0, s>>>(g, zs);
+    const nn_layer* L = layers;
+    const NetBuffers b = carve(workspace, L, nlayers, nb, false);
+    {
+        const nn_layer& l = L[0];  // x is [nb, cin, lin]
+        const long long total = (long long)nb * l.lout * (l.kpad / 8);
+        im2col8_kernel<<<(unsigned)((total + 255) / 256), 256, 0, s>>>(x, nb, l.lin, l.cin, l.cin * l.lin, 1, l.lin,
+                                                                       l.k, l.stride, l.pad, l.lout, in_scale,
+                                                                       b.cols, l.kpad);
+    }
+    for (int i = 0; i < nlayers; ++i) {
+        const nn_layer& l = L[i];
+        const bool last = i == nlayers - 1;
+        GemmArgs g{};
+        g.A = layer_input(L, b, i, nb);
+        g.B = lines(params_bf16 + l.w, l.kpad, l.cout, l.kpad);
+        g.M = rows_of(l, nb);
+        g.N = l.cout;
+        g.K = l.kpad;
+        g.bias = params + l.b;
+        g.act = last ? NN_ACT_NONE : NN_ACT_GELU;
+        g.ldc = l.cout;
+        g.out_f32 = last ? out : nullptr;
+        g.out_bf16 = last ? nullptr : b.act[i];
+        g.pre_f32 = b.pre[i];
+        g.err = err;
+        g.wait_ns = (unsigned long long)wait_ns;
+        const int rc = launch_gemm<false, false>(g, 1, nullptr, s);
+        if (rc != SWE_OK) return rc;
+    }
+    return cudaGetLastError() == cudaSuccess ? SWE_OK : SWE_ECUDA;
+}
+
+extern "C" int nn_net_backward(const nn_layer* layers, int nlayers, const uint16_t* params_bf16,
+                               const float* dout, int nb, void* workspace, float* grads,
+                               long long wait_ns, uint32_t* err, void* stream) {
+    if (!valid_layers(layers, nlayers, nb) || !params_bf16 || !dout || !workspace || !grads || wait_ns < 0)
+        return SWE_EARG;
+    const nn_layer* L = layers;
+    const int n = nlayers;
+    if (L[n - 1].cout % 16 || L[n - 1].cout > 1024 || 256 % (L[n - 1].cout / 4)) return SWE_EARG;
+    if (((uintptr_t)workspace & 255u) || ((uintptr_t)params_bf16 & 15u) || ((uintptr_t)dout & 15u)) return SWE_EARG;
+    cudaStream_t s = (cudaStream_t)stream;
+    const NetBuffers b = carve(workspace, L, n, nb, true);
+    BiasArgs ba{};
+    int columns = 0;
+    ba.layers = n;
+    for (int i = 0; i < n; ++i) {
+        ba.part[i] = b.colpart[i];
+        ba.out[i] = grads + L[i].b;
+        ba.T[i] = column_tiles(L, n, i, nb);
+        ba.n[i] = L[i].cout;
+        columns += L[i].cout;
+    }
+    adjoint_rows_kernel<<<(nb + ADJ_ROWS - 1) / ADJ_ROWS, 256, 0, s>>>(
+        dout, L[n - 1].cout, nb, L[n - 1].cout, 0, 0, 0, 0, 0, nullptr, b.d[n - 1], b.colpart[n - 1]);
+    for (int i = n - 1; i >= 0; --i) {
+        const nn_layer& l = L[i];
+        const int rows = rows_of(l, nb), Mp = round_up(rows, 64);
+        GemmArgs g{};
+        g.err = err;
+        g.wait_ns = (unsigned long long)wait_ns;
+        // dW [cout, kpad] = d^T X: both operands read in place, a line per data row
+        g.A = lines(b.d[i], l.cout, rows, l.cout);
+        g.B = layer_input(L, b, i, nb);
+        g.M = l.cout;
+        g.N = g.ldc = l.kpad;
+        g.K = Mp;
+        g.out_f32 = grads + l.w;
+        int rc = launch_gemm<true, true>(g, split_of(Mp), b.split, s);
+        if (rc != SWE_OK) return rc;
+        if (i == 0) break;
+        // dX [rows, kpad] = d W
+        g.A = lines(b.d[i], l.cout, rows, l.cout);
+        g.B = lines(params_bf16 + l.w, l.kpad, l.cout, l.kpad);
+        g.M = rows;
+        g.N = g.ldc = l.kpad;
+        g.K = l.cout;
+        g.out_f32 = nullptr;
+        if (!l.conv) {  // straight to the adjoint of the previous pre-activations
+            g.adj_pre = b.pre[i - 1];
+            g.out_bf16 = b.d[i - 1];
+            g.colpart = b.colpart[i - 1];
+            rc = launch_gemm<false, true>(g, 1, nullptr, s);
+            if (rc != SWE_OK) return rc;
+        } else {
+            g.out_f32 = b.dcols;
+            rc = launch_gemm<false, true>(g, 1, nullptr, s);
+            if (rc != SWE_OK) return rc;
+            const int prows = nb * l.lin;
+            adjoint_rows_kernel<<<(prows + ADJ_ROWS - 1) / ADJ_ROWS, 256, 0, s>>>(
+                b.dcols, l.kpad, prows, l.cin, l.lin, l.k, l.stride, l.pad, l.lout, b.pre[i - 1], b.d[i - 1],
+                b.colpart[i - 1]);
+        }
+    }
+    bias_reduce_kernel<<<(columns + 7) / 8, 256, 0, s>>>(ba);
     return cudaGetLastError() == cudaSuccess ? SWE_OK : SWE_ECUDA;
 }
 
@@ -705,12 +1129,17 @@ extern "C" int nn_mse(const float* pred, const float* target, int M, int N, floa
     return cudaGetLastError() == cudaSuccess ? SWE_OK : SWE_ECUDA;
 }
 
-extern "C" int nn_adam(float* params, const float* grads, float* m, float* v, long long count, float lr,
-                       float beta1, float beta2, float eps, int step, void* stream) {
+extern "C" int nn_adam_bf16(float* params, const float* grads, float* m, float* v, long long count, float lr,
+                            float beta1, float beta2, float eps, int step, uint16_t* params_bf16, void* stream) {
     if (!params || !grads || !m || !v || count < 1 || step < 1) return SWE_EARG;
     const float c1 = 1.0f - powf(beta1, (float)step);
     const float c2 = 1.0f - powf(beta2, (float)step);
-    adam_kernel<<<grid_for(count, 256), 256, 0, (cudaStream_t)stream>>>(params, grads, m, v, count, lr,
-                                                                        beta1, beta2, eps, c1, c2);
+    adam_kernel<<<grid_for(count, 256), 256, 0, (cudaStream_t)stream>>>(params, grads, m, v, count, lr, beta1,
+                                                                        beta2, eps, c1, c2, params_bf16);
     return cudaGetLastError() == cudaSuccess ? SWE_OK : SWE_ECUDA;
+}
+
+extern "C" int nn_adam(float* params, const float* grads, float* m, float* v, long long count, float lr,
+                       float beta1, float beta2, float eps, int step, void* stream) {
+    return nn_adam_bf16(params, grads, m, v, count, lr, beta1, beta2, eps, step, nullptr, stream);
 }

@@ -10,8 +10,10 @@ part; its inversion is
 bc_inversion_train.py:648-768``).
 
 Every training and inference kernel is this project's (``csrc/nn_b200.cu``):
-bf16 matrix products with fp32 accumulation on the tcgen05 tensor cores,
-im2col / col2im, activation adjoints, Adam.  The network:
+bf16 matrix products with fp32 accumulation on the tcgen05 tensor cores
+(convolutions read their patches in place, weight gradients their operands
+untransposed), activation adjoints fused into them, Adam.  A pass is one
+call into the library.  The network:
 
 =======  ==============================================  ===========
 layer    shape                                           parameters
@@ -25,9 +27,9 @@ fc3      96 -> 16 (normalised controls)                  1,552
 =======  ==============================================  ===========
 
 GELU after every layer but the last; 508,528 parameters (fp32 master copy,
-bf16 copies for the products).  Activations are kept channel-last (NLC), so
-a convolution's output matrix [N*L, C] is the next im2col's input and the
-last one flattens to fc1's input without a copy.
+a bf16 copy for the products).  Activations are kept channel-last (NLC), so
+a patch of the next convolution is a contiguous slice of them and the last
+one flattens to fc1's input without a copy.
 """
 from __future__ import annotations
 
@@ -39,7 +41,6 @@ import torch
 
 from . import _native as nat
 
-ACT_NONE, ACT_GELU = 0, 1
 SAMPLES, GAUGES, CONTROLS = 1125, 6, 16
 INPUT_SCALE = 100.0                   # eta [m] -> input units (1 cm -> 1)
 CONTROL_MEAN, CONTROL_SCALE = 0.0015, 0.0078   # controls ~ U[-0.012, 0.015] m
@@ -84,10 +85,6 @@ def architecture(samples: int = SAMPLES, gauges: int = GAUGES, controls: int = C
     return [c1, c2, c3, Dense(c3.cout * c3.lout, 96), Dense(96, 96), Dense(96, controls)]
 
 
-def _round_up(x: int, m: int) -> int:
-    return -(-x // m) * m
-
-
 def param_layout(layers) -> List[Tuple[int, int, int, int]]:
     """(weight offset, rows, padded cols, bias offset) per layer in the flat
     parameter vector."""
@@ -129,12 +126,15 @@ class WarmStartNet:
             host[w:w + rows * kp] = Wp.reshape(-1)
             host[b:b + rows] = (torch.rand(rows, generator=g) * 2 - 1) * bound
         self.params.copy_(host)
-        self.W_bf16 = [torch.empty((L.cout, L.kpad), dtype=torch.int16, device=self.dev)
-                       for L in self.layers]
-        self.Wt_bf16 = [torch.empty((L.kpad, L.cout), dtype=torch.int16, device=self.dev)
-                        for L in self.layers]
+        self.params_bf16 = torch.empty(self.nparams, dtype=torch.int16, device=self.dev)
         self._refresh_bf16()
-        self._nb = None
+        self._table = (nat.NnLayer * len(self.layers))()
+        for t, L, (w, _, kp, b) in zip(self._table, self.layers, self.layout):
+            conv = isinstance(L, Conv)
+            t.conv, t.cin, t.cout, t.kpad, t.w, t.b = int(conv), L.cin, L.cout, kp, w, b
+            if conv:
+                t.k, t.stride, t.pad, t.lin, t.lout = L.k, L.stride, L.pad, L.lin, L.lout
+        self._cap = 0  # the largest batch that the workspace and the outputs hold
 
     # ----------------------------------------------------------- helpers
     def weight(self, i):
@@ -157,56 +157,22 @@ class WarmStartNet:
         return nat.stream_handle(self.dev)
 
     def _refresh_bf16(self):
-        lib = nat.lib()
-        for i, L in enumerate(self.layers):
-            W = self.weight(i)
-            nat.check(lib.nn_cast_bf16(nat.ptr(W), L.cout, L.kpad, L.kpad, nat.ptr(self.W_bf16[i]),
-                                       L.kpad, nat.ptr(self.Wt_bf16[i]), L.cout, self._st()),
-                      "nn cast")
-
-    def _gemm(self, A, lda, B, ldb, M, N, K, bias=None, act=ACT_NONE, out_f32=None, out_bf16=None,
-              pre=None, ldc=None, ksplit=1):
-        ws = None
-        if ksplit > 1:
-            need = ksplit * M * N
-            if self._ws is None or self._ws.numel() < need:
-                self._ws = torch.empty(need, device=self.dev)
-            ws = self._ws
-        rc = nat.lib().nn_gemm_bf16(nat.ptr(A), lda, nat.ptr(B), ldb, M, N, K, nat.ptr(bias), act,
-                                    nat.ptr(out_f32), nat.ptr(out_bf16), nat.ptr(pre),
-                                    N if ldc is None else ldc, ksplit, nat.ptr(ws), self.wait_ns,
-                                    nat.ptr(self.err), self._st())
-        nat.check(rc, "nn gemm")
-
-    @staticmethod
-    def _ksplit(K: int) -> int:
-        return max(1, min(128, K // 2048))
+        nat.check(nat.lib().nn_cast_bf16(nat.ptr(self.params), 1, self.nparams, self.nparams,
+                                         nat.ptr(self.params_bf16), self.nparams, None, 0, self._st()),
+                  "nn cast")
 
     def _buffers(self, nb: int):
-        if self._nb == nb:
+        """Workspace and outputs, for the largest batch seen."""
+        if nb <= self._cap:
             return
-        dev, L = self.dev, self.layers
-        bf = dict(dtype=torch.int16, device=dev)
-        self._ws = None
-        self.cols = [torch.empty((nb * c.lout, c.kpad), **bf) for c in L[:3]]
-        self.pre = [torch.empty((nb * c.lout, c.cout), device=dev) for c in L[:3]]
-        self.act = [torch.empty((nb * c.lout, c.cout), **bf) for c in L[:3]]
-        self.pre += [torch.empty((nb, d.cout), device=dev) for d in L[3:]]
-        self.act += [torch.empty((nb, d.cout), **bf) for d in L[3:5]]
-        self.out = torch.empty((nb, L[5].cout), device=dev)
-        self.dpred = torch.empty_like(self.out)
-        self.loss = torch.zeros(1, device=dev)
-        # backward scratch
-        rows = [nb * c.lout for c in L[:3]] + [nb] * 3
-        self.rows = rows
-        self.rows_pad = [_round_up(r, 64) for r in rows]
-        self.dact = [torch.empty((r, l.cout), device=dev) for r, l in zip(rows, L)]
-        self.d_bf16 = [torch.empty((r, l.cout), **bf) for r, l in zip(rows, L)]
-        self.dT_bf16 = [torch.empty((l.cout, rp), **bf) for rp, l in zip(self.rows_pad, L)]
-        ins = [c.kpad for c in L[:3]] + [d.cin for d in L[3:]]
-        self.xT_bf16 = [torch.empty((k, rp), **bf) for k, rp in zip(ins, self.rows_pad)]
-        self.dcols = [None] + [torch.empty((nb * c.lout, c.kpad), device=dev) for c in L[1:3]]
-        self._nb = nb
+        nbytes = nat.lib().nn_net_workspace_bytes(self._table, len(self.layers), nb, 1)
+        if nbytes < 0:
+            raise ValueError(f"the network's shapes are not supported for a batch of {nb}")
+        self._ws = torch.empty(int(nbytes), dtype=torch.uint8, device=self.dev)
+        self._out = torch.empty((nb, self.controls), device=self.dev)
+        self._dpred = torch.empty_like(self._out)
+        self.loss = torch.zeros(1, device=self.dev)
+        self._cap = nb
 
     # ----------------------------------------------------------- forward
     def forward(self, x: torch.Tensor) -> torch.Tensor:
@@ -217,92 +183,24 @@ class WarmStartNet:
         if G != self.gauges or T != self.samples:
             raise ValueError(f"expected [N, {self.gauges}, {self.samples}] gauge series, got {tuple(x.shape)}")
         self._buffers(nb)
-        lib, L = nat.lib(), self.layers
-        src_f32, src_bf16 = x, None
-        strides = (G * T, 1, T)  # NCL input
-        for i in range(3):
-            c = L[i]
-            scale = INPUT_SCALE if i == 0 else 1.0
-            rc = lib.nn_im2col(nat.ptr(src_f32), nat.ptr(src_bf16), nb, c.lin, c.cin, strides[0],
-                               strides[1], strides[2], c.k, c.stride, c.pad, c.lout, scale, 0.0,
-                               nat.ptr(self.cols[i]), c.kpad, self._st())
-            nat.check(rc, "nn im2col")
-            self._gemm(self.cols[i], c.kpad, self.W_bf16[i], c.kpad, nb * c.lout, c.cout, c.kpad,
-                       bias=self.bias(i), act=ACT_GELU, out_bf16=self.act[i], pre=self.pre[i])
-            src_f32, src_bf16 = None, self.act[i]
-            strides = (c.lout * c.cout, c.cout, 1)  # NLC
-        h = self.act[2]  # [nb * L3, 128] == [nb, 4480]
-        for j, i in enumerate(range(3, 6)):
-            d = L[i]
-            last = i == 5
-            self._gemm(h, d.cin, self.W_bf16[i], d.kpad, nb, d.cout, d.kpad, bias=self.bias(i),
-                       act=ACT_NONE if last else ACT_GELU, out_f32=self.out if last else None,
-                       out_bf16=None if last else self.act[i], pre=self.pre[i])
-            if not last:
-                h = self.act[i]
+        self._nb = nb
+        self.out, self.dpred = self._out[:nb], self._dpred[:nb]
+        rc = nat.lib().nn_net_forward(self._table, len(self.layers), nat.ptr(self.params),
+                                      nat.ptr(self.params_bf16), nat.ptr(x), INPUT_SCALE, nb,
+                                      nat.ptr(self._ws), nat.ptr(self.out), self.wait_ns,
+                                      nat.ptr(self.err), self._st())
+        nat.check(rc, "nn forward")
         return self.out
 
     # ---------------------------------------------------------- backward
     def backward(self, dout: torch.Tensor) -> None:
         """Gradients of all parameters into self.grads for the cotangent of
         the last forward's output [Nb, controls]."""
-        lib, L, nb = nat.lib(), self.layers, self._nb
-        st = self._st()
-        self.grads.zero_()
-        dact = dout  # [rows, cout] fp32
-        for i in range(5, -1, -1):
-            lay = L[i]
-            M, N = self.rows[i], lay.cout
-            Mp = self.rows_pad[i]
-            act = ACT_NONE if i == 5 else ACT_GELU
-            rc = lib.nn_act_backward(nat.ptr(dact), nat.ptr(self.pre[i]), M, N, N, act,
-                                     nat.ptr(self.d_bf16[i]), N, nat.ptr(self.dT_bf16[i]), Mp,
-                                     nat.ptr(self.dact[i]), st)
-            nat.check(rc, "nn act backward")
-            nat.check(lib.nn_colsum(nat.ptr(self.dact[i]), M, N, N, nat.ptr(self.bias_grad(i)), st),
-                      "nn colsum")
-            # layer input X [M, Kin] (bf16) and its transpose [Kin, Mp]
-            if i < 3:
-                X, kin = self.cols[i], lay.kpad
-            elif i == 3:
-                X, kin = self.act[2], lay.cin
-            else:
-                X, kin = self.act[i - 1], lay.cin
-            nat.check(lib.nn_transpose_bf16(nat.ptr(X), M, kin, kin, nat.ptr(self.xT_bf16[i]), Mp, st),
-                      "nn transpose")
-            # dW [N, Kin] = d^T X
-            self._gemm(self.dT_bf16[i], Mp, self.xT_bf16[i], Mp, N, kin, Mp,
-                       out_f32=self.weight_grad(i), ldc=lay.kpad, ksplit=self._ksplit(Mp))
-            if i == 0:
-                break
-            # dX [M, Kin] = d W
-            if i > 3:
-                dst = self.dact_in(i)
-                self._gemm(self.d_bf16[i], N, self.Wt_bf16[i], N, M, kin, N, out_f32=dst)
-                dact = dst
-            elif i == 3:
-                dst = self.dact_in(3)  # [nb, 4480] == conv3 output [nb * L3, 128]
-                self._gemm(self.d_bf16[i], N, self.Wt_bf16[i], N, M, kin, N, out_f32=dst)
-                dact = dst
-            else:
-                self._gemm(self.d_bf16[i], N, self.Wt_bf16[i], N, M, kin, N, out_f32=self.dcols[i])
-                prev = L[i - 1]
-                dst = self.dact_in(i)
-                rc = lib.nn_col2im(nat.ptr(self.dcols[i]), lay.kpad, nb, lay.lin, lay.cin, lay.k,
-                                   lay.stride, lay.pad, lay.lout, nat.ptr(dst), st)
-                nat.check(rc, "nn col2im")
-                dact = dst
-
-    def dact_in(self, i):
-        """Buffer for the adjoint of layer i's input (= layer i-1's output)."""
-        if not hasattr(self, "_din") or self._din_nb != self._nb:
-            L, nb = self.layers, self._nb
-            self._din = {}
-            for j in range(1, 6):
-                prev_rows = self.rows[j - 1]
-                self._din[j] = torch.empty((prev_rows, L[j - 1].cout), device=self.dev)
-            self._din_nb = nb
-        return self._din[i]
+        dout = nat.require_cuda_f32("dout", dout)
+        rc = nat.lib().nn_net_backward(self._table, len(self.layers), nat.ptr(self.params_bf16),
+                                       nat.ptr(dout), self._nb, nat.ptr(self._ws), nat.ptr(self.grads),
+                                       self.wait_ns, nat.ptr(self.err), self._st())
+        nat.check(rc, "nn backward")
 
     # ---------------------------------------------------------- training
     def loss_and_grad(self, x, y_norm) -> torch.Tensor:
@@ -316,11 +214,10 @@ class WarmStartNet:
 
     def adam_step(self, lr=1e-3, beta1=0.9, beta2=0.999, eps=1e-8):
         self.step_count += 1
-        rc = nat.lib().nn_adam(nat.ptr(self.params), nat.ptr(self.grads), nat.ptr(self.m),
-                               nat.ptr(self.v), self.nparams, lr, beta1, beta2, eps, self.step_count,
-                               self._st())
+        rc = nat.lib().nn_adam_bf16(nat.ptr(self.params), nat.ptr(self.grads), nat.ptr(self.m),
+                                    nat.ptr(self.v), self.nparams, lr, beta1, beta2, eps,
+                                    self.step_count, nat.ptr(self.params_bf16), self._st())
         nat.check(rc, "nn adam")
-        self._refresh_bf16()
 
     def train_step(self, x, y_norm, lr=1e-3):
         loss = self.loss_and_grad(x, y_norm)

@@ -104,6 +104,45 @@ int nn_mse(const float* pred, const float* target, int M, int N, float* loss, fl
 int nn_adam(float* params, const float* grads, float* m, float* v, long long count, float lr,
             float beta1, float beta2, float eps, int step, void* stream);
 
+/* nn_adam that also writes the updated parameters as bf16 (may be NULL). */
+int nn_adam_bf16(float* params, const float* grads, float* m, float* v, long long count, float lr,
+                 float beta1, float beta2, float eps, int step, uint16_t* params_bf16, void* stream);
+
+/*
+ * The whole network: 1-D convolutions on channel-last activations, then
+ * dense layers, GELU after every layer but the last.  A layer's weight
+ * [cout, kpad] (column kk*cin + ci of a convolution) and bias [cout] lie at
+ * offsets w (a multiple of 8) and b of the flat parameter vector; kpad is
+ * k*cin (dense: cin) rounded up to 16 for the first layer, equal to it for
+ * the others.  cout of every layer but the last is a multiple of 16, that of
+ * a convolution before another one (and, for training, of the last layer)
+ * also a divisor of 1024.  At most 8 layers; others are refused (SWE_EARG,
+ * workspace -1).
+ */
+typedef struct {
+    int32_t conv; /* 1: convolution, 0: dense (k, stride, pad, lin, lout unused) */
+    int32_t cin, cout, k, stride, pad, lin, lout, kpad;
+    int32_t reserved;
+    int64_t w, b;
+} nn_layer;
+
+/* Bytes of the workspace (256-byte aligned) of a batch of nb records; with
+ * training != 0 for nn_net_backward too.  A larger batch's serves a smaller. */
+long long nn_net_workspace_bytes(const nn_layer* layers, int nlayers, int nb, int training);
+
+/* out [nb, cout of the last layer] from x [nb, cin, lin] fp32 (times
+ * in_scale); params fp32 and its bf16 copy.  Leaves the activations in the
+ * workspace for nn_net_backward. */
+int nn_net_forward(const nn_layer* layers, int nlayers, const float* params,
+                   const uint16_t* params_bf16, const float* x, float in_scale, int nb,
+                   void* workspace, float* out, long long wait_ns, uint32_t* err, void* stream);
+
+/* grads (every parameter, padding columns zero) for the cotangent dout of
+ * the last nn_net_forward with this workspace and batch. */
+int nn_net_backward(const nn_layer* layers, int nlayers, const uint16_t* params_bf16,
+                    const float* dout, int nb, void* workspace, float* grads, long long wait_ns,
+                    uint32_t* err, void* stream);
+
 #ifdef __cplusplus
 }
 #endif

@@ -247,3 +247,81 @@ def test_training_reduces_loss():
     net.check_errors()
     print("loss", first, last)
     assert last < 0.3 * first
+
+
+def _composed_pass(net, x, dout):
+    """Output, weight gradients and bias gradients (with the sum of the
+    magnitudes behind each) by the elementary entry points: patches and
+    transposes written out, one product or kernel at a time."""
+    lib, z, st = nat.lib(), ctypes.c_void_p(0), nat.stream_handle(torch.device(DEV))
+    nb, L = x.shape[0], net.layers
+    bf = dict(dtype=torch.int16, device=DEV)
+    err = torch.zeros(1, dtype=torch.int32, device=DEV)
+
+    def gemm(A, B, M, N, K, bias=None, act=0, ksplit=1):
+        out, ob, pre = (torch.zeros((M, N), device=DEV), torch.zeros((M, N), **bf), torch.zeros((M, N), device=DEV))
+        ws = torch.empty(ksplit * M * N, device=DEV)
+        nat.check(lib.nn_gemm_bf16(nat.ptr(A), A.shape[1], nat.ptr(B), B.shape[1], M, N, K, nat.ptr(bias), act,
+                                   nat.ptr(out), nat.ptr(ob), nat.ptr(pre), N, ksplit, nat.ptr(ws),
+                                   nat.NN_GEMM_WAIT_NS, nat.ptr(err), st), "gemm")
+        return out, ob, pre
+
+    def transposed(A, rows):
+        T = torch.zeros((A.shape[1], rows), **bf)
+        nat.check(lib.nn_transpose_bf16(nat.ptr(A), A.shape[0], A.shape[1], A.shape[1], nat.ptr(T), rows, st), "T")
+        return T
+
+    W, ins, pres, rows = [], [], [], []
+    src, h = x, None
+    for i, l in enumerate(L):
+        Wi = torch.zeros((l.cout, l.kpad), **bf)
+        nat.check(lib.nn_cast_bf16(nat.ptr(net.weight(i)), l.cout, l.kpad, l.kpad, nat.ptr(Wi), l.kpad, z, 0, st), "c")
+        M = nb * l.lout if i < 3 else nb
+        if i < 3:
+            X = torch.zeros((M, l.kpad), **bf)
+            strides = (l.cin * l.lin, 1, l.lin) if i == 0 else (l.lin * l.cin, l.cin, 1)
+            nat.check(lib.nn_im2col(nat.ptr(src) if i == 0 else z, nat.ptr(h), nb, l.lin, l.cin, *strides, l.k,
+                                    l.stride, l.pad, l.lout, INPUT_SCALE if i == 0 else 1.0, 0.0, nat.ptr(X),
+                                    l.kpad, st), "im2col")
+        else:
+            X = h.reshape(nb, l.cin)
+        out, h, pre = gemm(X, Wi, M, l.cout, l.kpad, net.bias(i), 0 if i == 5 else 1)
+        W.append(Wi), ins.append(X), pres.append(pre), rows.append(M)
+    dW, db, dact = [None] * 6, [None] * 6, dout
+    for i in range(5, -1, -1):
+        l, M, Mp = L[i], rows[i], -(-rows[i] // 64) * 64
+        d, dT, df = (torch.zeros((M, l.cout), **bf), torch.zeros((l.cout, Mp), **bf), torch.zeros((M, l.cout), device=DEV))
+        nat.check(lib.nn_act_backward(nat.ptr(dact), nat.ptr(pres[i]), M, l.cout, l.cout, 0 if i == 5 else 1,
+                                      nat.ptr(d), l.cout, nat.ptr(dT), Mp, nat.ptr(df), st), "act")
+        db[i] = (df.double().sum(0), df.double().abs().sum(0))
+        dW[i] = gemm(dT, transposed(ins[i], Mp), l.cout, l.kpad, Mp, ksplit=max(1, min(128, Mp // 2048)))[0]
+        if i == 0:
+            return out, dW, db
+        dact = gemm(d, transposed(W[i], l.cout), M, l.kpad, l.cout)[0]
+        if i < 3:
+            dX = torch.zeros((nb * l.lin, l.cin), device=DEV)
+            nat.check(lib.nn_col2im(nat.ptr(dact), l.kpad, nb, l.lin, l.cin, l.k, l.stride, l.pad, l.lout,
+                                    nat.ptr(dX), st), "col2im")
+            dact = dX
+
+
+@pytest.mark.parametrize("nb", [1, 2, 64, 129])
+def test_network_pass_equals_elementary_kernels(nb):
+    """Batches of one record, of a row tile and just past one, in a larger
+    batch's workspace: patches read in place, untransposed operands and fused
+    adjoints give the outputs and weight gradients of the elementary kernels
+    bit for bit (same products in the same order); bias gradients to fp32
+    summation error (a tree of at most a few hundred terms per lane)."""
+    net = WarmStartNet(DEV, seed=nb)
+    g = torch.Generator(device=DEV).manual_seed(nb)
+    net.forward(torch.zeros((nb + 3, 6, 1125), device=DEV))
+    x = torch.randn((nb, 6, 1125), device=DEV, generator=g) * 0.008
+    dout = torch.randn((nb, 16), device=DEV, generator=g) / nb
+    out = net.forward(x).clone()
+    net.backward(dout)
+    net.check_errors()
+    ref, dW, db = _composed_pass(net, x, dout)
+    assert torch.equal(out, ref)
+    for i in range(6):
+        assert torch.equal(net.weight_grad(i), dW[i])
+        assert bool(((net.bias_grad(i).double() - db[i][0]).abs() <= 600 * 2.0 ** -24 * db[i][1] + 1e-30).all())
