@@ -51,15 +51,17 @@ class AdjointStepper:
         self.model = model
         self.B, self.ny, self.nx, self.levelB = B, ny, nx, levelB
         self.bed_grad = bool(bed_grad)
-        rec = 16 if self.bed_grad else 12  # floats per face record
-        self.K1, self.K2, self.P = (torch.empty(shape, device=dev) for _ in range(3))
-        self.lam_k = torch.empty(shape, device=dev)
+        self.K1 = self.K2 = self.P = None  # stage intermediates, if they have to be recomputed
+        self.lam_k, self.lam_k1 = torch.empty(shape, device=dev), torch.empty(shape, device=dev)
         self.red = torch.empty(nat.RED_WORDS, dtype=torch.int32, device=dev)
-        self.cx = torch.empty(B * ny * (nx + 1) * rec, device=dev)
-        self.cy = torch.empty(B * (ny + 1) * nx * rec, device=dev)
+        # ghost adjoints and the frame's cells (include/swe_b200.h)
+        self.cx = torch.empty(16 * B * ny, device=dev)
+        self.cy = torch.empty(16 * B * nx + 4 * B * ny * nx, device=dev)
         # bed adjoint per batch member, accumulated over the steps of a pass
         self.lam_bed = torch.zeros((B, ny, nx), device=dev) if self.bed_grad else None
-        self.level_blocks = level_blocks(ny, nx)
+        # the launch that writes the partial sums works on the frame of two
+        # cells along the sides: a block per 256 of its cells
+        self.level_blocks = min(level_blocks(ny, nx), -(-4 * (ny + nx) // 256))
         self.part = torch.empty((2, B * self.level_blocks), device=dev)
         probe = torch.empty((B, 1, ny, nx), device=dev)
         self.bed, self.n = model._fields(probe.expand(B, 3, ny, nx))
@@ -95,14 +97,15 @@ class AdjointStepper:
     def _stage2(self, P, U, K1, lv, dt, lam_U):
         """Spatial adjoint at the predictor P (lam_rhs = self.lam_k, the
         adjoint of k2) and the predictor's adjoint in one call: lam_U += ...,
-        self.lam_k = adjoint of k1 (written after the last read of k2's)."""
+        self.lam_k1 = adjoint of k1.  P None: formed from U and K1 on the way."""
         dev_dt = torch.is_tensor(dt)
-        rc = self.lib.swe_adj_stage2_f32(
-            nat.ptr(P), nat.ptr(U), nat.ptr(K1), nat.ptr(self.bed), self.bed.shape[0], self.B, self.ny,
-            self.nx, self.p, nat.ptr(lv), self.levelB, nat.ptr(self.lam_k), nat.ptr(self.cx),
-            nat.ptr(self.cy), 0.0 if dev_dt else float(dt), nat.ptr(dt) if dev_dt else None,
-            nat.ptr(lam_U), nat.ptr(self.lam_k), nat.ptr(self.part[0]), self.level_blocks,
-            nat.ptr(self.lam_bed) if self.bed_grad else None, self.st)
+        args = (nat.ptr(U), nat.ptr(K1), nat.ptr(self.bed), self.bed.shape[0], self.B, self.ny, self.nx,
+                self.p, nat.ptr(lv), self.levelB, nat.ptr(self.lam_k), nat.ptr(self.cx),
+                nat.ptr(self.cy), 0.0 if dev_dt else float(dt), nat.ptr(dt) if dev_dt else None,
+                nat.ptr(lam_U), nat.ptr(self.lam_k1), nat.ptr(self.part[0]), self.level_blocks,
+                nat.ptr(self.lam_bed) if self.bed_grad else None, self.st)
+        rc = (self.lib.swe_adj_stage2_k1_f32(*args) if P is None
+              else self.lib.swe_adj_stage2_f32(nat.ptr(P), *args))
         nat.check(rc, "adjoint spatial operator and predictor (stage 2)")
 
     def bed_adjoint(self):
@@ -141,21 +144,25 @@ class AdjointStepper:
         from the forward recompute (else it is recomputed here); K2 likewise
         the step's stage-2 tendency.  With overwrite, lam_U's previous
         contents are ignored (lam_U = ... rather than +=)."""
-        P, lam_k = self.P, self.lam_k
         # recompute the step's stage intermediates (solver.py:613-646)
         if K1 is None:
+            if self.K1 is None:
+                self.K1 = torch.empty_like(U)
             K1 = self.K1
             self._tendency(U, lv, K1)
-        self._pointwise(2, U, K1, dt, None, None, None, P)
+        P = None
         if K2 is None:
-            K2 = self.K2
+            if self.K2 is None:
+                self.K2, self.P = torch.empty_like(U), torch.empty_like(U)
+            P, K2 = self.P, self.K2
+            self._pointwise(2, U, K1, dt, None, None, None, P)
             self._tendency(P, lv, K2)
         # corrector + friction: lam_k = adjoint of k2
         self._pointwise(3 if overwrite else 0, U, K2, dt, lam_out, lam_U, lam_n, None)
-        # spatial operator at the predictor, then the predictor: lam_k = adjoint of k1
+        # spatial operator at the predictor, then the predictor: lam_k1 = adjoint of k1
         self._stage2(P, U, K1, lv, dt, lam_U)
         # spatial operator at the input state
-        self._spatial(U, lv, lam_k, lam_U, self.part[1], "adjoint spatial operator (stage 1)")
+        self._spatial(U, lv, self.lam_k1, lam_U, self.part[1], "adjoint spatial operator (stage 1)")
         return self.part
 
     def level_adjoint(self, part):

@@ -26,7 +26,7 @@ int adj_args(AdjArgs& a, const float* S, const float* bed, int bedB, int B, int 
              const swe_params* p, const float* level, int levelB, const float* lam_rhs,
              float* scratch_cx, float* scratch_cy, float* level_part, int level_blocks,
              float* lam_bed) {
-    if (!S || !bed || !level || !lam_rhs || !scratch_cx || !scratch_cy || !level_part)
+    if (!bed || !level || !lam_rhs || !scratch_cx || !scratch_cy || !level_part)
         return SWE_EARG;
     if (!valid_params(p) || B < 1 || ny < 2 || nx < 2 || level_blocks < 1) return SWE_EARG;
     if ((bedB != 1 && bedB != B) || (levelB != 1 && levelB != B) || B > 65535) return SWE_EARG;
@@ -35,8 +35,9 @@ int adj_args(AdjArgs& a, const float* S, const float* bed, int bedB, int B, int 
     a.bed = bed;
     a.level = level;
     a.lrhs = lam_rhs;
-    a.cx = scratch_cx;
-    a.cy = scratch_cy;
+    a.gx = scratch_cx;  // 16 B ny floats
+    a.gy = scratch_cy;  // 16 B nx floats, then the frame's planes
+    a.frame = scratch_cy + (size_t)16 * B * nx;
     a.llevel_part = level_part;
     a.lbed = lam_bed;
     a.B = B;
@@ -69,7 +70,7 @@ int adj_spatial(const float* S, const float* bed, int bedB, int B, int ny, int n
     const int rc = adj_args(a, S, bed, bedB, B, ny, nx, p, level, levelB, lam_rhs, scratch_cx,
                             scratch_cy, level_part, level_blocks, lam_bed);
     if (rc != SWE_OK) return rc;
-    if (!lam_S) return SWE_EARG;
+    if (!S || !lam_S) return SWE_EARG;
     a.lS = lam_S;
     return run_spatial(a, p, level_blocks, false, stream);
 }
@@ -94,13 +95,11 @@ extern "C" int swe_adj_spatial_bed_f32(const float* S, const float* bed, int bed
                        lam_S, level_part, level_blocks, lam_bed, stream);
 }
 
-extern "C" int swe_adj_stage2_f32(const float* P, const float* U, const float* k1, const float* bed,
-                                  int bedB, int B, int ny, int nx, const swe_params* p,
-                                  const float* level, int levelB, const float* lam_k2,
-                                  float* scratch_cx, float* scratch_cy, float dt,
-                                  const float* dt_dev, float* lam_U, float* lam_k1,
-                                  float* level_part, int level_blocks, float* lam_bed,
-                                  void* stream) {
+namespace {
+int adj_stage2(const float* P, const float* U, const float* k1, const float* bed, int bedB, int B, int ny,
+               int nx, const swe_params* p, const float* level, int levelB, const float* lam_k2,
+               float* scratch_cx, float* scratch_cy, float dt, const float* dt_dev, float* lam_U,
+               float* lam_k1, float* level_part, int level_blocks, float* lam_bed, void* stream) {
     AdjArgs a;
     const int rc = adj_args(a, P, bed, bedB, B, ny, nx, p, level, levelB, lam_k2, scratch_cx,
                             scratch_cy, level_part, level_blocks, lam_bed);
@@ -112,7 +111,38 @@ extern "C" int swe_adj_stage2_f32(const float* P, const float* U, const float* k
     a.dt_dev = dt_dev;
     a.lU = lam_U;
     a.lk1 = lam_k1;
+    if (lam_k1 == lam_k2) {
+        // blocks write lam_k1 while others still read lam_k2: read a copy, kept
+        // past the ghosts of scratch_cx
+        float* copy = scratch_cx + (size_t)16 * B * ny;
+        if (cudaMemcpyAsync(copy, lam_k2, sizeof(float) * 3 * B * ny * nx, cudaMemcpyDeviceToDevice,
+                            (cudaStream_t)stream) != cudaSuccess)
+            return SWE_ECUDA;
+        a.lrhs = copy;
+    }
     return run_spatial(a, p, level_blocks, true, stream);
+}
+}  // namespace
+
+extern "C" int swe_adj_stage2_f32(const float* P, const float* U, const float* k1, const float* bed,
+                                  int bedB, int B, int ny, int nx, const swe_params* p,
+                                  const float* level, int levelB, const float* lam_k2,
+                                  float* scratch_cx, float* scratch_cy, float dt,
+                                  const float* dt_dev, float* lam_U, float* lam_k1,
+                                  float* level_part, int level_blocks, float* lam_bed,
+                                  void* stream) {
+    if (!P) return SWE_EARG;
+    return adj_stage2(P, U, k1, bed, bedB, B, ny, nx, p, level, levelB, lam_k2, scratch_cx, scratch_cy, dt,
+                      dt_dev, lam_U, lam_k1, level_part, level_blocks, lam_bed, stream);
+}
+
+extern "C" int swe_adj_stage2_k1_f32(const float* U, const float* k1, const float* bed, int bedB, int B,
+                                     int ny, int nx, const swe_params* p, const float* level, int levelB,
+                                     const float* lam_k2, float* scratch_cx, float* scratch_cy, float dt,
+                                     const float* dt_dev, float* lam_U, float* lam_k1,
+                                     float* level_part, int level_blocks, float* lam_bed, void* stream) {
+    return adj_stage2(nullptr, U, k1, bed, bedB, B, ny, nx, p, level, levelB, lam_k2, scratch_cx, scratch_cy,
+                      dt, dt_dev, lam_U, lam_k1, level_part, level_blocks, lam_bed, stream);
 }
 
 namespace {

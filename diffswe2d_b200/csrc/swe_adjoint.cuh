@@ -102,164 +102,180 @@ struct FastMath {
 #endif
 };
 
-// Forward values of one cell kept for the backward pass.
-struct PrimRec {
-    float U0, U1, U2, z;
-    float h, safe, u, v, eta;
-    float rsafe;  // M::rcp(safe): every quotient by safe uses it
-    bool wet;
+// Forward values of one cell: primitive() (riemann.py:20-38) and
+// eta = h + bed (reconstruction.py:23-24).
+struct CellPrim {
+    float h, u, v, eta, z;
 };
 
 template <class M>
-SWE_HD PrimRec prim_rec(float U0, float U1, float U2, float z, const SweConsts& k) {
-    PrimRec p;
-    p.U0 = U0;
-    p.U1 = U1;
-    p.U2 = U2;
-    p.z = z;
+SWE_HD CellPrim cell_prim(float U0, float U1, float U2, float z, const SweConsts& k) {
+    CellPrim p;
     p.h = fmaxf(U0, 0.0f);
-    p.wet = p.h > k.dry;
-    p.safe = fmaxf(p.h, k.floor_h);
-    p.rsafe = M::rcp(p.safe);
-    p.u = p.wet ? M::div(U1, p.safe, p.rsafe) : 0.0f;
-    p.v = p.wet ? M::div(U2, p.safe, p.rsafe) : 0.0f;
+    const bool wet = p.h > k.dry;
+    const float safe = fmaxf(p.h, k.floor_h);
+    const float y = M::rcp(safe);
+    p.u = wet ? M::div(U1, safe, y) : 0.0f;
+    p.v = wet ? M::div(U2, safe, y) : 0.0f;
     p.eta = p.h + z;
+    p.z = z;
     return p;
 }
 
-// Adjoint of primitive() + eta = h + bed (riemann.py:20-38,
-// reconstruction.py:23-24, :71-73): lh includes everything that reached h
-// (directly, via eta and via the reconstruction's own clamp of h).
+// Adjoint of a cell's primitives.
+struct PrimAdj {
+    float h, safe, u, v, z;  // h: of h and of eta = h + z together; z likewise (BEDG only)
+};
+
+// Adjoint of primitive() and of the reconstruction's own clamp of h
+// (riemann.py:20-38, reconstruction.py:71-73).  u0_pass: U0 >= 0.
 template <class M>
-SWE_HD void prim_bwd(const PrimRec& p, float lh, float lsafe, float lu, float lv, float leta,
-                     const SweConsts& k, float& lU0, float& lU1, float& lU2, float& lz) {
-    lh += leta;
-    lz += leta;  // eta = h + bed
-    if (p.wet) {
-        lU1 += M::div(lu, p.safe, p.rsafe);
-        lU2 += M::div(lv, p.safe, p.rsafe);
-        lsafe -= lu * M::div(p.u, p.safe, p.rsafe) + lv * M::div(p.v, p.safe, p.rsafe);
+SWE_HD void prim_bwd(const CellPrim& p, bool u0_pass, const PrimAdj& l, const SweConsts& k, float& lU0,
+                     float& lU1, float& lU2) {
+    const float safe = fmaxf(p.h, k.floor_h);
+    float lh = l.h, lsafe = l.safe;
+    lU1 = lU2 = 0.0f;
+    if (p.h > k.dry) {
+        const float y = M::rcp(safe);
+        lU1 = l.u * y;
+        lU2 = l.v * y;
+        lsafe -= lU1 * p.u + lU2 * p.v;
     }
     if (p.h >= k.floor_h) lh += lsafe;
-    if (p.U0 >= 0.0f) lU0 += lh;
+    lU0 = u0_pass ? lh : 0.0f;
 }
 
-// One side of a cell in one direction (reconstruction.py:26-96) with what
-// the backward pass needs.  plus = true: the "p" side (h + dh/2 ...),
-// false: the "m" side.
-struct SideRec {
-    Incr ih, ie, iz, iu, iv;
-    bool reset;
-    float q, f_raw, f;  // 0.5 dh / safe, factor before and after the clamp
-    Side s;
+// The two face sides of cell c between its neighbours a and b along a line
+// (reconstruction.py:26-96): p faces b, m faces a.
+struct SidePair {
+    Side p, m;
 };
 
+// Sides' increments as the limiter and the bed reset leave them, and the
+// factors of the velocity increments before their clamp.
 template <class M>
-SWE_HD SideRec side_fwd(const PrimRec& a, const PrimRec& c, const PrimRec& b, bool plus,
-                        const SweConsts& k, bool wsr) {
-    SideRec r;
-    r.ih = incr_fwd(a.h, c.h, b.h, k.theta);
-    r.ie = incr_fwd(a.eta, c.eta, b.eta, k.theta);
-    r.iz = incr_fwd(a.z, c.z, b.z, k.theta);
-    r.iu = incr_fwd(a.u, c.u, b.u, k.theta);
-    r.iv = incr_fwd(a.v, c.v, b.v, k.theta);
-    const float dh = r.ih.val, dz = r.iz.val;
-    float deta = r.ie.val;
-    r.reset = false;
+SWE_HD SidePair side_pair(const CellPrim& a, const CellPrim& c, const CellPrim& b, const SweConsts& k, bool wsr) {
+    const float dh = limited_increment(a.h, c.h, b.h, k.theta);
+    float de = limited_increment(a.eta, c.eta, b.eta, k.theta);
+    const float dz = limited_increment(a.z, c.z, b.z, k.theta);
+    const float du = limited_increment(a.u, c.u, b.u, k.theta);
+    const float dv = limited_increment(a.v, c.v, b.v, k.theta);
     if (wsr) {
-        const float half = 0.5f * (deta - dh);
-        const float base = c.eta - c.h;
-        const float bm = base - half, bp = base + half;
-        r.reset = (deta * deta > dz * dz) && ((bm > a.eta) || (bp > b.eta));
-        if (r.reset) deta = dh + dz;
+        const float half = 0.5f * (de - dh), base = c.eta - c.h;
+        if ((de * de > dz * dz) && ((base - half > a.eta) || (base + half > b.eta))) de = dh + dz;
     }
-    const float hdh = 0.5f * dh;
-    r.q = M::div(hdh, c.safe, c.rsafe);
-    if (plus) {
-        r.s.hlin = c.h + hdh;
-        r.s.eta = c.eta + 0.5f * deta;
-        r.s.bed = c.z + 0.5f * dz;
-        r.f_raw = c.h > k.dry ? 1.0f - r.q : 1.0f;
-    } else {
-        r.s.hlin = c.h - hdh;
-        r.s.eta = c.eta - 0.5f * deta;
-        r.s.bed = c.z - 0.5f * dz;
-        r.f_raw = c.h > k.dry ? 1.0f + r.q : 1.0f;
-    }
-    r.f = fminf(fmaxf(r.f_raw, -10.0f), 10.0f);
-    const float hf = 0.5f * r.f;
-    if (plus) {
-        r.s.u = c.u + hf * r.iu.val;
-        r.s.v = c.v + hf * r.iv.val;
-    } else {
-        r.s.u = c.u - hf * r.iu.val;
-        r.s.v = c.v - hf * r.iv.val;
-    }
-    return r;
+    const float hdh = 0.5f * dh, hde = 0.5f * de, hdz = 0.5f * dz;
+    const float safe = fmaxf(c.h, k.floor_h);
+    const float q = M::div(hdh, safe, M::rcp(safe));
+    const bool wet = c.h > k.dry;
+    const float fp = 0.5f * fminf(fmaxf(wet ? 1.0f - q : 1.0f, -10.0f), 10.0f);
+    const float fm = 0.5f * fminf(fmaxf(wet ? 1.0f + q : 1.0f, -10.0f), 10.0f);
+    SidePair s;
+    s.p.hlin = c.h + hdh;
+    s.m.hlin = c.h - hdh;
+    s.p.eta = c.eta + hde;
+    s.m.eta = c.eta - hde;
+    s.p.bed = c.z + hdz;
+    s.m.bed = c.z - hdz;
+    s.p.u = c.u + fp * du;
+    s.p.v = c.v + fp * dv;
+    s.m.u = c.u - fm * du;
+    s.m.v = c.v - fm * dv;
+    return s;
 }
 
-// Adjoints of the three cells' primitives (h, safe, u, v, eta per cell).
-struct PrimAdj {
-    float h, safe, u, v, eta, z;
+// Adjoint of one face side of a cell, with the terms that reach the cell's
+// depth (and bed) directly through the face's source.
+struct SideAdj {
+    float hlin, eta, u, v;
+    float dh;       // of the cell's h (source)
+    float bed, dz;  // of the side's bed and of the cell's bed (BEDG only)
 };
 
+// Contributions of a cell's two sides to the adjoints of its primitives and
+// of its neighbours' (h: of h and eta together, z: of z and eta together).
+struct LineAdj {
+    float h, u, v, z;
+};
+
+// Adjoint of side_pair() for the cotangents lp, lm of its two sides.  Each
+// increment's share of the three values is formed once for both sides.
+// Quotients by the safe depth are products with its reciprocal here (the
+// cotangent's rounding; no branch depends on them).
 template <bool BEDG, class M>
-SWE_HD void side_bwd(const SideRec& r, const PrimRec& c, bool plus, float l_hlin, float l_eta,
-                     float l_u, float l_v, float l_bed, const SweConsts& k, PrimAdj& la,
-                     PrimAdj& lc, PrimAdj& lb) {
-    const float sg = plus ? 1.0f : -1.0f;
-    // u_side = u +/- (0.5 f) du ; v likewise
-    const float hf = 0.5f * r.f;
-    lc.u += l_u;
-    lc.v += l_v;
-    float l_du = sg * (l_u * hf);
-    float l_dv = sg * (l_v * hf);
-    float l_hf = sg * (l_u * r.iu.val + l_v * r.iv.val);
-    float l_f = 0.5f * l_hf;
+SWE_HD void side_pair_bwd(const CellPrim& a, const CellPrim& c, const CellPrim& b, const SideAdj& lp,
+                          const SideAdj& lm, const SweConsts& k, bool wsr, LineAdj& left, PrimAdj& own,
+                          LineAdj& right) {
+    const Incr ih = incr_fwd(a.h, c.h, b.h, k.theta);
+    const Incr ie = incr_fwd(a.eta, c.eta, b.eta, k.theta);
+    const Incr iz = incr_fwd(a.z, c.z, b.z, k.theta);
+    bool reset = false;
+    if (wsr) {
+        const float half = 0.5f * (ie.val - ih.val), base = c.eta - c.h;
+        reset = (ie.val * ie.val > iz.val * iz.val) && ((base - half > a.eta) || (base + half > b.eta));
+    }
+    const float safe = fmaxf(c.h, k.floor_h), y = M::rcp(safe);
+    const float q = M::div(0.5f * ih.val, safe, y);
+    const bool wet = c.h > k.dry;
+    const float rp = wet ? 1.0f - q : 1.0f, rm = wet ? 1.0f + q : 1.0f;  // before the clamp
+    const float fp = 0.5f * fminf(fmaxf(rp, -10.0f), 10.0f), fm = 0.5f * fminf(fmaxf(rm, -10.0f), 10.0f);
+    left.h = right.h = left.z = right.z = 0.0f;
+    own.h = lp.hlin + lm.hlin + lp.dh + lm.dh + lp.eta + lm.eta;
+    own.z = BEDG ? lp.bed + lm.bed + lp.dz + lm.dz + lp.eta + lm.eta : 0.0f;
+    // u_side = u +/- (factor / 2) du ; v likewise
+    own.u = lp.u + lm.u;
+    own.v = lp.v + lm.v;
+    float l_fp, l_fm;
+    {
+        const Incr iu = incr_fwd(a.u, c.u, b.u, k.theta), iv = incr_fwd(a.v, c.v, b.v, k.theta);
+        left.u = right.u = left.v = right.v = 0.0f;
+        incr_bwd(iu, lp.u * fp - lm.u * fm, k.theta, left.u, own.u, right.u);
+        incr_bwd(iv, lp.v * fp - lm.v * fm, k.theta, left.v, own.v, right.v);
+        l_fp = 0.5f * (lp.u * iu.val + lp.v * iv.val);
+        l_fm = -0.5f * (lm.u * iu.val + lm.v * iv.val);
+    }
     // clamp(-10, 10) then where(h > dry, 1 -/+ q, 1)
-    float l_fraw = (r.f_raw >= -10.0f && r.f_raw <= 10.0f) ? l_f : 0.0f;
-    float l_q = c.h > k.dry ? -sg * l_fraw : 0.0f;
-    // q = (0.5 dh) / safe
-    float l_dh = 0.5f * M::div(l_q, c.safe, c.rsafe);
-    lc.safe -= l_q * M::div(r.q, c.safe, c.rsafe);
-    // hlin = h +/- 0.5 dh ; eta_side = eta +/- 0.5 deta
-    lc.h += l_hlin;
-    l_dh += sg * (0.5f * l_hlin);
-    lc.eta += l_eta;
-    float l_deta = sg * (0.5f * l_eta);
-    float l_dz = 0.0f;
-    if (BEDG) {  // bed_side = bed +/- 0.5 dz
-        lc.z += l_bed;
-        l_dz = sg * (0.5f * l_bed);
+    float l_q = 0.0f;
+    if (wet) {
+        if (rp >= -10.0f && rp <= 10.0f) l_q -= l_fp;
+        if (rm >= -10.0f && rm <= 10.0f) l_q += l_fm;
     }
-    if (r.reset) {  // deta = dh + dz
-        l_dh += l_deta;
-        if (BEDG) l_dz += l_deta;
-        l_deta = 0.0f;
+    // q = (dh / 2) / safe
+    const float l_qy = l_q * y;
+    own.safe = -l_qy * q;
+    float l_dh = 0.5f * (l_qy + lp.hlin - lm.hlin);
+    float l_de = 0.5f * (lp.eta - lm.eta);
+    float l_dz = BEDG ? 0.5f * (lp.bed - lm.bed) : 0.0f;
+    if (reset) {  // deta = dh + dz
+        l_dh += l_de;
+        if (BEDG) l_dz += l_de;
+        l_de = 0.0f;
     }
-    if (BEDG) incr_bwd(r.iz, l_dz, k.theta, la.z, lc.z, lb.z);
-    incr_bwd(r.ih, l_dh, k.theta, la.h, lc.h, lb.h);
-    incr_bwd(r.ie, l_deta, k.theta, la.eta, lc.eta, lb.eta);
-    incr_bwd(r.iu, l_du, k.theta, la.u, lc.u, lb.u);
-    incr_bwd(r.iv, l_dv, k.theta, la.v, lc.v, lb.v);
+    incr_bwd(ih, l_dh, k.theta, left.h, own.h, right.h);
+    float el = 0.0f, eo = 0.0f, er = 0.0f;
+    incr_bwd(ie, l_de, k.theta, el, eo, er);
+    left.h += el;
+    own.h += eo;
+    right.h += er;
+    if (BEDG) {
+        incr_bwd(iz, l_dz, k.theta, left.z, own.z, right.z);
+        left.z += el;
+        own.z += eo;
+        right.z += er;
+    }
 }
 
-// Adjoint of the face function for cells (p0, p1 | p2, p3) along a line: the
-// face lies between p1 and p2.  Inputs: adjoints of the face outputs
-// (mass flux, normal flux minus source_L, normal flux minus source_R,
-// tangential flux).  Outputs: adjoints of (U0, U1, U2) of the four cells.
-struct CellAdj {
-    float U0, U1, U2, Z;  // Z: adjoint of the cell's bed (BEDG only)
-};
-
+// Adjoint of one face between cells of depths h1, h2 and beds z1, z2 with
+// sides Lp and Rm (reconstruction.py:59-106, riemann.py:41-105): from the
+// adjoints of the face outputs (mass flux, normal flux minus source_L,
+// normal flux minus source_R, tangential flux) to those of the two sides.
+// The forward part is the step's, operation for operation (its comparisons
+// decide the branches); the cotangents' quotients are products with
+// reciprocals.
 template <bool BEDG, class M>
-SWE_HD void face_vjp(const PrimRec P[4], float l_mass, float l_nL, float l_nR, float l_tan,
-                     bool normal_y, const SweConsts& k, bool wsr, CellAdj out[4]) {
-    // ---- forward: sides of p1 ("p") and p2 ("m")
-    const SideRec SL_ = side_fwd<M>(P[0], P[1], P[2], true, k, wsr);
-    const SideRec SR_ = side_fwd<M>(P[1], P[2], P[3], false, k, wsr);
-    const Side& Lp = SL_.s;
-    const Side& Rm = SR_.s;
+SWE_HD void face_adj(const Side& Lp, float h1, float z1, const Side& Rm, float h2, float z2, float l_mass,
+                     float l_nL, float l_nR, float l_tan, bool normal_y, const SweConsts& k, SideAdj& lL,
+                     SideAdj& lR) {
     // face reconstruction (reconstruction.py:59-106)
     const float baud = fmaxf(Lp.bed, Rm.bed);
     const float inner = fminf(Lp.eta, Rm.eta);
@@ -268,8 +284,8 @@ SWE_HD void face_vjp(const PrimRec P[4], float l_mass, float l_nL, float l_nR, f
     const float mL = fminf(AL, Lp.hlin), mR = fminf(AR, Rm.hlin);
     const float hcL = fmaxf(mL, 0.0f), hcR = fmaxf(mR, 0.0f);
     const float UL1 = hcL * Lp.u, UL2 = hcL * Lp.v, UR1 = hcR * Rm.u, UR2 = hcR * Rm.v;
-    const float sL1 = k.half_g * (P[1].h + hcL), sL2 = P[1].z - bcn;
-    const float sR1 = k.half_g * (hcR + P[2].h), sR2 = P[2].z - bcn;
+    const float sL1 = k.half_g * (h1 + hcL), sL2 = z1 - bcn;
+    const float sR1 = k.half_g * (hcR + h2), sR2 = z2 - bcn;
     // HLL (riemann.py:57-105)
     const float hL = fmaxf(hcL, 0.0f), hR = fmaxf(hcR, 0.0f);
     const bool wetL = hL > k.dry, wetR = hR > k.dry;
@@ -327,8 +343,8 @@ SWE_HD void face_vjp(const PrimRec P[4], float l_mass, float l_nL, float l_nR, f
         l_fqs = l_fq;
     }
     // fhs = numh / den, fqs = numq / den
-    const float l_numh = M::div(l_fhs, den, yden), l_numq = M::div(l_fqs, den, yden);
-    const float l_den = -(l_fhs * M::div(fhs, den, yden)) - l_fqs * M::div(fqs, den, yden);
+    const float l_numh = l_fhs * yden, l_numq = l_fqs * yden;
+    const float l_den = -l_numh * fhs - l_numq * fqs;
     float l_SL = 0.0f, l_SR = 0.0f, l_hL = 0.0f, l_hR = 0.0f, l_unL = 0.0f, l_unR = 0.0f;
     float l_cL = 0.0f, l_cR = 0.0f;
     // numh = (SR fhL - SL fhR) + SLSR (hR - hL)
@@ -409,18 +425,16 @@ SWE_HD void face_vjp(const PrimRec P[4], float l_mass, float l_nL, float l_nR, f
     // primitive() of the face states
     float l_UL1 = 0.0f, l_UL2 = 0.0f, l_UR1 = 0.0f, l_UR2 = 0.0f, l_safeL = 0.0f, l_safeR = 0.0f;
     if (wetL) {
-        l_UL1 = M::div(l_uL, safeL, ysL);
-        l_UL2 = M::div(l_vL, safeL, ysL);
-        l_safeL -= l_uL * M::div(uL, safeL, ysL) + l_vL * M::div(vL, safeL, ysL);
-        const float c2 = 2.0f * cL;
-        l_safeL += k.g * M::div(l_cL, c2, M::rcp(c2));
+        l_UL1 = l_uL * ysL;
+        l_UL2 = l_vL * ysL;
+        l_safeL -= l_UL1 * uL + l_UL2 * vL;
+        l_safeL += (k.half_g * l_cL) * M::rcp(cL);  // c = sqrt(g safe)
     }
     if (wetR) {
-        l_UR1 = M::div(l_uR, safeR, ysR);
-        l_UR2 = M::div(l_vR, safeR, ysR);
-        l_safeR -= l_uR * M::div(uR, safeR, ysR) + l_vR * M::div(vR, safeR, ysR);
-        const float c2 = 2.0f * cR;
-        l_safeR += k.g * M::div(l_cR, c2, M::rcp(c2));
+        l_UR1 = l_uR * ysR;
+        l_UR2 = l_vR * ysR;
+        l_safeR -= l_UR1 * uR + l_UR2 * vR;
+        l_safeR += (k.half_g * l_cR) * M::rcp(cR);  // c = sqrt(g safe)
     }
     if (hL >= k.floor_h) l_hL += l_safeL;
     if (hR >= k.floor_h) l_hR += l_safeR;
@@ -433,19 +447,20 @@ SWE_HD void face_vjp(const PrimRec P[4], float l_mass, float l_nL, float l_nR, f
     const float l_Ru = l_UR1 * hcR, l_Rv = l_UR2 * hcR;
     // sources: srcL = (g/2 (h1 + hcL)) (z1 - bcn)
     float l_bcn = 0.0f;
-    PrimAdj la[4] = {};
+    lL = SideAdj{};
+    lR = SideAdj{};
     {
         const float l_s1 = l_srcL * sL2;
         l_bcn -= l_srcL * sL1;
-        la[1].h += k.half_g * l_s1;
+        lL.dh = k.half_g * l_s1;
         l_hcL += k.half_g * l_s1;
         const float l_s2 = l_srcR * sR2;
         l_bcn -= l_srcR * sR1;
-        la[2].h += k.half_g * l_s2;
+        lR.dh = k.half_g * l_s2;
         l_hcR += k.half_g * l_s2;
         if (BEDG) {  // srcL = (g/2 (h1 + hcL)) (z1 - bcn), srcR likewise with z2
-            la[1].z += l_srcL * sL1;
-            la[2].z += l_srcR * sR1;
+            lL.dz = l_srcL * sL1;
+            lR.dz = l_srcR * sR1;
         }
     }
     // hc = clamp(min(eta_side - bcn, hlin), min=0)
@@ -472,15 +487,16 @@ SWE_HD void face_vjp(const PrimRec P[4], float l_mass, float l_nL, float l_nR, f
     minmax_shares(Lp.eta, Rm.eta, false, sa, sb);
     l_Leta += l_inner * sa;
     l_Reta += l_inner * sb;
-    // sides -> primitives of the four cells
-    side_bwd<BEDG, M>(SL_, P[1], true, l_Lhlin, l_Leta, l_Lu, l_Lv, l_Lbed, k, la[0], la[1], la[2]);
-    side_bwd<BEDG, M>(SR_, P[2], false, l_Rhlin, l_Reta, l_Ru, l_Rv, l_Rbed, k, la[1], la[2], la[3]);
-    for (int i = 0; i < 4; ++i) {
-        out[i].U0 = out[i].U1 = out[i].U2 = 0.0f;
-        out[i].Z = la[i].z;  // sources, increments, face beds; prim_bwd adds the eta term
-        prim_bwd<M>(P[i], la[i].h, la[i].safe, la[i].u, la[i].v, la[i].eta, k, out[i].U0, out[i].U1,
-                 out[i].U2, out[i].Z);
-    }
+    lL.hlin = l_Lhlin;
+    lL.eta = l_Leta;
+    lL.u = l_Lu;
+    lL.v = l_Lv;
+    lL.bed = l_Lbed;
+    lR.hlin = l_Rhlin;
+    lR.eta = l_Reta;
+    lR.u = l_Ru;
+    lR.v = l_Rv;
+    lR.bed = l_Rbed;
 }
 
 }  // namespace swe

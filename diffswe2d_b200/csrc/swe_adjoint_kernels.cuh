@@ -3,19 +3,23 @@
 // ExactMath in swe_adjoint.cu (IEEE flags) and with FastMath in
 // swe_adjoint_fast.cu (compiled like the tolerance-mode step).
 //
-// The spatial-operator adjoint is two launches: adj_face_kernel, one thread
-// per face (x faces, then y faces, in one grid), computes the face's reverse
-// mode (swe_adjoint.cuh) and writes its contributions to its four stencil
-// cells into face-record planes; adj_gather_kernel, one thread per cell,
-// sums them in a fixed order and folds the adjoints of ghost cells back into
-// the interior cells and boundary level they were made from (the adjoint of
-// add_ghost_cells, src/boundary.py:150-413), and, for stage 2, goes on
-// through the predictor's adjoint.  No float atomics: results are
-// deterministic.
+// The spatial-operator adjoint is two launches.  adj_tile_kernel owns a tile
+// of cells per block and keeps everything between the state and its adjoint
+// in shared memory: primitives of the tile and a three-cell halo, the face
+// sides of its cells in both directions, the reverse mode of each face
+// (swe_adjoint.cuh) written over the sides it read, each cell's reverse mode
+// of its two sides written over those, and their sums.  The adjoints of
+// ghost cells go to a small buffer; adj_edge_kernel folds them back into the
+// cells and boundary level they were made from (the adjoint of
+// add_ghost_cells, src/boundary.py:150-413) and finishes the two-cell frame
+// along the sides.  Stage 2 goes on through the predictor's adjoint in both.
+// No float atomics: results are deterministic.
 #pragma once
 
 #include <cuda_runtime.h>
 #include <stdint.h>
+
+#include <atomic>
 
 #include "swe_adjoint.cuh"
 #include "swe_common.cuh"
@@ -23,25 +27,24 @@
 namespace swe {
 
 constexpr int ADJ_THREADS = 256;
-// Blocks per SM the kernels are compiled for (register budgets): the face
-// kernel at three (80 registers, a few hundred bytes of spills) measured
-// 2.5-9 % faster per inversion iteration than at two (no spills) and 3 %
-// faster than at four; the gather kernel is memory-latency bound and runs
-// 7 % faster per adjoint step at eight (32 registers) than at three.
-#ifndef SWE_ADJ_FACE_MINB
-#define SWE_ADJ_FACE_MINB 3
-#endif
-#ifndef SWE_ADJ_GATHER_MINB
-#define SWE_ADJ_GATHER_MINB 8
+constexpr int ADJ_TX = 32;  // tile columns
+// Blocks per SM the tile kernel is compiled for (80 registers, no spills).
+// Measured with 16-row tiles at 4 x 244 x 393, stage 2 / stage 1: three
+// 58.5 / 52.0 us, two 69 / 60; with 8-row tiles (37 KB instead of 65) at
+// three, four and five blocks 67 / 59, 64 / 57 and 66 / 59.
+#ifndef SWE_ADJ_TILE_MINB
+#define SWE_ADJ_TILE_MINB 3
 #endif
 
 struct AdjArgs {
-    const float* S;      // state whose tendency is differentiated, [B,3,ny,nx]
+    const float* S;      // state whose tendency is differentiated, [B,3,ny,nx]; with the
+                         // predictor fused in: P, or null to form it from U and k1
     const float* bed;    // [bedB,1,ny,nx]
     const float* level;  // [levelB]
     const float* lrhs;   // adjoint of the tendency, [B,3,ny,nx]
-    float* cx;           // x-face contributions [12 or 16 planes][B][ny][nx+1]
-    float* cy;           // y-face contributions [12 or 16 planes][B][ny+1][nx]
+    float* gx;           // adjoints of the x ghosts [B][left, right][1st, 2nd][ny][4]
+    float* gy;           // adjoints of the y ghosts [B][top, bottom][1st, 2nd][nx][4]
+    float* frame;        // adjoints of the frame's cells before the folds [B][3 or 4][ny][nx]
     float* lS;           // adjoint of S, accumulated (+=)
     float* llevel_part;  // per-block partial level adjoints [B][gridDim.x]
     float* lbed;         // adjoint of the bed [B,ny,nx], accumulated (+=); BEDG only
@@ -50,9 +53,9 @@ struct AdjArgs {
     float cval;
     int wsr;
     SweConsts kc;
-    // Predictor adjoint fused into the gather (adj_gather_kernel with PRED;
-    // S is then the predictor P = clean(U, U + dt/2 k1)): the cell's adjoint
-    // of P is not stored but taken through the clean-up's adjoint at once.
+    // Predictor adjoint fused in (PRED; S is then the predictor
+    // P = clean(U, U + dt/2 k1)): the cell's adjoint of P is not stored but
+    // taken through the clean-up's adjoint at once.
     const float* U;       // step input [B,3,ny,nx]
     const float* k1;      // stage-1 tendency [B,3,ny,nx]
     const float* dt_dev;  // the step's dt in device memory, or null: dt
@@ -86,266 +89,6 @@ __device__ __forceinline__ size_t a3(int b, int c, int j, int i, int ny, int nx)
 
 __device__ __forceinline__ float bed_of(const AdjArgs& a, int b, int j, int i) {
     return a.bed[((size_t)(a.bedB == 1 ? 0 : b) * a.ny + j) * a.nx + i];
-}
-
-// Padded cell (j, i) of S with the ghost rules (arm cells only; corners are
-// never part of an interior face's stencil).
-template <class M>
-__device__ PrimRec padded_prim(const AdjArgs& a, int b, int j, int i) {
-    const int ny = a.ny, nx = a.nx;
-    const bool jin = (unsigned)j < (unsigned)ny, iin = (unsigned)i < (unsigned)nx;
-    int js = min(max(j, 0), ny - 1), is = min(max(i, 0), nx - 1);
-    const bool xarm = jin && !iin, yarm = iin && !jin;
-    int code = -1, side = 0;
-    if (xarm || yarm) {
-        side = xarm ? (i < 0 ? 0 : 1) : (j < 0 ? 2 : 3);
-        code = a.bc[side];
-        if (code == SWE_BC_PERIODIC) {
-            if (xarm) is = i < 0 ? nx + i : i - nx;
-            else js = j < 0 ? ny + j : j - ny;
-        }
-    }
-    const size_t plane = (size_t)ny * nx;
-    const size_t o = a3(b, 0, js, is, ny, nx);
-    float U0 = a.S[o], U1 = a.S[o + plane], U2 = a.S[o + 2 * plane];
-    const float z = bed_of(a, b, js, is);
-    const float lev = a.level[a.levelB == 1 ? 0 : b];
-    if (code == SWE_BC_CONSTANT) {
-        U0 = U1 = U2 = a.cval;
-    } else if (code == SWE_BC_WATER_LEVEL) {
-        U0 = fmaxf(lev - z, 0.0f);
-    } else if (code == SWE_BC_WALL) {
-        const int jm = xarm ? j : (j < 0 ? -1 - j : 2 * ny - 1 - j);
-        const int im = xarm ? (i < 0 ? -1 - i : 2 * nx - 1 - i) : i;
-        const size_t om = a3(b, xarm ? 1 : 2, jm, im, ny, nx);
-        if (xarm) U1 = -a.S[om];
-        else U2 = -a.S[om];
-    } else if (code == SWE_BC_ABSORBING) {
-        const float hr = fmaxf(lev - z, 0.0f);
-        const float hg = U0;
-        const float hc = hr > a.kc.absorb_lim ? hr : hg;
-        const float c = M::sqrt(a.kc.g981 * fmaxf(hc, a.kc.absorb_min));
-        const float val = ((side == 0 || side == 2) ? -c : c) * (hg - hr);
-        if (xarm) U1 = val;
-        else U2 = val;
-    }
-    return prim_rec<M>(U0, U1, U2, z, a.kc);
-}
-
-// Face records: 4 cells x (U0, U1, U2[, Z]) floats per face, stored as
-// planes (plane p = cell * C + channel, C = 3 or 4; within a plane, face t of
-// the launch at t) so that consecutive faces' writes and consecutive cells'
-// reads are coalesced.
-template <bool BEDG>
-__host__ __device__ constexpr int rec_floats() { return BEDG ? 16 : 12; }
-
-__device__ __forceinline__ size_t xfaces(const AdjArgs& a) { return (size_t)a.B * a.ny * (a.nx + 1); }
-__device__ __forceinline__ size_t yfaces(const AdjArgs& a) { return (size_t)a.B * (a.ny + 1) * a.nx; }
-
-// Faces of one direction, one thread per face, over blocks [blk, blk + nblk)
-// of the launch.
-template <bool DIRY, bool BEDG, class M>
-__device__ __forceinline__ void face_dir(const AdjArgs& a, int blk, int nblk) {
-    const int ny = a.ny, nx = a.nx;
-    const long long nfaces = DIRY ? (long long)(ny + 1) * nx : (long long)ny * (nx + 1);
-    const long long total = nfaces * a.B;
-    const size_t plane = (size_t)ny * nx;
-    for (long long t = blk * (long long)blockDim.x + threadIdx.x; t < total;
-         t += (long long)nblk * blockDim.x) {
-        const int b = (int)(t / nfaces);
-        const long long r = t - (long long)b * nfaces;
-        int row, f;  // x: row j, face f in [0, nx]; y: face f in [0, ny], column i (row var)
-        if (DIRY) {
-            f = (int)(r / nx);
-            row = (int)(r - (long long)f * nx);
-        } else {
-            row = (int)(r / (nx + 1));
-            f = (int)(r - (long long)row * (nx + 1));
-        }
-        PrimRec P[4];
-        if (f >= 2 && f <= (DIRY ? ny : nx) - 2) {  // the stencil's four cells are interior
-            const size_t o0 = DIRY ? a3(b, 0, f - 2, row, ny, nx) : a3(b, 0, row, f - 2, ny, nx);
-            const size_t z0 = DIRY ? ((size_t)(a.bedB == 1 ? 0 : b) * ny + (f - 2)) * nx + row
-                                   : ((size_t)(a.bedB == 1 ? 0 : b) * ny + row) * nx + (f - 2);
-            const size_t step = DIRY ? (size_t)nx : 1;
-            for (int s = 0; s < 4; ++s) {
-                const size_t o = o0 + s * step;
-                P[s] = prim_rec<M>(a.S[o], a.S[o + plane], a.S[o + 2 * plane], a.bed[z0 + s * step], a.kc);
-            }
-        } else {
-            for (int s = 0; s < 4; ++s)
-                P[s] = DIRY ? padded_prim<M>(a, b, f - 2 + s, row) : padded_prim<M>(a, b, row, f - 2 + s);
-        }
-        // adjoints of the face outputs from the tendencies of the two cells
-        // sharing the face: (F_right(f) - F_left(f+1)) / d
-        const float d = DIRY ? a.kc.dy : a.kc.dx;
-        const float rd = DIRY ? a.kc.rdy : a.kc.rdx;  // RN(1/d): lrhs / d below is exact RN
-        const int n = DIRY ? ny : nx;
-        float r0p = 0.0f, r1p = 0.0f, r2p = 0.0f, r0m = 0.0f, r1m = 0.0f, r2m = 0.0f;
-        if (f < n) {  // cell f: this face is its left/top face
-            const size_t o = DIRY ? a3(b, 0, f, row, ny, nx) : a3(b, 0, row, f, ny, nx);
-            r0p = M::div(a.lrhs[o], d, rd);
-            r1p = M::div(a.lrhs[o + plane], d, rd);
-            r2p = M::div(a.lrhs[o + 2 * plane], d, rd);
-        }
-        if (f >= 1) {  // cell f-1: this face is its right/bottom face
-            const size_t o = DIRY ? a3(b, 0, f - 1, row, ny, nx) : a3(b, 0, row, f - 1, ny, nx);
-            r0m = M::div(a.lrhs[o], d, rd);
-            r1m = M::div(a.lrhs[o + plane], d, rd);
-            r2m = M::div(a.lrhs[o + 2 * plane], d, rd);
-        }
-        const float l_mass = r0p - r0m;
-        // x: channel 1 normal, 2 tangential; y: channel 1 tangential, 2 normal
-        const float l_nR = DIRY ? r2p : r1p;
-        const float l_nL = DIRY ? -r2m : -r1m;
-        const float l_tan = DIRY ? (r1p - r1m) : (r2p - r2m);
-        CellAdj out[4];
-        face_vjp<BEDG, M>(P, l_mass, l_nL, l_nR, l_tan, DIRY, a.kc, a.wsr != 0, out);
-        constexpr int C = BEDG ? 4 : 3;
-        const size_t np = DIRY ? yfaces(a) : xfaces(a);
-        float* dst = (DIRY ? a.cy : a.cx) + t;
-        for (int s = 0; s < 4; ++s) {
-            dst[(C * s) * np] = out[s].U0;
-            dst[(C * s + 1) * np] = out[s].U1;
-            dst[(C * s + 2) * np] = out[s].U2;
-            if (BEDG) dst[(C * s + 3) * np] = out[s].Z;
-        }
-    }
-}
-
-// The x faces on the first xblocks blocks, the y faces on the rest.
-template <bool BEDG, class M>
-__global__ void __launch_bounds__(ADJ_THREADS, SWE_ADJ_FACE_MINB) adj_face_kernel(const AdjArgs a, int xblocks) {
-    chain_start();
-    if ((int)blockIdx.x < xblocks) face_dir<false, BEDG, M>(a, blockIdx.x, xblocks);
-    else face_dir<true, BEDG, M>(a, blockIdx.x - xblocks, gridDim.x - xblocks);
-}
-
-// Sum of the face contributions to padded cell (row j, column col) along x
-// (l[3], the bed channel, with BEDG only).
-template <bool BEDG>
-__device__ void lam_x(const AdjArgs& a, int b, int j, int col, float l[4]) {
-    constexpr int C = BEDG ? 4 : 3;
-    const size_t np = xfaces(a);
-    l[0] = l[1] = l[2] = l[3] = 0.0f;
-    for (int f = col - 1; f <= col + 2; ++f) {
-        if (f < 0 || f > a.nx) continue;
-        const float* c = a.cx + (((size_t)b * a.ny + j) * (a.nx + 1) + f) + C * (col - f + 2) * np;
-        l[0] += c[0];
-        l[1] += c[np];
-        l[2] += c[2 * np];
-        if (BEDG) l[3] += c[3 * np];
-    }
-}
-
-template <bool BEDG>
-__device__ void lam_y(const AdjArgs& a, int b, int row, int i, float l[4]) {
-    constexpr int C = BEDG ? 4 : 3;
-    const size_t np = yfaces(a);
-    l[0] = l[1] = l[2] = l[3] = 0.0f;
-    for (int f = row - 1; f <= row + 2; ++f) {
-        if (f < 0 || f > a.ny) continue;
-        const float* c = a.cy + (((size_t)b * (a.ny + 1) + f) * a.nx + i) + C * (row - f + 2) * np;
-        l[0] += c[0];
-        l[1] += c[np];
-        l[2] += c[2 * np];
-        if (BEDG) l[3] += c[3 * np];
-    }
-}
-
-// Folds the adjoint lg of ghost g (side `side`; g its column for left/right,
-// row for top/bottom) into cell (j, i) if the ghost was made from it, and
-// adds the level adjoint once per ghost (in the thread of the ghost's
-// clamped source cell).  BEDG: lg[3] is the ghost's bed adjoint, folded into
-// the cell its bed was copied from (replicate, or periodic), plus the bed
-// terms of the forced ghost depth max(level - z, 0) -> lzc.
-template <bool BEDG, class M>
-__device__ void fold_ghost(const AdjArgs& a, int b, int side, int g, const float lg[4], int j,
-                           int i, float lam[3], float& llev, float& lzc) {
-    const int ny = a.ny, nx = a.nx;
-    const bool xs = side < 2;
-    const int n = xs ? nx : ny;
-    const int pos = xs ? i : j;  // this cell's index along the side's direction
-    const int clamp_src = g < 0 ? 0 : n - 1;
-    const int mirror = g < 0 ? -1 - g : 2 * n - 1 - g;
-    const int periodic = g < 0 ? n + g : g - n;
-    const int normal = xs ? 1 : 2;  // momentum channel reflected by a wall
-    const int code = a.bc[side];
-    if (BEDG && pos == (code == SWE_BC_PERIODIC ? periodic : clamp_src)) lzc += lg[3];
-    switch (code) {
-    case SWE_BC_TRANSMISSIVE:
-        if (pos == clamp_src) {
-            lam[0] += lg[0];
-            lam[1] += lg[1];
-            lam[2] += lg[2];
-        }
-        break;
-    case SWE_BC_PERIODIC:
-        if (pos == periodic) {
-            lam[0] += lg[0];
-            lam[1] += lg[1];
-            lam[2] += lg[2];
-        }
-        break;
-    case SWE_BC_CONSTANT:
-        break;
-    case SWE_BC_WATER_LEVEL:
-        if (pos == clamp_src) {
-            lam[1] += lg[1];
-            lam[2] += lg[2];
-            const float z = bed_of(a, b, xs ? j : clamp_src, xs ? clamp_src : i);
-            const float lev = a.level[a.levelB == 1 ? 0 : b];
-            if (lev - z >= 0.0f) {  // clamp(level - z, min=0)
-                llev += lg[0];
-                if (BEDG) lzc -= lg[0];
-            }
-        }
-        break;
-    case SWE_BC_WALL:
-        if (pos == clamp_src) {
-            lam[0] += lg[0];
-            lam[3 - normal] += lg[3 - normal];
-        }
-        if (pos == mirror) lam[normal] -= lg[normal];
-        break;
-    case SWE_BC_ABSORBING:
-        if (pos == clamp_src) {
-            lam[3 - normal] += lg[3 - normal];
-            lam[0] += lg[0];
-            // value = s c (hg - hr), hr = max(level - z, 0),
-            // c = sqrt(9.81 max(where(hr > 1e-4, hr, hg), 1e-6))
-            const size_t plane = (size_t)ny * nx;
-            const int jj = xs ? j : clamp_src, ii = xs ? clamp_src : i;
-            const float hg = a.S[a3(b, 0, jj, ii, ny, nx)];
-            (void)plane;
-            const float z = bed_of(a, b, jj, ii);
-            const float lev = a.level[a.levelB == 1 ? 0 : b];
-            const float hr = fmaxf(lev - z, 0.0f);
-            const bool use_hr = hr > a.kc.absorb_lim;
-            const float hc = use_hr ? hr : hg;
-            const float cm = fmaxf(hc, a.kc.absorb_min);
-            const float c = M::sqrt(a.kc.g981 * cm);
-            const float s = (side == 0 || side == 2) ? -1.0f : 1.0f;
-            const float lv = lg[normal];
-            const float l_c = lv * (s * (hg - hr));
-            const float l_diff = lv * (s * c);
-            float l_hc = 0.0f;
-            if (hc >= a.kc.absorb_min) {
-                const float c2 = 2.0f * c;
-                l_hc = a.kc.g981 * M::div(l_c, c2, M::rcp(c2));
-            }
-            float l_hg = l_diff + (use_hr ? 0.0f : l_hc);
-            float l_hr = -l_diff + (use_hr ? l_hc : 0.0f);
-            lam[0] += l_hg;
-            if (lev - z >= 0.0f) {
-                llev += l_hr;
-                if (BEDG) lzc -= l_hr;
-            }
-        }
-        break;
-    default:
-        break;
-    }
 }
 
 // _clean_and_limit (solver.py:547-570) in the arithmetic M.
@@ -411,6 +154,547 @@ __device__ void clean_bwd(const State& o, const State& c, const State& lout, con
     lold.h -= ld0;
     lold.hu -= ld1;
     lold.hv -= ld2;
+}
+
+// State of interior cell (j, i): S, or the predictor formed from U and k1.
+template <bool PRED, class M>
+__device__ __forceinline__ State cell_state(const AdjArgs& a, int b, int j, int i, float scale) {
+    const size_t plane = (size_t)a.ny * a.nx;
+    const size_t o = a3(b, 0, j, i, a.ny, a.nx);
+    if (!PRED || a.S != nullptr) return State{a.S[o], a.S[o + plane], a.S[o + 2 * plane]};
+    const State u{a.U[o], a.U[o + plane], a.U[o + 2 * plane]};
+    const State cand{u.h + scale * a.k1[o], u.hu + scale * a.k1[o + plane], u.hv + scale * a.k1[o + 2 * plane]};
+    return clean_fwd<M>(u, cand, a.kc, a.positivity != 0);
+}
+
+// Padded cell (j, i) with the ghost rules (arm cells only: in the interior
+// along one direction, at most two cells outside along the other).
+template <bool PRED, class M>
+__device__ State padded_state(const AdjArgs& a, int b, int j, int i, float scale, float& z) {
+    const int ny = a.ny, nx = a.nx;
+    const bool jin = (unsigned)j < (unsigned)ny, iin = (unsigned)i < (unsigned)nx;
+    int js = min(max(j, 0), ny - 1), is = min(max(i, 0), nx - 1);
+    const bool xarm = jin && !iin, yarm = iin && !jin;
+    int code = -1, side = 0;
+    if (xarm || yarm) {
+        side = xarm ? (i < 0 ? 0 : 1) : (j < 0 ? 2 : 3);
+        code = a.bc[side];
+        if (code == SWE_BC_PERIODIC) {
+            if (xarm) is = i < 0 ? nx + i : i - nx;
+            else js = j < 0 ? ny + j : j - ny;
+        }
+    }
+    State s = cell_state<PRED, M>(a, b, js, is, scale);
+    z = bed_of(a, b, js, is);
+    if (code < 0) return s;
+    const float lev = a.level[a.levelB == 1 ? 0 : b];
+    if (code == SWE_BC_CONSTANT) {
+        s = State{a.cval, a.cval, a.cval};
+    } else if (code == SWE_BC_WATER_LEVEL) {
+        s.h = fmaxf(lev - z, 0.0f);
+    } else if (code == SWE_BC_WALL) {
+        const int jm = xarm ? j : (j < 0 ? -1 - j : 2 * ny - 1 - j);
+        const int im = xarm ? (i < 0 ? -1 - i : 2 * nx - 1 - i) : i;
+        const State m = cell_state<PRED, M>(a, b, jm, im, scale);
+        if (xarm) s.hu = -m.hu;
+        else s.hv = -m.hv;
+    } else if (code == SWE_BC_ABSORBING) {
+        const float hr = fmaxf(lev - z, 0.0f);
+        const float hg = s.h;
+        const float hc = hr > a.kc.absorb_lim ? hr : hg;
+        const float c = M::sqrt(a.kc.g981 * fmaxf(hc, a.kc.absorb_min));
+        const float val = ((side == 0 || side == 2) ? -c : c) * (hg - hr);
+        if (xarm) s.hu = val;
+        else s.hv = val;
+    }
+    return s;
+}
+
+// Floats per cell of the sides' and adjoints' slots (see adj_tile_kernel).
+template <bool BEDG>
+__host__ __device__ constexpr int adj_slots() { return BEDG ? 14 : 10; }
+
+template <bool BEDG, int TY>
+__host__ __device__ constexpr int adj_tile_smem() {
+    return (int)sizeof(float) * (5 * (TY + 6) * (ADJ_TX + 6) + adj_slots<BEDG>() * TY * (ADJ_TX + 4) +
+                                 adj_slots<BEDG>() * (TY + 4) * ADJ_TX);
+}
+
+// A line of cells through the tile in one direction: the primitives and the
+// slots of its cells, `ps` and `ss` floats apart from one cell to the next,
+// `pf` and `sf` from one field or slot to the next.
+//
+// Slots of a cell: the sides p (0-4: hlin, eta, bed, u, v) and m (5-9), over
+// which each face writes its adjoints of the sides it read (p: 0 hlin, 1 eta,
+// 2 the cell's h, 3 u, 4 v, BEDG: 10 bed, 11 the cell's z; m: 5-9, 12, 13),
+// over which each cell writes what its sides contribute to its left
+// neighbour (0 h, 1 u, 2 v, BEDG 10 z), itself (3 h, 4 safe, 5 u, 6 v, 11 z)
+// and its right neighbour (7 h, 8 u, 9 v, 12 z).
+struct Line {
+    const float* prim;
+    float* slot;
+    int pf, sf;
+};
+
+__device__ __forceinline__ CellPrim prim_at(const Line& l, int off) {
+    const float* p = l.prim + off;
+    return CellPrim{p[0], p[l.pf], p[2 * l.pf], p[3 * l.pf], p[4 * l.pf]};
+}
+
+template <class M>
+__device__ __forceinline__ void line_sides(const Line& l, int ps, const SweConsts& k, bool wsr) {
+    const SidePair s = side_pair<M>(prim_at(l, -ps), prim_at(l, 0), prim_at(l, ps), k, wsr);
+    float* q = l.slot;
+    const int f = l.sf;
+    q[0] = s.p.hlin;
+    q[f] = s.p.eta;
+    q[2 * f] = s.p.bed;
+    q[3 * f] = s.p.u;
+    q[4 * f] = s.p.v;
+    q[5 * f] = s.m.hlin;
+    q[6 * f] = s.m.eta;
+    q[7 * f] = s.m.bed;
+    q[8 * f] = s.m.u;
+    q[9 * f] = s.m.v;
+}
+
+// The face between the line's cell and the next one.  lo / hi: the
+// tendency's cotangents (mass, normal, tangential, already over d) of the
+// two cells (zero outside the grid).
+template <bool BEDG, class M>
+__device__ __forceinline__ void line_face(const Line& l, int ps, int ss, bool exists, const float lo[3],
+                                          const float hi[3], bool normal_y, const SweConsts& k) {
+    float* qp = l.slot;
+    float* qm = l.slot + ss;
+    const int f = l.sf;
+    SideAdj lL{}, lR{};
+    if (exists) {
+        const Side L{qp[0], qp[f], qp[2 * f], qp[3 * f], qp[4 * f]};
+        const Side R{qm[5 * f], qm[6 * f], qm[7 * f], qm[8 * f], qm[9 * f]};
+        const float* p = l.prim;
+        // (F_right(f) - F_left(f + 1)) / d
+        face_adj<BEDG, M>(L, p[0], p[4 * l.pf], R, p[ps], p[4 * l.pf + ps], hi[0] - lo[0], -lo[1], hi[1],
+                          hi[2] - lo[2], normal_y, k, lL, lR);
+    }
+    qp[0] = lL.hlin;
+    qp[f] = lL.eta;
+    qp[2 * f] = lL.dh;
+    qp[3 * f] = lL.u;
+    qp[4 * f] = lL.v;
+    qm[5 * f] = lR.hlin;
+    qm[6 * f] = lR.eta;
+    qm[7 * f] = lR.dh;
+    qm[8 * f] = lR.u;
+    qm[9 * f] = lR.v;
+    if (BEDG) {
+        qp[10 * f] = lL.bed;
+        qp[11 * f] = lL.dz;
+        qm[12 * f] = lR.bed;
+        qm[13 * f] = lR.dz;
+    }
+}
+
+template <bool BEDG, class M>
+__device__ __forceinline__ void line_cell(const Line& l, int ps, bool exists, const SweConsts& k, bool wsr) {
+    float* q = l.slot;
+    const int f = l.sf;
+    LineAdj left{}, right{};
+    PrimAdj own{};
+    if (exists) {
+        SideAdj lp{q[0], q[f], q[3 * f], q[4 * f], q[2 * f], 0.0f, 0.0f};
+        SideAdj lm{q[5 * f], q[6 * f], q[8 * f], q[9 * f], q[7 * f], 0.0f, 0.0f};
+        if (BEDG) {
+            lp.bed = q[10 * f];
+            lp.dz = q[11 * f];
+            lm.bed = q[12 * f];
+            lm.dz = q[13 * f];
+        }
+        side_pair_bwd<BEDG, M>(prim_at(l, -ps), prim_at(l, 0), prim_at(l, ps), lp, lm, k, wsr, left, own, right);
+    }
+    q[0] = left.h;
+    q[f] = left.u;
+    q[2 * f] = left.v;
+    q[3 * f] = own.h;
+    q[4 * f] = own.safe;
+    q[5 * f] = own.u;
+    q[6 * f] = own.v;
+    q[7 * f] = right.h;
+    q[8 * f] = right.u;
+    q[9 * f] = right.v;
+    if (BEDG) {
+        q[10 * f] = left.z;
+        q[11 * f] = own.z;
+        q[12 * f] = right.z;
+    }
+}
+
+// Adds what reaches a cell's primitives along a line: its own slots and, if
+// they are there, its neighbours'.
+template <bool BEDG>
+__device__ __forceinline__ void line_sum(const Line& l, int ss, bool self, bool lower, bool upper, PrimAdj& t) {
+    const float* q = l.slot;
+    const int f = l.sf;
+    if (self) {
+        t.h += q[3 * f];
+        t.safe += q[4 * f];
+        t.u += q[5 * f];
+        t.v += q[6 * f];
+        if (BEDG) t.z += q[11 * f];
+    }
+    if (lower) {
+        const float* r = q - ss;
+        t.h += r[7 * f];
+        t.u += r[8 * f];
+        t.v += r[9 * f];
+        if (BEDG) t.z += r[12 * f];
+    }
+    if (upper) {
+        const float* r = q + ss;
+        t.h += r[0];
+        t.u += r[f];
+        t.v += r[2 * f];
+        if (BEDG) t.z += r[10 * f];
+    }
+}
+
+__device__ __forceinline__ bool in_frame(const AdjArgs& a, int j, int i) {
+    return i < 2 || i >= a.nx - 2 || j < 2 || j >= a.ny - 2;
+}
+
+// What becomes of a cell's adjoint lam of S (or of P).
+template <bool PRED, class M>
+__device__ __forceinline__ void finish_cell(const AdjArgs& a, size_t o, size_t plane, const float lam[3],
+                                            float scale) {
+    if (PRED) {  // predictor P = clean(U, U + dt/2 k1), solver.py:639
+        const State u{a.U[o], a.U[o + plane], a.U[o + 2 * plane]};
+        const State cand{u.h + scale * a.k1[o], u.hu + scale * a.k1[o + plane], u.hv + scale * a.k1[o + 2 * plane]};
+        State lold, lcand;
+        clean_bwd<M>(u, cand, State{lam[0], lam[1], lam[2]}, a.kc, a.positivity != 0, lold, lcand);
+        a.lU[o] += lold.h + lcand.h;
+        a.lU[o + plane] += lold.hu + lcand.hu;
+        a.lU[o + 2 * plane] += lold.hv + lcand.hv;
+        a.lk1[o] = lcand.h * scale;
+        a.lk1[o + plane] = lcand.hu * scale;
+        a.lk1[o + 2 * plane] = lcand.hv * scale;
+    } else {
+        a.lS[o] += lam[0];
+        a.lS[o + plane] += lam[1];
+        a.lS[o + 2 * plane] += lam[2];
+    }
+}
+
+// Instruction and latency bound (its operands fit in L2 at the grids it runs
+// on).  Each cell's limiters and each face's reverse mode are evaluated once
+// per direction and a cell's primitives once per pass; 16 rows keep the halo
+// work at 1.1 (x) to 1.2 (y) times the tile's.  The form it replaces ran a
+// thread per face (both cells' sides and four cells' primitives again for
+// each) and moved 24 floats per cell through memory to a gather kernel: 114
+// us for the faces and 18 to 21 for the gather of one launch pair at 4 x 244
+// x 393 in the IEEE arithmetic, against 58.5 (stage 2) and 52 (stage 1) here
+// plus 6 for the edges.
+template <bool BEDG, bool PRED, class M, int TY>
+__global__ void __launch_bounds__(ADJ_THREADS, SWE_ADJ_TILE_MINB) adj_tile_kernel(const AdjArgs a) {
+    constexpr int TX = ADJ_TX, RX = TX + 6, RY = TY + 6, SX = TX + 4, SY = TY + 4, NS = adj_slots<BEDG>();
+    extern __shared__ float s_mem[];
+    float* const s_p = s_mem;                    // primitives [5][RY][RX], cell (ry, rx) = (j0 - 3 + ry, i0 - 3 + rx)
+    float* const s_x = s_p + 5 * RY * RX;        // x slots [NS][TY][SX], columns from i0 - 2
+    float* const s_y = s_x + NS * TY * SX;       // y slots [NS][SY][TX], rows from j0 - 2
+    chain_start();
+    const int ny = a.ny, nx = a.nx, tid = threadIdx.x, b = blockIdx.y;
+    const int ntx = (nx + TX - 1) / TX;
+    const int i0 = (int)(blockIdx.x % (unsigned)ntx) * TX, j0 = (int)(blockIdx.x / (unsigned)ntx) * TY;
+    const size_t plane = (size_t)ny * nx;
+    const SweConsts& kc = a.kc;
+    const bool wsr = a.wsr != 0;
+    float scale = 0.0f;
+    if (PRED) scale = 0.5f * (a.dt_dev != nullptr ? *a.dt_dev : a.dt);
+
+    // primitives of the tile's cross: rows of the tile with three columns
+    // either side, columns of the tile with three rows either side
+    for (int w = tid; w < RY * RX; w += ADJ_THREADS) {
+        const int ry = w / RX, rx = w - ry * RX;
+        const int j = j0 + ry - 3, i = i0 + rx - 3;
+        const bool xin = ry >= 3 && ry < TY + 3 && j < ny && i >= -2 && i <= nx + 1;
+        const bool yin = rx >= 3 && rx < TX + 3 && i < nx && j >= -2 && j <= ny + 1;
+        CellPrim p{};
+        if (xin || yin) {
+            float z;
+            const State s = padded_state<PRED, M>(a, b, j, i, scale, z);
+            p = cell_prim<M>(s.h, s.hu, s.hv, z, kc);
+        }
+        s_p[w] = p.h;
+        s_p[RY * RX + w] = p.u;
+        s_p[2 * RY * RX + w] = p.v;
+        s_p[3 * RY * RX + w] = p.eta;
+        s_p[4 * RY * RX + w] = p.z;
+    }
+    __syncthreads();
+
+    // x line of row ty, slot column sx; y line of column tx, slot row sy
+    auto xline = [&](int ty, int sx) {
+        return Line{s_p + (ty + 3) * RX + sx + 1, s_x + ty * SX + sx, RY * RX, TY * SX};
+    };
+    auto yline = [&](int sy, int tx) {
+        return Line{s_p + (sy + 1) * RX + tx + 3, s_y + sy * TX + tx, RY * RX, SY * TX};
+    };
+
+    for (int w = tid; w < TY * SX + SY * TX; w += ADJ_THREADS) {
+        if (w < TY * SX) line_sides<M>(xline(w / SX, w % SX), 1, kc, wsr);
+        else line_sides<M>(yline((w - TY * SX) / TX, (w - TY * SX) % TX), RX, kc, wsr);
+    }
+    __syncthreads();
+
+    // x faces between slot columns fx and fx + 1, y faces between slot rows
+    constexpr int NFX = TY * (SX - 1), NFY = (SY - 1) * TX;
+    for (int w = tid; w < NFX + NFY; w += ADJ_THREADS) {
+        const bool isx = w < NFX;
+        const int v = isx ? w : w - NFX;
+        const int line = isx ? v / (SX - 1) : v / TX, pos = isx ? v - line * (SX - 1) : v - line * TX;
+        // first of the face's two cells
+        const int j = isx ? j0 + line : j0 - 2 + line, i = isx ? i0 - 2 + pos : i0 + pos;
+        const bool exists = isx ? j < ny && i >= -1 && i < nx : i < nx && j >= -1 && j < ny;
+        float lo[3] = {0.0f, 0.0f, 0.0f}, hi[3] = {0.0f, 0.0f, 0.0f};
+        const float rd = isx ? kc.rdx : kc.rdy;
+        const size_t cn = isx ? plane : 2 * plane, ct = isx ? 2 * plane : plane;  // normal, tangential channels
+        const float* q = a.lrhs + (size_t)b * 3 * plane + (ptrdiff_t)j * nx + i;
+        if (exists && (isx ? i : j) >= 0) {
+            lo[0] = q[0] * rd;
+            lo[1] = q[cn] * rd;
+            lo[2] = q[ct] * rd;
+        }
+        if (exists && (isx ? i + 1 < nx : j + 1 < ny)) {
+            q += isx ? 1 : nx;
+            hi[0] = q[0] * rd;
+            hi[1] = q[cn] * rd;
+            hi[2] = q[ct] * rd;
+        }
+        if (isx) line_face<BEDG, M>(xline(line, pos), 1, 1, exists, lo, hi, false, kc);
+        else line_face<BEDG, M>(yline(line, pos), RX, TX, exists, lo, hi, true, kc);
+    }
+    __syncthreads();
+
+    // cells whose sides have adjoints: the tile's and one more either side
+    constexpr int NCX = TY * (TX + 2), NCY = (TY + 2) * TX;
+    for (int w = tid; w < NCX + NCY; w += ADJ_THREADS) {
+        if (w < NCX) {
+            const int ty = w / (TX + 2), sx = 1 + w - ty * (TX + 2), i = i0 - 2 + sx;
+            line_cell<BEDG, M>(xline(ty, sx), 1, j0 + ty < ny && i <= nx, kc, wsr);
+        } else {
+            const int v = w - NCX, sy = 1 + v / TX, tx = v % TX, j = j0 - 2 + sy;
+            line_cell<BEDG, M>(yline(sy, tx), RX, i0 + tx < nx && j <= ny, kc, wsr);
+        }
+    }
+    __syncthreads();
+
+    for (int w = tid; w < TY * TX; w += ADJ_THREADS) {
+        const int ty = w / TX, tx = w - ty * TX, j = j0 + ty, i = i0 + tx;
+        if (j >= ny || i >= nx) continue;
+        PrimAdj t{};
+        line_sum<BEDG>(xline(ty, tx + 2), 1, true, true, true, t);
+        line_sum<BEDG>(yline(ty + 2, tx), TX, true, true, true, t);
+        const size_t o = a3(b, 0, j, i, ny, nx);
+        const bool pass = PRED || a.S[o] >= 0.0f;  // a cleaned depth is never negative
+        float lam[3];
+        prim_bwd<M>(prim_at(xline(ty, tx + 2), 0), pass, t, kc, lam[0], lam[1], lam[2]);
+        if (in_frame(a, j, i)) {
+            const size_t c = (size_t)j * nx + i;
+            float* fr = a.frame + (size_t)b * (BEDG ? 4 : 3) * plane + c;
+            fr[0] = lam[0];
+            fr[plane] = lam[1];
+            fr[2 * plane] = lam[2];
+            if (BEDG) fr[3 * plane] = t.z;
+            continue;
+        }
+        finish_cell<PRED, M>(a, o, plane, lam, scale);
+        if (BEDG) a.lbed[(size_t)b * plane + (size_t)j * nx + i] += t.z;
+    }
+
+    // the ghosts along the sides that this tile touches: the first one has
+    // slots of its own, the second only what the first's increments give it
+    auto ghost = [&](const Line& l, int ss, int dir, bool second, int j, int i, float* out) {
+        PrimAdj t{};
+        // dir: -1 below / left of the grid, +1 above / right of it
+        if (!second) line_sum<BEDG>(l, ss, true, dir > 0, dir < 0, t);
+        else line_sum<BEDG>(l, ss, false, dir > 0, dir < 0, t);
+        float z, l0, l1, l2;
+        const State s = padded_state<PRED, M>(a, b, j, i, scale, z);
+        prim_bwd<M>(cell_prim<M>(s.h, s.hu, s.hv, z, kc), s.h >= 0.0f, t, kc, l0, l1, l2);
+        out[0] = l0;
+        out[1] = l1;
+        out[2] = l2;
+        out[3] = t.z;
+    };
+    const bool sides[4] = {i0 == 0, nx - i0 <= TX, j0 == 0, ny - j0 <= TY};
+    for (int w = tid; w < 4 * TY; w += ADJ_THREADS) {
+        const int side = w / (2 * TY), second = (w / TY) & 1, ty = w % TY, j = j0 + ty;
+        if (!sides[side] || j >= ny) continue;
+        const int i = side == 0 ? -1 - second : nx + second;
+        ghost(xline(ty, i - i0 + 2), 1, side == 0 ? -1 : 1, second != 0, j, i,
+              a.gx + 4 * ((((size_t)b * 2 + side) * 2 + second) * ny + j));
+    }
+    for (int w = tid; w < 4 * TX; w += ADJ_THREADS) {
+        const int side = w / (2 * TX), second = (w / TX) & 1, tx = w % TX, i = i0 + tx;
+        if (!sides[2 + side] || i >= nx) continue;
+        const int j = side == 0 ? -1 - second : ny + second;
+        ghost(yline(j - j0 + 2, tx), TX, side == 0 ? -1 : 1, second != 0, j, i,
+              a.gy + 4 * ((((size_t)b * 2 + side) * 2 + second) * nx + i));
+    }
+}
+
+// Folds the adjoint lg of ghost g (side `side`; g its column for left/right,
+// row for top/bottom) into cell (j, i) if the ghost was made from it, and
+// adds the level adjoint once per ghost (in the thread of the ghost's
+// clamped source cell).  BEDG: lg[3] is the ghost's bed adjoint, folded into
+// the cell its bed was copied from (replicate, or periodic), plus the bed
+// terms of the forced ghost depth max(level - z, 0) -> lzc.
+template <bool BEDG, bool PRED, class M>
+__device__ void fold_ghost(const AdjArgs& a, int b, int side, int g, const float* lg, int j, int i,
+                           float scale, float lam[3], float& llev, float& lzc) {
+    const int ny = a.ny, nx = a.nx;
+    const bool xs = side < 2;
+    const int n = xs ? nx : ny;
+    const int pos = xs ? i : j;  // this cell's index along the side's direction
+    const int clamp_src = g < 0 ? 0 : n - 1;
+    const int mirror = g < 0 ? -1 - g : 2 * n - 1 - g;
+    const int periodic = g < 0 ? n + g : g - n;
+    const int normal = xs ? 1 : 2;  // momentum channel reflected by a wall
+    const int code = a.bc[side];
+    if (BEDG && pos == (code == SWE_BC_PERIODIC ? periodic : clamp_src)) lzc += lg[3];
+    switch (code) {
+    case SWE_BC_TRANSMISSIVE:
+        if (pos == clamp_src) {
+            lam[0] += lg[0];
+            lam[1] += lg[1];
+            lam[2] += lg[2];
+        }
+        break;
+    case SWE_BC_PERIODIC:
+        if (pos == periodic) {
+            lam[0] += lg[0];
+            lam[1] += lg[1];
+            lam[2] += lg[2];
+        }
+        break;
+    case SWE_BC_CONSTANT:
+        break;
+    case SWE_BC_WATER_LEVEL:
+        if (pos == clamp_src) {
+            lam[1] += lg[1];
+            lam[2] += lg[2];
+            const float z = bed_of(a, b, xs ? j : clamp_src, xs ? clamp_src : i);
+            const float lev = a.level[a.levelB == 1 ? 0 : b];
+            if (lev - z >= 0.0f) {  // clamp(level - z, min=0)
+                llev += lg[0];
+                if (BEDG) lzc -= lg[0];
+            }
+        }
+        break;
+    case SWE_BC_WALL:
+        if (pos == clamp_src) {
+            lam[0] += lg[0];
+            lam[3 - normal] += lg[3 - normal];
+        }
+        if (pos == mirror) lam[normal] -= lg[normal];
+        break;
+    case SWE_BC_ABSORBING:
+        if (pos == clamp_src) {
+            lam[3 - normal] += lg[3 - normal];
+            lam[0] += lg[0];
+            // value = s c (hg - hr), hr = max(level - z, 0),
+            // c = sqrt(9.81 max(where(hr > 1e-4, hr, hg), 1e-6))
+            const int jj = xs ? j : clamp_src, ii = xs ? clamp_src : i;
+            const float hg = cell_state<PRED, M>(a, b, jj, ii, scale).h;
+            const float z = bed_of(a, b, jj, ii);
+            const float lev = a.level[a.levelB == 1 ? 0 : b];
+            const float hr = fmaxf(lev - z, 0.0f);
+            const bool use_hr = hr > a.kc.absorb_lim;
+            const float hc = use_hr ? hr : hg;
+            const float cm = fmaxf(hc, a.kc.absorb_min);
+            const float c = M::sqrt(a.kc.g981 * cm);
+            const float s = (side == 0 || side == 2) ? -1.0f : 1.0f;
+            const float lv = lg[normal];
+            const float l_c = lv * (s * (hg - hr));
+            const float l_diff = lv * (s * c);
+            float l_hc = 0.0f;
+            if (hc >= a.kc.absorb_min) {
+                const float c2 = 2.0f * c;
+                l_hc = a.kc.g981 * M::div(l_c, c2, M::rcp(c2));
+            }
+            float l_hg = l_diff + (use_hr ? 0.0f : l_hc);
+            float l_hr = -l_diff + (use_hr ? l_hc : 0.0f);
+            lam[0] += l_hg;
+            if (lev - z >= 0.0f) {
+                llev += l_hr;
+                if (BEDG) lzc -= l_hr;
+            }
+        }
+        break;
+    default:
+        break;
+    }
+}
+
+// The frame: cells within two of a side, numbered along the top and bottom
+// pairs of rows, then down the left and right pairs of columns.
+__host__ __device__ __forceinline__ long long frame_cells(int ny, int nx) {
+    return (ny <= 4 || nx <= 4) ? (long long)ny * nx : 4LL * nx + 4LL * (ny - 4);
+}
+__device__ __forceinline__ void frame_cell(int ny, int nx, long long t, int& j, int& i) {
+    if (ny <= 4 || nx <= 4) {
+        j = (int)(t / nx);
+        i = (int)(t - (long long)j * nx);
+    } else if (t < 4LL * nx) {
+        const int r = (int)(t / nx);
+        j = r < 2 ? r : ny - 4 + r;
+        i = (int)(t - (long long)r * nx);
+    } else {
+        t -= 4LL * nx;
+        const int c = (int)(t & 3);
+        j = 2 + (int)(t >> 2);
+        i = c < 2 ? c : nx - 4 + c;
+    }
+}
+
+template <bool BEDG, bool PRED, class M>
+__global__ void __launch_bounds__(ADJ_THREADS) adj_edge_kernel(const AdjArgs a) {
+    chain_start();
+    const int ny = a.ny, nx = a.nx, b = blockIdx.y;
+    const size_t plane = (size_t)ny * nx;
+    const long long cells = frame_cells(ny, nx);
+    float llev = 0.0f;
+    float scale = 0.0f;
+    if (PRED) scale = 0.5f * (a.dt_dev != nullptr ? *a.dt_dev : a.dt);
+    for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < cells;
+         t += (long long)gridDim.x * blockDim.x) {
+        int j, i;
+        frame_cell(ny, nx, t, j, i);
+        const float* fr = a.frame + (size_t)b * (BEDG ? 4 : 3) * plane + (size_t)j * nx + i;
+        float lam[4] = {fr[0], fr[plane], fr[2 * plane], 0.0f};
+        float lz = BEDG ? fr[3 * plane] : 0.0f;
+        if (i < 2 || i >= nx - 2)
+            for (int q = 0; q < 4; ++q) {
+                const float* l = a.gx + 4 * (((size_t)b * 4 + q) * ny + j);
+                fold_ghost<BEDG, PRED, M>(a, b, q >> 1, q < 2 ? -1 - q : nx + q - 2, l, j, i, scale, lam, llev, lz);
+            }
+        if (j < 2 || j >= ny - 2)
+            for (int q = 0; q < 4; ++q) {
+                const float* l = a.gy + 4 * (((size_t)b * 4 + q) * nx + i);
+                fold_ghost<BEDG, PRED, M>(a, b, 2 + (q >> 1), q < 2 ? -1 - q : ny + q - 2, l, j, i, scale, lam, llev,
+                                          lz);
+            }
+        finish_cell<PRED, M>(a, a3(b, 0, j, i, ny, nx), plane, lam, scale);
+        if (BEDG) a.lbed[(size_t)b * plane + (size_t)j * nx + i] += lz;
+    }
+    // per-block partial sum of the level adjoint (fixed order)
+    __shared__ float s_part[ADJ_THREADS / 32];
+    for (int off = 16; off > 0; off >>= 1) llev += __shfl_down_sync(0xffffffffu, llev, off);
+    if ((threadIdx.x & 31) == 0) s_part[threadIdx.x >> 5] = llev;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        float sum = 0.0f;
+        for (int w = 0; w < ADJ_THREADS / 32; ++w) sum += s_part[w];
+        a.llevel_part[(size_t)b * gridDim.x + blockIdx.x] = sum;
+    }
 }
 
 // Adjoint of the friction update (friction.py:12-131) w.r.t. its input state
@@ -503,73 +787,6 @@ __device__ void friction_bwd(const State& s0, float n, float dt, int model, cons
     if (s0.h >= 0.0f) ls.h += l_h;
 }
 
-template <bool BEDG, bool PRED, class M>
-__global__ void __launch_bounds__(ADJ_THREADS, SWE_ADJ_GATHER_MINB) adj_gather_kernel(const AdjArgs a) {
-    chain_start();
-    const int ny = a.ny, nx = a.nx;
-    const int b = blockIdx.y;
-    const long long ncell = (long long)ny * nx;
-    const size_t plane = (size_t)ny * nx;
-    float llev = 0.0f;
-    float scale = 0.0f;
-    if (PRED) scale = 0.5f * (a.dt_dev != nullptr ? *a.dt_dev : a.dt);
-    for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < ncell;
-         t += (long long)gridDim.x * blockDim.x) {
-        const int j = (int)(t / nx), i = (int)(t - (long long)(t / nx) * nx);
-        float lam[4], l[4];
-        lam_x<BEDG>(a, b, j, i, lam);
-        lam_y<BEDG>(a, b, j, i, l);
-        lam[0] += l[0];
-        lam[1] += l[1];
-        lam[2] += l[2];
-        float lz = BEDG ? lam[3] + l[3] : 0.0f;
-        if (i < 2 || i >= nx - 2) {
-            const int gx[4] = {-1, -2, nx, nx + 1};
-            for (int q = 0; q < 4; ++q) {
-                lam_x<BEDG>(a, b, j, gx[q], l);
-                fold_ghost<BEDG, M>(a, b, q < 2 ? 0 : 1, gx[q], l, j, i, lam, llev, lz);
-            }
-        }
-        if (j < 2 || j >= ny - 2) {
-            const int gy[4] = {-1, -2, ny, ny + 1};
-            for (int q = 0; q < 4; ++q) {
-                lam_y<BEDG>(a, b, gy[q], i, l);
-                fold_ghost<BEDG, M>(a, b, q < 2 ? 2 : 3, gy[q], l, j, i, lam, llev, lz);
-            }
-        }
-        const size_t o = a3(b, 0, j, i, ny, nx);
-        if (PRED) {  // predictor P = clean(U, U + dt/2 k1), solver.py:639
-            const State u{a.U[o], a.U[o + plane], a.U[o + 2 * plane]};
-            const State cand{u.h + scale * a.k1[o], u.hu + scale * a.k1[o + plane],
-                             u.hv + scale * a.k1[o + 2 * plane]};
-            State lold, lcand;
-            clean_bwd<M>(u, cand, State{lam[0], lam[1], lam[2]}, a.kc, a.positivity != 0, lold,
-                         lcand);
-            a.lU[o] += lold.h + lcand.h;
-            a.lU[o + plane] += lold.hu + lcand.hu;
-            a.lU[o + 2 * plane] += lold.hv + lcand.hv;
-            a.lk1[o] = lcand.h * scale;
-            a.lk1[o + plane] = lcand.hu * scale;
-            a.lk1[o + 2 * plane] = lcand.hv * scale;
-        } else {
-            a.lS[o] += lam[0];
-            a.lS[o + plane] += lam[1];
-            a.lS[o + 2 * plane] += lam[2];
-        }
-        if (BEDG) a.lbed[(size_t)b * plane + (size_t)j * nx + i] += lz;
-    }
-    // per-block partial sum of the level adjoint (fixed order)
-    __shared__ float s_part[ADJ_THREADS / 32];
-    for (int off = 16; off > 0; off >>= 1) llev += __shfl_down_sync(0xffffffffu, llev, off);
-    if ((threadIdx.x & 31) == 0) s_part[threadIdx.x >> 5] = llev;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        float sum = 0.0f;
-        for (int w = 0; w < ADJ_THREADS / 32; ++w) sum += s_part[w];
-        a.llevel_part[(size_t)b * gridDim.x + blockIdx.x] = sum;
-    }
-}
-
 // ------------------------------------------------------- pointwise adjoints
 
 template <class M>
@@ -632,24 +849,40 @@ inline int blocks_for(long long n) {
     return (int)(b > 148LL * 32 ? 148LL * 32 : b);
 }
 
+// Tile kernel of height TY, its shared-memory limit raised once per device.
+template <bool BEDG, bool PRED, class M, int TY>
+cudaError_t launch_tiles(const AdjArgs& a, cudaStream_t s) {
+    static std::atomic<uint64_t> set{0};
+    constexpr int smem = adj_tile_smem<BEDG, TY>();
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    if (dev >= 64 || !(set.load(std::memory_order_acquire) >> dev & 1)) {
+        e = cudaFuncSetAttribute(adj_tile_kernel<BEDG, PRED, M, TY>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        if (e != cudaSuccess) return e;
+        if (dev < 64) set.fetch_or(1ull << dev, std::memory_order_release);
+    }
+    const dim3 g((unsigned)((a.nx + ADJ_TX - 1) / ADJ_TX) * (unsigned)((a.ny + TY - 1) / TY), a.B);
+    return launch_chained_smem(adj_tile_kernel<BEDG, PRED, M, TY>, g, dim3(ADJ_THREADS), smem, s, a);
+}
+
 // Enqueue the spatial adjoint of a (a.lbed set: with the bed's adjoint;
-// pred: the stage-2 form, the predictor adjoint fused into the gather).
+// pred: the stage-2 form, the predictor adjoint fused in).
 template <class M>
 int launch_adj_spatial(const AdjArgs& a, int level_blocks, bool pred, cudaStream_t s) {
-    const int gx = blocks_for((long long)a.B * a.ny * (a.nx + 1));
-    const int gy = blocks_for((long long)a.B * (a.ny + 1) * a.nx);
-    const dim3 gg(level_blocks, a.B), gf(gx + gy), th(ADJ_THREADS);
+    constexpr int TY = 16;
+    const dim3 ge(level_blocks, a.B), th(ADJ_THREADS);
     cudaError_t e;
     if (a.lbed) {
-        e = launch_chained(adj_face_kernel<true, M>, gf, th, s, a, gx);
+        e = pred ? launch_tiles<true, true, M, TY>(a, s) : launch_tiles<true, false, M, TY>(a, s);
         if (e == cudaSuccess)
-            e = pred ? launch_chained(adj_gather_kernel<true, true, M>, gg, th, s, a)
-                     : launch_chained(adj_gather_kernel<true, false, M>, gg, th, s, a);
+            e = pred ? launch_chained(adj_edge_kernel<true, true, M>, ge, th, s, a)
+                     : launch_chained(adj_edge_kernel<true, false, M>, ge, th, s, a);
     } else {
-        e = launch_chained(adj_face_kernel<false, M>, gf, th, s, a, gx);
+        e = pred ? launch_tiles<false, true, M, TY>(a, s) : launch_tiles<false, false, M, TY>(a, s);
         if (e == cudaSuccess)
-            e = pred ? launch_chained(adj_gather_kernel<false, true, M>, gg, th, s, a)
-                     : launch_chained(adj_gather_kernel<false, false, M>, gg, th, s, a);
+            e = pred ? launch_chained(adj_edge_kernel<false, true, M>, ge, th, s, a)
+                     : launch_chained(adj_edge_kernel<false, false, M>, ge, th, s, a);
     }
     return e == cudaSuccess && cudaGetLastError() == cudaSuccess ? SWE_OK : SWE_ECUDA;
 }

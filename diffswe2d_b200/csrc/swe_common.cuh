@@ -87,12 +87,12 @@ __device__ __forceinline__ void chain_start() {
 }
 
 template <typename... K, typename... A>
-inline cudaError_t launch_chained(void (*kernel)(K...), dim3 grid, dim3 block, cudaStream_t s,
-                                  A&&... args) {
+inline cudaError_t launch_chained_smem(void (*kernel)(K...), dim3 grid, dim3 block, size_t smem, cudaStream_t s,
+                                       A&&... args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = block;
-    cfg.dynamicSmemBytes = 0;
+    cfg.dynamicSmemBytes = smem;
     cfg.stream = s;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -100,6 +100,12 @@ inline cudaError_t launch_chained(void (*kernel)(K...), dim3 grid, dim3 block, c
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     return cudaLaunchKernelEx(&cfg, kernel, static_cast<K>(args)...);
+}
+
+template <typename... K, typename... A>
+inline cudaError_t launch_chained(void (*kernel)(K...), dim3 grid, dim3 block, cudaStream_t s,
+                                  A&&... args) {
+    return launch_chained_smem(kernel, grid, block, 0, s, static_cast<A&&>(args)...);
 }
 
 }  // namespace swe

@@ -19,7 +19,7 @@ state after each call, autograd through everything (optionally
   stage tendencies are recomputed from its checkpoint in replay mode (bit
   for bit the forward's), then the hand-written step adjoint runs in
   reverse over the segment with the gauge cotangents injected at the end of
-  each interval (it re-evaluates only the predictor).  When the whole
+  each interval.  When the whole
   trajectory fits in device memory (``store_states``, decided by free
   memory by default), the forward pass keeps every step's output state and
   stage tendencies instead (its graphs write two alternating rings, copied
@@ -43,10 +43,10 @@ GRAPH_STEPS = 32
 CHECKPOINT_EVERY = 128
 # Kernels of this library per solver step: forward (stage 1, stage 2, the
 # run clock) and adjoint with both stage tendencies kept (cursor set-up,
-# predictor, corrector adjoint, stage-2 spatial + predictor adjoint (2),
-# stage-1 spatial adjoint (2), cursor finish).
+# corrector adjoint, stage-2 spatial + predictor adjoint (2), stage-1 spatial
+# adjoint (2), cursor finish).
 FORWARD_KERNELS_PER_STEP = 3
-ADJOINT_KERNELS_PER_STEP = 8
+ADJOINT_KERNELS_PER_STEP = 7
 
 
 class GaugeRunWorkspace:

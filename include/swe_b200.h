@@ -308,7 +308,7 @@ int swe_step_clocked_k2_f32(int stage, const float* U, const float* bed, int bed
 /*
  * Adjoint of SWE2D.spatial_operator (src/solver.py:448-531) at state S with
  * respect to S and the boundary level: lam_S += (d rhs / d S)^T lam_rhs.
- * scratch_cx holds B*ny*(nx+1)*12 floats, scratch_cy B*(ny+1)*nx*12.
+ * scratch_cx holds 16*B*ny floats, scratch_cy 16*B*nx + 4*B*ny*nx.
  * level_part receives level_blocks partial sums per batch member
  * ([B][level_blocks]); their sum is the level adjoint of batch member b
  * (summed over b when levelB = 1).  Deterministic (no float atomics).
@@ -325,8 +325,7 @@ int swe_adj_spatial_f32(const float* S, const float* bed, int bedB, int B, int n
  * ([B,ny,nx]; the caller sums over b when bedB = 1).  The bed enters through
  * eta = h + z, its limited increments and face values, the Audusse bed,
  * the well-balanced sources and the ghost cells (replicated or periodic
- * copies, forced depth max(level - z, 0)).  Scratch as above but 16 floats
- * per face (B*ny*(nx+1)*16 and B*(ny+1)*nx*16).
+ * copies, forced depth max(level - z, 0)).  Scratch as above.
  */
 int swe_adj_spatial_bed_f32(const float* S, const float* bed, int bedB, int B, int ny, int nx,
                             const swe_params* p, const float* level, int levelB,
@@ -345,14 +344,23 @@ int swe_adj_spatial_bed_f32(const float* S, const float* bed, int bedB, int B, i
  * launches instead of three.  dt_dev, if not null, holds the step's dt in
  * device memory (read in place of dt, for captured graphs).  lam_bed may be
  * null; if not, the bed's adjoint is accumulated as in
- * swe_adj_spatial_bed_f32 (with its 16-float scratch records).  lam_k1 may
- * be the lam_k2 buffer itself (it is written after the last read of lam_k2).
+ * swe_adj_spatial_bed_f32.  lam_k1 may be the lam_k2 buffer itself (at the
+ * cost of a copy of lam_k2, for which scratch_cx then holds 3*B*ny*nx more
+ * floats).
  */
 int swe_adj_stage2_f32(const float* P, const float* U, const float* k1, const float* bed, int bedB,
                        int B, int ny, int nx, const swe_params* p, const float* level, int levelB,
                        const float* lam_k2, float* scratch_cx, float* scratch_cy, float dt,
                        const float* dt_dev, float* lam_U, float* lam_k1, float* level_part,
                        int level_blocks, float* lam_bed, void* stream);
+
+/* swe_adj_stage2_f32 that forms P from U and k1 itself (as mode 2 of
+ * swe_adj_pointwise_f32 does) instead of reading it. */
+int swe_adj_stage2_k1_f32(const float* U, const float* k1, const float* bed, int bedB, int B, int ny,
+                          int nx, const swe_params* p, const float* level, int levelB,
+                          const float* lam_k2, float* scratch_cx, float* scratch_cy, float dt,
+                          const float* dt_dev, float* lam_U, float* lam_k1, float* level_part,
+                          int level_blocks, float* lam_bed, void* stream);
 
 /*
  * Pointwise parts of the step adjoint, for step input U, tendency k and

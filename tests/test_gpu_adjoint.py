@@ -487,3 +487,61 @@ def test_bed_gradient_matches_fp64_finite_differences(golden):
         fd = (loss64(up.reshape(bed64.shape)) - loss64(dn.reshape(bed64.shape))) / 2e-7
         print("bed", idx, gb.ravel()[idx], fd)
         assert abs(gb.ravel()[idx] - fd) <= 2e-2 * abs(fd)
+
+
+
+def _spatial_adjoint(U, z, lam, dx, dy, sides, level, arithmetic):
+    """Adjoints of the state, the level and the bed of one tendency."""
+    from diffswe2d_b200.adjoint import AdjointStepper
+    cfg = SWEConfig(**dict(zip(("boundary_left", "boundary_right", "boundary_top", "boundary_bottom"), sides)))
+    B, _, ny, nx = U.shape
+    m = SWE2D(z, torch.full((ny, nx), 0.02, device=DEV), dx, dy, config=cfg, train_dem=False,
+              arithmetic=arithmetic)
+    st = AdjointStepper(m, B, ny, nx, torch.device(DEV), 1, bed_grad=True)
+    out = torch.zeros_like(U)
+    st._spatial(U.contiguous(), torch.tensor([level], device=DEV), lam.contiguous(), out, st.part[1], "adjoint")
+    return out, st.part[1].sum(), st.lam_bed
+
+
+# grids of one tile (32 x 16 cells) less one, exactly, plus one cell and
+# more, and grids that are all frame; a grid and its transpose meet the tiles
+# at different cells
+@pytest.mark.parametrize("ny,nx", [(2, 2), (3, 5), (5, 4), (15, 31), (16, 32), (17, 33), (34, 18), (50, 67)])
+@pytest.mark.parametrize("arithmetic", ["exact", "fast"])
+def test_spatial_adjoint_of_the_transposed_grid(ny, nx, arithmetic):
+    """Swapping x and y of the grid, its sides, momenta and cotangent swaps
+    the adjoints: equal up to the order of fp32 sums (IEEE: a few dozen
+    roundings, 1e-5 normwise; tolerance mode: hardware approximations also
+    contract differently by direction, 1e-4)."""
+    g = torch.Generator().manual_seed(ny * 100 + nx)
+    z = torch.rand((ny, nx), generator=g) * 0.3 - 0.2
+    h = torch.clamp(torch.rand((2, 1, ny, nx), generator=g) * 0.6 - 0.15, min=0.0)
+    U = torch.cat([h, h * torch.randn((2, 2, ny, nx), generator=g)], 1).to(DEV)
+    lam = torch.randn(U.shape, generator=g).to(DEV)
+    z = z.to(DEV)
+    swap = lambda q: q[:, [0, 2, 1]].transpose(2, 3).contiguous()  # noqa: E731
+    for sides in (("periodic",) * 4, ("water_level", "wall", "absorbing", "transmissive")):
+        a, al, ab = _spatial_adjoint(U, z, lam, 0.5, 0.7, sides, 0.1, arithmetic)
+        c, cl, cb = _spatial_adjoint(swap(U), z.t().contiguous(), swap(lam), 0.7, 0.5,
+                                     sides[2:] + sides[:2], 0.1, arithmetic)
+        bound = 1e-5 if arithmetic == "exact" else 1e-4
+        assert float((a - swap(c)).abs().max()) <= bound * float(a.abs().max())
+        assert float((ab - cb.transpose(1, 2)).abs().max()) <= bound * float(ab.abs().max())
+        assert abs(float(al) - float(cl)) <= bound * max(abs(float(al)), float(a.abs().max()))
+
+
+@pytest.mark.parametrize("ny,nx,dj,di", [(16, 32, 5, 9), (33, 70, 17, 33), (50, 67, 1, 31)])
+def test_spatial_adjoint_of_a_rolled_periodic_grid(ny, nx, dj, di):
+    """Rolling a periodic grid rolls the adjoint: every cell meets a tile's
+    seams and the ghost folds somewhere (sums in another order: 1e-5)."""
+    g = torch.Generator().manual_seed(ny)
+    z = (torch.rand((ny, nx), generator=g) * 0.3 - 0.2).to(DEV)
+    h = torch.clamp(torch.rand((1, 1, ny, nx), generator=g) * 0.6 - 0.15, min=0.0)
+    U = torch.cat([h, h * torch.randn((1, 2, ny, nx), generator=g)], 1).to(DEV)
+    lam = torch.randn(U.shape, generator=g).to(DEV)
+    roll = lambda q: torch.roll(q, (dj, di), (-2, -1))  # noqa: E731
+    a, _, ab = _spatial_adjoint(U, z, lam, 0.5, 0.7, ("periodic",) * 4, 0.0, "exact")
+    c, _, cb = _spatial_adjoint(roll(U), roll(z).contiguous(), roll(lam), 0.5, 0.7, ("periodic",) * 4, 0.0,
+                                "exact")
+    assert float((roll(a) - c).abs().max()) <= 1e-5 * float(a.abs().max())
+    assert float((roll(ab) - cb).abs().max()) <= 1e-5 * float(ab.abs().max())
