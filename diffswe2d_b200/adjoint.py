@@ -27,7 +27,7 @@ import torch
 from . import _native as nat
 
 def level_blocks(ny: int, nx: int) -> int:
-    """Blocks per batch member of the spatial adjoint's gather launch (one
+    """Blocks per batch member of the spatial adjoint's second launch (one
     cell per thread of 256, at most 1024 blocks): each writes one partial
     sum of the level adjoint, summed in a fixed order afterwards."""
     return max(1, min(1024, -(-ny * nx // 256)))
@@ -46,7 +46,10 @@ class AdjointStepper:
     with their scratch buffers allocated once (a run's backward pass calls
     it once per step)."""
 
-    def __init__(self, model, B, ny, nx, dev, levelB, infiltration=None, bed_grad=False):
+    def __init__(self, model, B, ny, nx, dev, levelB, infiltration=None, bed_grad=False, run=False):
+        # run: one of many steps whose level adjoints are summed (and whose
+        # stage tendencies are given): see swe_adj_spatial_run_f32
+        self.run = bool(run)
         shape = (B, 3, ny, nx)
         self.model = model
         self.B, self.ny, self.nx, self.levelB = B, ny, nx, levelB
@@ -54,14 +57,14 @@ class AdjointStepper:
         self.K1 = self.K2 = self.P = None  # stage intermediates, if they have to be recomputed
         self.lam_k, self.lam_k1 = torch.empty(shape, device=dev), torch.empty(shape, device=dev)
         self.red = torch.empty(nat.RED_WORDS, dtype=torch.int32, device=dev)
-        # ghost adjoints and the frame's cells (include/swe_b200.h)
-        self.cx = torch.empty(16 * B * ny, device=dev)
-        self.cy = torch.empty(16 * B * nx + 4 * B * ny * nx, device=dev)
+        # ghost adjoints, the frame's cells, face records along level sides (include/swe_b200.h)
+        self.cx = torch.empty(B * (208 * ny + 64), device=dev)
+        self.cy = torch.empty(B * (208 * nx + 64 + 4 * ny * nx), device=dev)
         # bed adjoint per batch member, accumulated over the steps of a pass
         self.lam_bed = torch.zeros((B, ny, nx), device=dev) if self.bed_grad else None
-        # the launch that writes the partial sums works on the frame of two
-        # cells along the sides: a block per 256 of its cells
-        self.level_blocks = min(level_blocks(ny, nx), -(-4 * (ny + nx) // 256))
+        self.level_blocks = level_blocks(ny, nx)
+        if self.run:  # the partial sums of the frame's blocks
+            self.level_blocks = min(self.level_blocks, -(-4 * (ny + nx) // 256))
         self.part = torch.empty((2, B * self.level_blocks), device=dev)
         probe = torch.empty((B, 1, ny, nx), device=dev)
         self.bed, self.n = model._fields(probe.expand(B, 3, ny, nx))
@@ -88,7 +91,9 @@ class AdjointStepper:
         args = (nat.ptr(S), nat.ptr(self.bed), self.bed.shape[0], self.B, self.ny, self.nx, self.p,
                 nat.ptr(lv), self.levelB, nat.ptr(lam_rhs), nat.ptr(self.cx), nat.ptr(self.cy),
                 nat.ptr(lam_S), nat.ptr(part), self.level_blocks)
-        if self.bed_grad:
+        if self.run:
+            rc = self.lib.swe_adj_spatial_run_f32(*args, nat.ptr(self.lam_bed), self.st)
+        elif self.bed_grad:
             rc = self.lib.swe_adj_spatial_bed_f32(*args, nat.ptr(self.lam_bed), self.st)
         else:
             rc = self.lib.swe_adj_spatial_f32(*args, self.st)
@@ -97,14 +102,14 @@ class AdjointStepper:
     def _stage2(self, P, U, K1, lv, dt, lam_U):
         """Spatial adjoint at the predictor P (lam_rhs = self.lam_k, the
         adjoint of k2) and the predictor's adjoint in one call: lam_U += ...,
-        self.lam_k1 = adjoint of k1.  P None: formed from U and K1 on the way."""
+        self.lam_k1 = adjoint of k1.  In a run P is formed from U and K1 on the way."""
         dev_dt = torch.is_tensor(dt)
         args = (nat.ptr(U), nat.ptr(K1), nat.ptr(self.bed), self.bed.shape[0], self.B, self.ny, self.nx,
                 self.p, nat.ptr(lv), self.levelB, nat.ptr(self.lam_k), nat.ptr(self.cx),
                 nat.ptr(self.cy), 0.0 if dev_dt else float(dt), nat.ptr(dt) if dev_dt else None,
                 nat.ptr(lam_U), nat.ptr(self.lam_k1), nat.ptr(self.part[0]), self.level_blocks,
                 nat.ptr(self.lam_bed) if self.bed_grad else None, self.st)
-        rc = (self.lib.swe_adj_stage2_k1_f32(*args) if P is None
+        rc = (self.lib.swe_adj_stage2_k1_f32(*args) if self.run
               else self.lib.swe_adj_stage2_f32(nat.ptr(P), *args))
         nat.check(rc, "adjoint spatial operator and predictor (stage 2)")
 
@@ -151,11 +156,15 @@ class AdjointStepper:
             K1 = self.K1
             self._tendency(U, lv, K1)
         P = None
+        if K2 is None or not self.run:
+            if self.P is None:
+                self.P = torch.empty_like(U)
+            P = self.P
+            self._pointwise(2, U, K1, dt, None, None, None, P)
         if K2 is None:
             if self.K2 is None:
-                self.K2, self.P = torch.empty_like(U), torch.empty_like(U)
-            P, K2 = self.P, self.K2
-            self._pointwise(2, U, K1, dt, None, None, None, P)
+                self.K2 = torch.empty_like(U)
+            K2 = self.K2
             self._tendency(P, lv, K2)
         # corrector + friction: lam_k = adjoint of k2
         self._pointwise(3 if overwrite else 0, U, K2, dt, lam_out, lam_U, lam_n, None)
@@ -270,7 +279,7 @@ class _ChunkFunction(torch.autograd.Function):
         lam_n = torch.zeros_like(n) if model.cfg.apply_friction else None
         B, _, ny, nx = U0.shape
         ws = AdjointStepper(model, B, ny, nx, U0.device, model._level_arg(level_vec, B)[1],
-                            bed_grad=need_bed)
+                            bed_grad=need_bed, run=True)
         lv = model._level_arg(level_vec.detach(), B)[0]
         for U_s, dt_s in zip(reversed(states), reversed(dts)):
             lam_out, lam = lam, torch.zeros_like(lam)

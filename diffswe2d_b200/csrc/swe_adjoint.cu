@@ -25,7 +25,7 @@ namespace {
 int adj_args(AdjArgs& a, const float* S, const float* bed, int bedB, int B, int ny, int nx,
              const swe_params* p, const float* level, int levelB, const float* lam_rhs,
              float* scratch_cx, float* scratch_cy, float* level_part, int level_blocks,
-             float* lam_bed) {
+             float* lam_bed, bool bands) {
     if (!bed || !level || !lam_rhs || !scratch_cx || !scratch_cy || !level_part)
         return SWE_EARG;
     if (!valid_params(p) || B < 1 || ny < 2 || nx < 2 || level_blocks < 1) return SWE_EARG;
@@ -35,8 +35,8 @@ int adj_args(AdjArgs& a, const float* S, const float* bed, int bedB, int B, int 
     a.bed = bed;
     a.level = level;
     a.lrhs = lam_rhs;
-    a.gx = scratch_cx;  // 16 B ny floats
-    a.gy = scratch_cy;  // 16 B nx floats, then the frame's planes
+    a.gx = scratch_cx;  // 16 B ny floats, then the x bands
+    a.gy = scratch_cy;  // 16 B nx floats, then the frame's planes, then the y bands
     a.frame = scratch_cy + (size_t)16 * B * nx;
     a.llevel_part = level_part;
     a.lbed = lam_bed;
@@ -53,26 +53,31 @@ int adj_args(AdjArgs& a, const float* S, const float* bed, int bedB, int B, int 
     a.wsr = p->water_slope_reset;
     a.kc = make_consts(*p);
     a.positivity = p->positivity_limiter;
+    a.level_blocks = level_blocks;
+    if (bands && ny >= BAND_MIN && nx >= BAND_MIN) {
+        a.bandx = scratch_cx + (size_t)16 * B * ny;
+        a.bandy = a.frame + (size_t)4 * B * ny * nx;
+    }
     return SWE_OK;
 }
 
-int run_spatial(const AdjArgs& a, const swe_params* p, int level_blocks, bool pred, void* stream) {
+int run_spatial(const AdjArgs& a, const swe_params* p, bool pred, void* stream) {
     cudaStream_t s = (cudaStream_t)stream;
-    if (p->arithmetic == SWE_ARITH_FAST) return fast_launch_adj_spatial(a, level_blocks, pred, s);
-    return launch_adj_spatial<ExactMath>(a, level_blocks, pred, s);
+    if (p->arithmetic == SWE_ARITH_FAST) return fast_launch_adj_spatial(a, pred, s);
+    return launch_adj_spatial<ExactMath>(a, pred, s);
 }
 
 int adj_spatial(const float* S, const float* bed, int bedB, int B, int ny, int nx,
                 const swe_params* p, const float* level, int levelB, const float* lam_rhs,
                 float* scratch_cx, float* scratch_cy, float* lam_S, float* level_part,
-                int level_blocks, float* lam_bed, void* stream) {
+                int level_blocks, float* lam_bed, bool bands, void* stream) {
     AdjArgs a;
     const int rc = adj_args(a, S, bed, bedB, B, ny, nx, p, level, levelB, lam_rhs, scratch_cx,
-                            scratch_cy, level_part, level_blocks, lam_bed);
+                            scratch_cy, level_part, level_blocks, lam_bed, bands);
     if (rc != SWE_OK) return rc;
     if (!S || !lam_S) return SWE_EARG;
     a.lS = lam_S;
-    return run_spatial(a, p, level_blocks, false, stream);
+    return run_spatial(a, p, false, stream);
 }
 }  // namespace
 
@@ -82,7 +87,7 @@ extern "C" int swe_adj_spatial_f32(const float* S, const float* bed, int bedB, i
                                    float* lam_S, float* level_part, int level_blocks,
                                    void* stream) {
     return adj_spatial(S, bed, bedB, B, ny, nx, p, level, levelB, lam_rhs, scratch_cx, scratch_cy,
-                       lam_S, level_part, level_blocks, nullptr, stream);
+                       lam_S, level_part, level_blocks, nullptr, true, stream);
 }
 
 extern "C" int swe_adj_spatial_bed_f32(const float* S, const float* bed, int bedB, int B, int ny,
@@ -92,17 +97,26 @@ extern "C" int swe_adj_spatial_bed_f32(const float* S, const float* bed, int bed
                                        float* lam_bed, void* stream) {
     if (!lam_bed) return SWE_EARG;
     return adj_spatial(S, bed, bedB, B, ny, nx, p, level, levelB, lam_rhs, scratch_cx, scratch_cy,
-                       lam_S, level_part, level_blocks, lam_bed, stream);
+                       lam_S, level_part, level_blocks, lam_bed, true, stream);
+}
+
+extern "C" int swe_adj_spatial_run_f32(const float* S, const float* bed, int bedB, int B, int ny, int nx,
+                                       const swe_params* p, const float* level, int levelB,
+                                       const float* lam_rhs, float* scratch_cx, float* scratch_cy,
+                                       float* lam_S, float* level_part, int level_blocks,
+                                       float* lam_bed, void* stream) {
+    return adj_spatial(S, bed, bedB, B, ny, nx, p, level, levelB, lam_rhs, scratch_cx, scratch_cy,
+                       lam_S, level_part, level_blocks, lam_bed, false, stream);
 }
 
 namespace {
 int adj_stage2(const float* P, const float* U, const float* k1, const float* bed, int bedB, int B, int ny,
                int nx, const swe_params* p, const float* level, int levelB, const float* lam_k2,
                float* scratch_cx, float* scratch_cy, float dt, const float* dt_dev, float* lam_U,
-               float* lam_k1, float* level_part, int level_blocks, float* lam_bed, void* stream) {
+               float* lam_k1, float* level_part, int level_blocks, float* lam_bed, bool bands, void* stream) {
     AdjArgs a;
     const int rc = adj_args(a, P, bed, bedB, B, ny, nx, p, level, levelB, lam_k2, scratch_cx,
-                            scratch_cy, level_part, level_blocks, lam_bed);
+                            scratch_cy, level_part, level_blocks, lam_bed, bands);
     if (rc != SWE_OK) return rc;
     if (!U || !k1 || !lam_U || !lam_k1) return SWE_EARG;
     a.U = U;
@@ -113,14 +127,14 @@ int adj_stage2(const float* P, const float* U, const float* k1, const float* bed
     a.lk1 = lam_k1;
     if (lam_k1 == lam_k2) {
         // blocks write lam_k1 while others still read lam_k2: read a copy, kept
-        // past the ghosts of scratch_cx
-        float* copy = scratch_cx + (size_t)16 * B * ny;
+        // past the ghosts and bands of scratch_cx
+        float* copy = scratch_cx + (size_t)16 * B * ny + (a.bandx ? (size_t)band_floats(B, ny) : 0);
         if (cudaMemcpyAsync(copy, lam_k2, sizeof(float) * 3 * B * ny * nx, cudaMemcpyDeviceToDevice,
                             (cudaStream_t)stream) != cudaSuccess)
             return SWE_ECUDA;
         a.lrhs = copy;
     }
-    return run_spatial(a, p, level_blocks, true, stream);
+    return run_spatial(a, p, true, stream);
 }
 }  // namespace
 
@@ -133,7 +147,7 @@ extern "C" int swe_adj_stage2_f32(const float* P, const float* U, const float* k
                                   void* stream) {
     if (!P) return SWE_EARG;
     return adj_stage2(P, U, k1, bed, bedB, B, ny, nx, p, level, levelB, lam_k2, scratch_cx, scratch_cy, dt,
-                      dt_dev, lam_U, lam_k1, level_part, level_blocks, lam_bed, stream);
+                      dt_dev, lam_U, lam_k1, level_part, level_blocks, lam_bed, true, stream);
 }
 
 extern "C" int swe_adj_stage2_k1_f32(const float* U, const float* k1, const float* bed, int bedB, int B,
@@ -142,7 +156,7 @@ extern "C" int swe_adj_stage2_k1_f32(const float* U, const float* k1, const floa
                                      const float* dt_dev, float* lam_U, float* lam_k1,
                                      float* level_part, int level_blocks, float* lam_bed, void* stream) {
     return adj_stage2(nullptr, U, k1, bed, bedB, B, ny, nx, p, level, levelB, lam_k2, scratch_cx, scratch_cy,
-                      dt, dt_dev, lam_U, lam_k1, level_part, level_blocks, lam_bed, stream);
+                      dt, dt_dev, lam_U, lam_k1, level_part, level_blocks, lam_bed, false, stream);
 }
 
 namespace {

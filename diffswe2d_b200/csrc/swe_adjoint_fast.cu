@@ -8,8 +8,8 @@
 
 namespace swe {
 
-int fast_launch_adj_spatial(const AdjArgs& a, int level_blocks, bool pred, cudaStream_t s) {
-    return launch_adj_spatial<FastMath>(a, level_blocks, pred, s);
+int fast_launch_adj_spatial(const AdjArgs& a, bool pred, cudaStream_t s) {
+    return launch_adj_spatial<FastMath>(a, pred, s);
 }
 
 int fast_launch_adj_pointwise(const PwArgs& a, cudaStream_t s) {

@@ -12,8 +12,10 @@
 // ghost cells go to a small buffer; adj_edge_kernel folds them back into the
 // cells and boundary level they were made from (the adjoint of
 // add_ghost_cells, src/boundary.py:150-413) and finishes the two-cell frame
-// along the sides.  Stage 2 goes on through the predictor's adjoint in both.
-// No float atomics: results are deterministic.
+// along the sides; adj_level_kernel sums the level's adjoint.  Stage 2 goes on through the predictor's adjoint in both.
+// No float atomics: results are deterministic.  On request the ghosts that
+// depend on the level are done face by face instead (level bands, below),
+// in two more launches.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -44,9 +46,13 @@ struct AdjArgs {
     const float* lrhs;   // adjoint of the tendency, [B,3,ny,nx]
     float* gx;           // adjoints of the x ghosts [B][left, right][1st, 2nd][ny][4]
     float* gy;           // adjoints of the y ghosts [B][top, bottom][1st, 2nd][nx][4]
-    float* frame;        // adjoints of the frame's cells before the folds [B][3 or 4][ny][nx]
+    float* frame;        // adjoints of the frame's cells before the folds [B][4][ny][nx] (the
+                         // fourth plane: the bed's, then the cell's share of the level's)
+    float* bandx;        // face records along the level's x sides (LevelBand), else null
+    float* bandy;        // the same along its y sides
     float* lS;           // adjoint of S, accumulated (+=)
-    float* llevel_part;  // per-block partial level adjoints [B][gridDim.x]
+    float* llevel_part;  // partial level adjoints [B][level_blocks]
+    int level_blocks, direct_level;  // the latter: written by adj_edge_kernel's own blocks
     float* lbed;         // adjoint of the bed [B,ny,nx], accumulated (+=); BEDG only
     int B, bedB, levelB, ny, nx;
     int bc[4];
@@ -208,6 +214,123 @@ __device__ State padded_state(const AdjArgs& a, int b, int j, int i, float scale
         else s.hv = val;
     }
     return s;
+}
+
+// ------------------------------------------------------------ level bands
+// Along a side whose ghosts depend on the level, the adjoints of its ghosts
+// are summed from face records (swe_adjoint.cuh, namespace line): of the
+// faces normal to the side, d = 0, 1 lines away from it.  In stage 2 also
+// those of the two lines of cells next to it, which stage 1's ghosts take
+// their cotangents from: normal faces to d = 3 and the faces along each line
+// of cells, e = 0, 1.  A record holds the face's contributions to its
+// four cells, 4 x (U0, U1, U2, Z).  Grids too small for the scratch buffers
+// (either side below BAND_MIN cells) do without.
+constexpr int BAND_MIN = 32;
+constexpr int BAND_REC = 16;
+
+__host__ __device__ inline long long band_faces(int n) { return 4LL * n + 2LL * (n + 1); }
+__host__ __device__ inline long long band_floats(int B, int n) { return 2LL * B * band_faces(n) * BAND_REC; }
+__host__ __device__ inline bool level_side(const AdjArgs& a, int side) {
+    return a.bandx != nullptr && (a.bc[side] == SWE_BC_WATER_LEVEL || a.bc[side] == SWE_BC_ABSORBING);
+}
+
+struct LevelBand {
+    float* base;  // this side's records of batch member b
+    int n;        // cells along the side
+    __device__ LevelBand(const AdjArgs& a, int b, int side) {
+        n = side < 2 ? a.ny : a.nx;
+        base = (side < 2 ? a.bandx : a.bandy) + ((long long)b * 2 + (side & 1)) * band_faces(n) * BAND_REC;
+    }
+    __device__ float* normal(int d, int pos) const { return base + ((long long)d * n + pos) * BAND_REC; }
+    __device__ float* along(int e, int face) const {
+        return base + (4LL * n + (long long)e * (n + 1) + face) * BAND_REC;
+    }
+};
+
+// One face of a band: the x face f of row `row`, or the y face f of column `row`.
+template <bool BEDG, bool PRED, class M>
+__device__ void band_face(const AdjArgs& a, int b, bool diry, int f, int row, float scale, float* rec) {
+    const int ny = a.ny, nx = a.nx;
+    const size_t plane = (size_t)ny * nx;
+    line::PrimRec P[4];
+#pragma unroll
+    for (int s = 0; s < 4; ++s) {
+        float z;
+        const State q = diry ? padded_state<PRED, M>(a, b, f - 2 + s, row, scale, z)
+                             : padded_state<PRED, M>(a, b, row, f - 2 + s, scale, z);
+        P[s] = line::prim_rec<M>(q.h, q.hu, q.hv, z, a.kc);
+    }
+    const float d = diry ? a.kc.dy : a.kc.dx, rd = diry ? a.kc.rdy : a.kc.rdx;
+    const int n = diry ? ny : nx;
+    float rp[3] = {0.0f, 0.0f, 0.0f}, rm[3] = {0.0f, 0.0f, 0.0f};
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+        if (f < n) rp[c] = M::div(a.lrhs[(diry ? a3(b, 0, f, row, ny, nx) : a3(b, 0, row, f, ny, nx)) + c * plane], d, rd);
+        if (f >= 1)
+            rm[c] = M::div(a.lrhs[(diry ? a3(b, 0, f - 1, row, ny, nx) : a3(b, 0, row, f - 1, ny, nx)) + c * plane], d, rd);
+    }
+    line::CellAdj out[4];
+    line::face_vjp<BEDG, M>(P, rp[0] - rm[0], diry ? -rm[2] : -rm[1], diry ? rp[2] : rp[1],
+                            diry ? rp[1] - rm[1] : rp[2] - rm[2], diry, a.kc, a.wsr != 0, out);
+#pragma unroll
+    for (int s = 0; s < 4; ++s) {
+        rec[4 * s] = out[s].U0;
+        rec[4 * s + 1] = out[s].U1;
+        rec[4 * s + 2] = out[s].U2;
+        rec[4 * s + 3] = BEDG ? out[s].Z : 0.0f;
+    }
+}
+
+// Faces of all bands of a batch member.
+__host__ __device__ inline long long side_items(const AdjArgs& a, int side, bool pred) {
+    const int n = side < 2 ? a.ny : a.nx;
+    return level_side(a, side) ? (pred ? band_faces(n) : 2LL * n) : 0;
+}
+__host__ __device__ inline long long band_items(const AdjArgs& a, bool pred) {
+    return side_items(a, 0, pred) + side_items(a, 1, pred) + side_items(a, 2, pred) + side_items(a, 3, pred);
+}
+
+// The bands' faces, one per thread.  (In the tile kernel's grid their code
+// cost every tile 8 to 25 %; here 10.5 and 8.4 us at 2 x 244 x 393.)
+template <bool BEDG, bool PRED, class M>
+__global__ void __launch_bounds__(64) adj_band_kernel(const AdjArgs a) {
+    chain_start();
+    const int b = blockIdx.y;
+    float scale = 0.0f;
+    if (PRED) scale = 0.5f * (a.dt_dev != nullptr ? *a.dt_dev : a.dt);
+    long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    int side = 0;
+    while (side < 4 && t >= side_items(a, side, PRED)) t -= side_items(a, side++, PRED);
+    if (side == 4) return;
+    const int n = side < 2 ? a.ny : a.nx, m = side < 2 ? a.nx : a.ny;  // along, across
+    const LevelBand band(a, b, side);
+    const bool far = (side & 1) != 0, normal = t < 4LL * n;
+    if (!normal) t -= 4LL * n;
+    const int len = normal ? n : n + 1;
+    const int d = (int)(t / len), pos = (int)(t - (long long)d * len);  // d: or the line of cells
+    const int across = far ? (normal ? m - d : m - 1 - d) : d;
+    band_face<BEDG, PRED, M>(a, b, normal == (side >= 2), normal ? across : pos, normal ? pos : across, scale,
+                             normal ? band.normal(d, pos) : band.along(d, pos));
+}
+
+// Sum over the band's faces along one axis of what they contribute to padded
+// cell `pos` (its index along that axis, n interior cells; `line` its index
+// along the other), in the faces' order.  normal: the axis is the side's
+// normal; e: the band's line of cells.
+__device__ __noinline__ void band_sum(const LevelBand& band, bool normal, bool far, int e, int line, int pos,
+                                      int n, float l[4]) {
+    float v[4][4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {  // all loads first: a face that is not there adds zero
+        int f = pos - 1 + q;
+        const bool ok = f >= 0 && f <= n;
+        f = min(max(f, max(pos - 1, 0)), min(pos + 2, n));
+        const float* r = (normal ? band.normal(far ? n - f : f, line) : band.along(e, f)) + 4 * (3 - q);
+#pragma unroll
+        for (int c = 0; c < 4; ++c) v[q][c] = ok ? r[c] : 0.0f;
+    }
+#pragma unroll
+    for (int c = 0; c < 4; ++c) l[c] = (((0.0f + v[0][c]) + v[1][c]) + v[2][c]) + v[3][c];
 }
 
 // Floats per cell of the sides' and adjoints' slots (see adj_tile_kernel).
@@ -391,7 +514,7 @@ __device__ __forceinline__ void finish_cell(const AdjArgs& a, size_t o, size_t p
 // each) and moved 24 floats per cell through memory to a gather kernel: 114
 // us for the faces and 18 to 21 for the gather of one launch pair at 4 x 244
 // x 393 in the IEEE arithmetic, against 58.5 (stage 2) and 52 (stage 1) here
-// plus 6 for the edges.
+// plus 8 for the edges.
 template <bool BEDG, bool PRED, class M, int TY>
 __global__ void __launch_bounds__(ADJ_THREADS, SWE_ADJ_TILE_MINB) adj_tile_kernel(const AdjArgs a) {
     constexpr int TX = ADJ_TX, RX = TX + 6, RY = TY + 6, SX = TX + 4, SY = TY + 4, NS = adj_slots<BEDG>();
@@ -401,13 +524,13 @@ __global__ void __launch_bounds__(ADJ_THREADS, SWE_ADJ_TILE_MINB) adj_tile_kerne
     float* const s_y = s_x + NS * TY * SX;       // y slots [NS][SY][TX], rows from j0 - 2
     chain_start();
     const int ny = a.ny, nx = a.nx, tid = threadIdx.x, b = blockIdx.y;
+    float scale = 0.0f;
+    if (PRED) scale = 0.5f * (a.dt_dev != nullptr ? *a.dt_dev : a.dt);
     const int ntx = (nx + TX - 1) / TX;
     const int i0 = (int)(blockIdx.x % (unsigned)ntx) * TX, j0 = (int)(blockIdx.x / (unsigned)ntx) * TY;
     const size_t plane = (size_t)ny * nx;
     const SweConsts& kc = a.kc;
     const bool wsr = a.wsr != 0;
-    float scale = 0.0f;
-    if (PRED) scale = 0.5f * (a.dt_dev != nullptr ? *a.dt_dev : a.dt);
 
     // primitives of the tile's cross: rows of the tile with three columns
     // either side, columns of the tile with three rows either side
@@ -498,7 +621,7 @@ __global__ void __launch_bounds__(ADJ_THREADS, SWE_ADJ_TILE_MINB) adj_tile_kerne
         prim_bwd<M>(prim_at(xline(ty, tx + 2), 0), pass, t, kc, lam[0], lam[1], lam[2]);
         if (in_frame(a, j, i)) {
             const size_t c = (size_t)j * nx + i;
-            float* fr = a.frame + (size_t)b * (BEDG ? 4 : 3) * plane + c;
+            float* fr = a.frame + (size_t)b * 4 * plane + c;
             fr[0] = lam[0];
             fr[plane] = lam[1];
             fr[2 * plane] = lam[2];
@@ -634,6 +757,18 @@ __device__ void fold_ghost(const AdjArgs& a, int b, int side, int g, const float
     }
 }
 
+// Sum over a block in a fixed order (valid in thread 0).
+__device__ __forceinline__ float block_sum(float v) {
+    __shared__ float s_part[ADJ_THREADS / 32];
+    for (int off = 16; off > 0; off >>= 1) v += __shfl_down_sync(0xffffffffu, v, off);
+    if ((threadIdx.x & 31) == 0) s_part[threadIdx.x >> 5] = v;
+    __syncthreads();
+    float sum = 0.0f;
+    if (threadIdx.x == 0)
+        for (int w = 0; w < ADJ_THREADS / 32; ++w) sum += s_part[w];
+    return sum;
+}
+
 // The frame: cells within two of a side, numbered along the top and bottom
 // pairs of rows, then down the left and right pairs of columns.
 __host__ __device__ __forceinline__ long long frame_cells(int ny, int nx) {
@@ -655,46 +790,97 @@ __device__ __forceinline__ void frame_cell(int ny, int nx, long long t, int& j, 
     }
 }
 
+// Finishes the frame, a cell per thread.  A few warps run through it once,
+// so its time is that of its instruction fetches and load chains: one copy
+// of each part, no ghost read in vain.
 template <bool BEDG, bool PRED, class M>
 __global__ void __launch_bounds__(ADJ_THREADS) adj_edge_kernel(const AdjArgs a) {
     chain_start();
     const int ny = a.ny, nx = a.nx, b = blockIdx.y;
     const size_t plane = (size_t)ny * nx;
-    const long long cells = frame_cells(ny, nx);
-    float llev = 0.0f;
     float scale = 0.0f;
     if (PRED) scale = 0.5f * (a.dt_dev != nullptr ? *a.dt_dev : a.dt);
-    for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < cells;
-         t += (long long)gridDim.x * blockDim.x) {
+    const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    float level = 0.0f;
+    if (t < frame_cells(ny, nx)) {
         int j, i;
         frame_cell(ny, nx, t, j, i);
-        const float* fr = a.frame + (size_t)b * (BEDG ? 4 : 3) * plane + (size_t)j * nx + i;
-        float lam[4] = {fr[0], fr[plane], fr[2 * plane], 0.0f};
-        float lz = BEDG ? fr[3 * plane] : 0.0f;
-        if (i < 2 || i >= nx - 2)
-            for (int q = 0; q < 4; ++q) {
-                const float* l = a.gx + 4 * (((size_t)b * 4 + q) * ny + j);
-                fold_ghost<BEDG, PRED, M>(a, b, q >> 1, q < 2 ? -1 - q : nx + q - 2, l, j, i, scale, lam, llev, lz);
+        float llev = 0.0f;
+        // the band this cell lies in, if any
+        int bs = -1;
+        for (int side = 3; side >= 0; --side) {
+            const int dist = side == 0 ? i : side == 1 ? nx - 1 - i : side == 2 ? j : ny - 1 - j;
+            if (dist < 2 && level_side(a, side)) bs = side;
+        }
+        const LevelBand band(a, b, bs < 0 ? 0 : bs);
+        const bool far = (bs & 1) != 0;
+        const int e = bs < 2 ? (far ? nx - 1 - i : i) : (far ? ny - 1 - j : j);
+        float lam[4], lz = 0.0f, l[4];
+        float* fr = a.frame + (size_t)b * 4 * plane + (size_t)j * nx + i;
+        if (bs < 0 || !PRED) {
+            lam[0] = fr[0];
+            lam[1] = fr[plane];
+            lam[2] = fr[2 * plane];
+            if (BEDG) lz = fr[3 * plane];
+        } else {
+            band_sum(band, bs < 2, far, e, j, i, nx, lam);
+            band_sum(band, bs >= 2, far, e, i, j, ny, l);
+            lam[0] += l[0];
+            lam[1] += l[1];
+            lam[2] += l[2];
+            if (BEDG) lz = lam[3] + l[3];
+        }
+#pragma unroll 1
+        for (int q = 0; q < 8; ++q) {  // ghosts -1, -2, nx, nx + 1, then the rows'
+            const int side = q >> 1, second = q & 1;
+            const bool yax = side >= 2;
+            const int n = yax ? ny : nx, pos = yax ? j : i;
+            const int g = (side & 1) ? n + second : -1 - second;
+            const int code = a.bc[side], edge = (side & 1) ? n - 1 : 0;
+            const int mirror = g < 0 ? -1 - g : 2 * n - 1 - g, periodic = g < 0 ? n + g : g - n;
+            const bool touches = code == SWE_BC_PERIODIC ? pos == periodic
+                                                         : pos == edge || (code == SWE_BC_WALL && pos == mirror);
+            if (!touches || (code == SWE_BC_CONSTANT && !BEDG)) continue;
+            // a band holds the records of its own side's ghosts, and in stage 2
+            // of those at the ends of its two lines
+            if (bs >= 0 && (bs == side || (PRED && (bs < 2) == yax))) {
+                band_sum(band, yax == (bs >= 2), far, e, yax ? i : j, g, n, l);
+            } else {
+                const float* gl = yax ? a.gy + 4 * (((size_t)b * 4 + (q - 4)) * nx + i)
+                                      : a.gx + 4 * (((size_t)b * 4 + q) * ny + j);
+                for (int c = 0; c < 4; ++c) l[c] = gl[c];
             }
-        if (j < 2 || j >= ny - 2)
-            for (int q = 0; q < 4; ++q) {
-                const float* l = a.gy + 4 * (((size_t)b * 4 + q) * nx + i);
-                fold_ghost<BEDG, PRED, M>(a, b, 2 + (q >> 1), q < 2 ? -1 - q : ny + q - 2, l, j, i, scale, lam, llev,
-                                          lz);
-            }
+            fold_ghost<BEDG, PRED, M>(a, b, side, g, l, j, i, scale, lam, llev, lz);
+        }
         finish_cell<PRED, M>(a, a3(b, 0, j, i, ny, nx), plane, lam, scale);
         if (BEDG) a.lbed[(size_t)b * plane + (size_t)j * nx + i] += lz;
+        fr[3 * plane] = level = llev;
     }
-    // per-block partial sum of the level adjoint (fixed order)
-    __shared__ float s_part[ADJ_THREADS / 32];
-    for (int off = 16; off > 0; off >>= 1) llev += __shfl_down_sync(0xffffffffu, llev, off);
-    if ((threadIdx.x & 31) == 0) s_part[threadIdx.x >> 5] = llev;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        float sum = 0.0f;
-        for (int w = 0; w < ADJ_THREADS / 32; ++w) sum += s_part[w];
-        a.llevel_part[(size_t)b * gridDim.x + blockIdx.x] = sum;
+    if (a.direct_level) {
+        const float sum = block_sum(level);
+        if (threadIdx.x == 0) {
+            float* part = a.llevel_part + (size_t)b * a.level_blocks;
+            part[blockIdx.x] = sum;
+            for (int k = blockIdx.x + gridDim.x; k < a.level_blocks; k += gridDim.x) part[k] = 0.0f;
+        }
     }
+}
+
+// Partial sums of the level's adjoint with bands: one cell of the grid per
+// thread, so that their order does not depend on how the frame is dealt out.
+static __global__ void __launch_bounds__(ADJ_THREADS, 8) adj_level_kernel(const float* frame, float* part, int ny,
+                                                                         int nx) {
+    chain_start();
+    const int b = blockIdx.y;
+    const size_t plane = (size_t)ny * nx;
+    float llev = 0.0f;
+    for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < (long long)plane;
+         t += (long long)gridDim.x * blockDim.x) {
+        const int j = (int)(t / nx), i = (int)(t - (long long)j * nx);
+        if (i < 2 || i >= nx - 2 || j < 2 || j >= ny - 2) llev += frame[((size_t)b * 4 + 3) * plane + t];
+    }
+    const float sum = block_sum(llev);
+    if (threadIdx.x == 0) part[(size_t)b * gridDim.x + blockIdx.x] = sum;
 }
 
 // Adjoint of the friction update (friction.py:12-131) w.r.t. its input state
@@ -868,22 +1054,29 @@ cudaError_t launch_tiles(const AdjArgs& a, cudaStream_t s) {
 
 // Enqueue the spatial adjoint of a (a.lbed set: with the bed's adjoint;
 // pred: the stage-2 form, the predictor adjoint fused in).
+template <bool BEDG, bool PRED, class M>
+cudaError_t launch_adj_forms(AdjArgs a, cudaStream_t s) {
+    const dim3 th(ADJ_THREADS);
+    const dim3 ge((unsigned)((frame_cells(a.ny, a.nx) + ADJ_THREADS - 1) / ADJ_THREADS), a.B);
+    const long long items = band_items(a, PRED);
+    cudaError_t e = cudaSuccess;
+    if (items > 0)
+        e = launch_chained(adj_band_kernel<BEDG, PRED, M>, dim3((unsigned)((items + 63) / 64), a.B), dim3(64), s, a);
+    a.direct_level = items == 0 && a.level_blocks >= (int)ge.x;
+    if (e == cudaSuccess) e = launch_tiles<BEDG, PRED, M, 16>(a, s);
+    if (e == cudaSuccess) e = launch_chained(adj_edge_kernel<BEDG, PRED, M>, ge, th, s, a);
+    if (e == cudaSuccess && !a.direct_level)
+        e = launch_chained(adj_level_kernel, dim3(a.level_blocks, a.B), th, s, a.frame, a.llevel_part, a.ny, a.nx);
+    return e;
+}
+
+// Enqueue the spatial adjoint of a (a.lbed set: with the bed's adjoint;
+// pred: the stage-2 form, the predictor adjoint fused in).
 template <class M>
-int launch_adj_spatial(const AdjArgs& a, int level_blocks, bool pred, cudaStream_t s) {
-    constexpr int TY = 16;
-    const dim3 ge(level_blocks, a.B), th(ADJ_THREADS);
-    cudaError_t e;
-    if (a.lbed) {
-        e = pred ? launch_tiles<true, true, M, TY>(a, s) : launch_tiles<true, false, M, TY>(a, s);
-        if (e == cudaSuccess)
-            e = pred ? launch_chained(adj_edge_kernel<true, true, M>, ge, th, s, a)
-                     : launch_chained(adj_edge_kernel<true, false, M>, ge, th, s, a);
-    } else {
-        e = pred ? launch_tiles<false, true, M, TY>(a, s) : launch_tiles<false, false, M, TY>(a, s);
-        if (e == cudaSuccess)
-            e = pred ? launch_chained(adj_edge_kernel<false, true, M>, ge, th, s, a)
-                     : launch_chained(adj_edge_kernel<false, false, M>, ge, th, s, a);
-    }
+int launch_adj_spatial(const AdjArgs& a, bool pred, cudaStream_t s) {
+    const cudaError_t e =
+        a.lbed ? (pred ? launch_adj_forms<true, true, M>(a, s) : launch_adj_forms<true, false, M>(a, s))
+               : (pred ? launch_adj_forms<false, true, M>(a, s) : launch_adj_forms<false, false, M>(a, s));
     return e == cudaSuccess && cudaGetLastError() == cudaSuccess ? SWE_OK : SWE_ECUDA;
 }
 
@@ -897,7 +1090,7 @@ int launch_adj_pointwise(const PwArgs& a, cudaStream_t s) {
 }  // namespace
 
 // The FastMath instantiations (swe_adjoint_fast.cu).
-int fast_launch_adj_spatial(const AdjArgs& a, int level_blocks, bool pred, cudaStream_t s);
+int fast_launch_adj_spatial(const AdjArgs& a, bool pred, cudaStream_t s);
 int fast_launch_adj_pointwise(const PwArgs& a, cudaStream_t s);
 
 }  // namespace swe

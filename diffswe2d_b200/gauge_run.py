@@ -303,7 +303,7 @@ class GaugeRunWorkspace:
     def _alloc_backward(self, bed_grad: bool):
         dev, shape = self.dev, self.bufs[0].shape
         self.stepper = AdjointStepper(self.model, self.B, self.ny, self.nx, dev, self.levelB,
-                                      bed_grad=bed_grad)
+                                      bed_grad=bed_grad, run=True)
         self.lam = [torch.empty(shape, device=dev), torch.empty(shape, device=dev)]
         self.g_gauge = torch.zeros_like(self.gauge_out)
         self.g_levels = torch.zeros_like(self.levels)

@@ -308,7 +308,9 @@ int swe_step_clocked_k2_f32(int stage, const float* U, const float* bed, int bed
 /*
  * Adjoint of SWE2D.spatial_operator (src/solver.py:448-531) at state S with
  * respect to S and the boundary level: lam_S += (d rhs / d S)^T lam_rhs.
- * scratch_cx holds 16*B*ny floats, scratch_cy 16*B*nx + 4*B*ny*nx.
+ * scratch_cx holds B*(208*ny + 64) floats, scratch_cy B*(208*nx + 64 +
+ * 4*ny*nx); on grids with fewer than 32 rows or columns 16*B*ny and
+ * B*(16*nx + 4*ny*nx).
  * level_part receives level_blocks partial sums per batch member
  * ([B][level_blocks]); their sum is the level adjoint of batch member b
  * (summed over b when levelB = 1).  Deterministic (no float atomics).
@@ -354,8 +356,19 @@ int swe_adj_stage2_f32(const float* P, const float* U, const float* k1, const fl
                        const float* dt_dev, float* lam_U, float* lam_k1, float* level_part,
                        int level_blocks, float* lam_bed, void* stream);
 
-/* swe_adj_stage2_f32 that forms P from U and k1 itself (as mode 2 of
- * swe_adj_pointwise_f32 does) instead of reading it. */
+/*
+ * The two calls above for the steps of a long run: the stage-2 form makes P
+ * from U and k1 itself (as mode 2 of swe_adj_pointwise_f32 does), and the
+ * ghosts that depend on the level are not done face by face.  (The calls
+ * above evaluate them in autograd's own order of operations, because one
+ * step's level adjoint is a sum of both signs over a side and may nearly
+ * cancel; that costs two more launches.)  lam_bed may be null.
+ */
+int swe_adj_spatial_run_f32(const float* S, const float* bed, int bedB, int B, int ny, int nx,
+                            const swe_params* p, const float* level, int levelB,
+                            const float* lam_rhs, float* scratch_cx, float* scratch_cy,
+                            float* lam_S, float* level_part, int level_blocks, float* lam_bed,
+                            void* stream);
 int swe_adj_stage2_k1_f32(const float* U, const float* k1, const float* bed, int bedB, int B, int ny,
                           int nx, const swe_params* p, const float* level, int levelB,
                           const float* lam_k2, float* scratch_cx, float* scratch_cy, float dt,
