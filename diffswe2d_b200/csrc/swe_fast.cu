@@ -297,6 +297,7 @@ __device__ __forceinline__ void fast_tile(const StepArgs& a, int bx, int by, int
     float rxA0 = 0.0f, rxA1 = 0.0f, rxA2 = 0.0f;  // x-part of row k-2's tendency
     uint32_t axb = 0u, ayb = 0u;
     bool bad = false;
+    bool dryA = false, dryB = false;  // rows k-2, k-1: no water on any lane
     for (int kk = j0 - 2, it = 0; kk < jend + 2; ++kk, ++it) {
         // ---- row kk: state (predictor on stage 2) and primitives
         float s0, s1, s2, z;
@@ -327,12 +328,15 @@ __device__ __forceinline__ void fast_tile(const StepArgs& a, int bx, int by, int
         }
         pC = fprim(s0, s1, s2, z, k);
         const FDiff dB = fdiff(pC, pB);  // row kk minus row kk-1
+        const bool dryC = warp_no_water(pC.h, pC.eta);
         if (it >= 2) {
             // ---- y-sides of row kk-1
-            const FSides sy = fsides(pB, dA, dB, k, wsr);
+            FSides sy{};
+            if (!(dryA && dryB && dryC)) sy = fsides(pB, dA, dB, k, wsr);
             if (it >= 3) {
                 // ---- y-face between rows kk-2 and kk-1
-                const FFace fy = fface<true>(sA, hA, zA, sy.m, pB.h, pB.z, k);
+                FFace fy{};
+                if (!(dryA && dryB)) fy = fface<true>(sA, hA, zA, sy.m, pB.h, pB.z, k);
                 if (STAGE == 1 && out_lane && kk - 1 >= 0 && kk - 1 <= ny) ayb = max(ayb, fy.speed_bits);
                 if (it >= 4) {
                     // ---- row o = kk-2 is complete
@@ -358,9 +362,10 @@ __device__ __forceinline__ void fast_tile(const StepArgs& a, int bx, int by, int
                             }
                             const State u{ld_state<CG>(a.U + oo), ld_state<CG>(a.U + oo + plane),
                                           ld_state<CG>(a.U + oo + 2 * plane)};
+                            const float nv = FRIC != 0 ? a.n[at1(a.nB == 1 ? 0 : b, o, c, ny, nx)] : 0.0f;
                             State upd = fclean(u, r0, r1, r2, dt, k.eps, k.dry, a.positivity);
-                            if (FRIC != 0)
-                                upd = ffriction<FRIC>(upd, a.n[at1(a.nB == 1 ? 0 : b, o, c, ny, nx)], dt, kc);
+                            if (FRIC != 0 && upd.h > k.dry)  // dry cells have no momentum left
+                                upd = ffriction<FRIC>(upd, nv, dt, kc);
                             a.U_out[oo] = upd.h;
                             a.U_out[oo + plane] = upd.hu;
                             a.U_out[oo + 2 * plane] = upd.hv;
@@ -376,7 +381,8 @@ __device__ __forceinline__ void fast_tile(const StepArgs& a, int bx, int by, int
                 fyA1 = fy.ftan;
                 fyA2 = fy.fnorm_R;
                 // ---- x-faces of row kk-1 (an output row for it <= rows + 2)
-                if (kk - 1 < jend) {
+                rxA0 = rxA1 = rxA2 = 0.0f;
+                if (kk - 1 < jend && !dryB) {
                     const float hr = shfl_dn1(pB.h), er = shfl_dn1(pB.eta), zr = shfl_dn1(pB.z);
                     const float ur = shfl_dn1(pB.u), vr = shfl_dn1(pB.v);
                     const FDiff fx{hr - pB.h, er - pB.eta, zr - pB.z, ur - pB.u, vr - pB.v};
@@ -400,6 +406,8 @@ __device__ __forceinline__ void fast_tile(const StepArgs& a, int bx, int by, int
         }
         pB = pC;
         dA = dB;
+        dryA = dryB;
+        dryB = dryC;
     }
     if (STAGE == 1) {
         axb = warp_max_u32(axb);

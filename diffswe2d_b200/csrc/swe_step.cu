@@ -191,10 +191,14 @@ __global__ void __launch_bounds__(NT) stage_kernel(const StepArgs a) {
 
     // Phase 1: face-side values (reconstruction.py:26-96) in x and y.
     const bool wsr = a.wsr != 0;
+    // (where a cell and both neighbours hold no water its sides feed no face)
     for (int w = tid; w < NXS + NYS; w += NT) {
         if (w < NXS) {
             const int ty = w / (TX + 2), sx = w - ty * (TX + 2);
             const int ry = ty + 2, cx = sx + 1;
+            if (no_water(s_h[ry][cx - 1], s_eta[ry][cx - 1]) && no_water(s_h[ry][cx], s_eta[ry][cx]) &&
+                no_water(s_h[ry][cx + 1], s_eta[ry][cx + 1]))
+                continue;
             const Prim pa{s_h[ry][cx - 1], s_u[ry][cx - 1], s_v[ry][cx - 1], s_eta[ry][cx - 1], s_z[ry][cx - 1]};
             const Prim pc{s_h[ry][cx], s_u[ry][cx], s_v[ry][cx], s_eta[ry][cx], s_z[ry][cx]};
             const Prim pb{s_h[ry][cx + 1], s_u[ry][cx + 1], s_v[ry][cx + 1], s_eta[ry][cx + 1], s_z[ry][cx + 1]};
@@ -205,6 +209,9 @@ __global__ void __launch_bounds__(NT) stage_kernel(const StepArgs a) {
             const int w2 = w - NXS;
             const int sy = w2 / TX, tx = w2 - sy * TX;
             const int cy = sy + 1, rx = tx + 2;
+            if (no_water(s_h[cy - 1][rx], s_eta[cy - 1][rx]) && no_water(s_h[cy][rx], s_eta[cy][rx]) &&
+                no_water(s_h[cy + 1][rx], s_eta[cy + 1][rx]))
+                continue;
             const Prim pa{s_h[cy - 1][rx], s_u[cy - 1][rx], s_v[cy - 1][rx], s_eta[cy - 1][rx], s_z[cy - 1][rx]};
             const Prim pc{s_h[cy][rx], s_u[cy][rx], s_v[cy][rx], s_eta[cy][rx], s_z[cy][rx]};
             const Prim pb{s_h[cy + 1][rx], s_u[cy + 1][rx], s_v[cy + 1][rx], s_eta[cy + 1][rx], s_z[cy + 1][rx]};
@@ -221,7 +228,9 @@ __global__ void __launch_bounds__(NT) stage_kernel(const StepArgs a) {
         if (w < NXF) {
             const int ty = w / (TX + 1), fx = w - ty * (TX + 1);
             const int ry = ty + 2;
-            const FaceFlux F = face_flux(s_xp[ty][fx], s_h[ry][fx + 1], s_z[ry][fx + 1], s_xm[ty][fx + 1],
+            FaceFlux F{};
+            if (!(no_water(s_h[ry][fx + 1], s_eta[ry][fx + 1]) && no_water(s_h[ry][fx + 2], s_eta[ry][fx + 2])))
+                F = face_flux(s_xp[ty][fx], s_h[ry][fx + 1], s_z[ry][fx + 1], s_xm[ty][fx + 1],
                                          s_h[ry][fx + 2], s_z[ry][fx + 2], false, kc);
             s_fx[ty][fx] = F;
             if (STAGE == 1 && j0 + ty < a.ny && i0 + fx <= a.nx) axb = max(axb, F.speed_bits);
@@ -229,7 +238,9 @@ __global__ void __launch_bounds__(NT) stage_kernel(const StepArgs a) {
             const int w2 = w - NXF;
             const int fy = w2 / TX, tx = w2 - fy * TX;
             const int rx = tx + 2;
-            const FaceFlux F = face_flux(s_yp[fy][tx], s_h[fy + 1][rx], s_z[fy + 1][rx], s_ym[fy + 1][tx],
+            FaceFlux F{};
+            if (!(no_water(s_h[fy + 1][rx], s_eta[fy + 1][rx]) && no_water(s_h[fy + 2][rx], s_eta[fy + 2][rx])))
+                F = face_flux(s_yp[fy][tx], s_h[fy + 1][rx], s_z[fy + 1][rx], s_ym[fy + 1][tx],
                                          s_h[fy + 2][rx], s_z[fy + 2][rx], true, kc);
             s_fy[fy][tx] = F;
             if (STAGE == 1 && j0 + fy <= a.ny && i0 + tx < a.nx) ayb = max(ayb, F.speed_bits);
@@ -268,7 +279,7 @@ __global__ void __launch_bounds__(NT) stage_kernel(const StepArgs a) {
         const State u{a.U[o], a.U[o + plane], a.U[o + 2 * plane]};
         const State c{u.h + dt * r.r0, u.hu + dt * r.r1, u.hv + dt * r.r2};
         State upd = clean_and_limit(u, c, kc, a.positivity != 0);
-        if (a.friction) {
+        if (a.friction && upd.h > kc.dry) {  // dry cells have no momentum left
             const float nv = a.n[at1(a.nB == 1 ? 0 : b, j, i, a.ny, a.nx)];
             upd = a.friction_model == 0 ? manning(upd, nv, dt, kc) : roughness_friction(upd, nv, dt, kc);
         }
@@ -308,6 +319,11 @@ struct ExactPredict {
 // One tile of the sweep: SW_WARPS strips side by side (tile column bx) times
 // `rows` output rows (tile row by) of batch member b.  The whole block calls
 // it; warps whose strip lies beyond the grid return at once.
+// CG is the persistent ensemble kernel: state written by other blocks is read
+// through L2, and dry rows are not skipped there: its blocks wait for their
+// slowest warp, whose chain the branch lengthens (64 members of 122 x 196:
+// 8.4 ms a run, 9.2 with the skip; a 4096 x 4096 step alone 1,968 -> 1,839
+// us with it).
 template <int STAGE, int FRIC, bool CG>
 __device__ __forceinline__ void sweep_tile(const StepArgs& a, int bx, int by, int b, int rows) {
     const SweConsts& kc = a.kc;
@@ -345,6 +361,7 @@ __device__ __forceinline__ void sweep_tile(const StepArgs& a, int bx, int by, in
     float fy_m = 0.0f, fy_nR = 0.0f, fy_t = 0.0f;  // face above row k-2
     uint32_t axb = 0u, ayb = 0u;
     bool bad = false;
+    bool dry2 = false, dry1 = false, dry0 = false;  // rows k-2, k-1, k: no water on any lane
     for (int k = j0 - 2, it = 0; k < jend + 2; ++k, ++it) {
         State s, ur;
         float z;
@@ -354,22 +371,26 @@ __device__ __forceinline__ void sweep_tile(const StepArgs& a, int bx, int by, in
         pm2 = pm1;
         pm1 = p0;
         p0 = make_prim(s.h, s.hu, s.hv, z, kc);
+        dry2 = dry1;
+        dry1 = dry0;
+        dry0 = !CG && warp_no_water(p0.h, p0.eta);
         if (STAGE == 2) {
             um2 = um1;
             um1 = u0;
             u0 = ur;
         }
         if (it < 2) continue;
-        // y-sides of row k-1 (reconstruction.py:26-96 along y)
-        const Sides sy = make_sides(pm2, pm1, p0, kc, wsr);
-        if (it >= 3) {
-            // y-face between rows k-2 and k-1
-            const FaceFlux fy = face_flux(sy_prev_p, pm2.h, pm2.z, sy.m, pm1.h, pm1.z, true, kc);
-            if (STAGE == 1 && out_lane && k - 1 >= 0 && k - 1 <= a.ny) ayb = max(ayb, fy.speed_bits);
+        // y-sides of row k-1, y-face between rows k-2 and k-1, x-sides and faces
+        // of row k-2: nothing where the three rows are dry.  One branch for
+        // all, so that the two directions' chains overlap where there is water.
+        Sides sy{};
+        FaceFlux fy{}, fx{}, fxl{};
+        if (!(dry2 && dry1 && dry0)) {
+            sy = make_sides(pm2, pm1, p0, kc, wsr);  // reconstruction.py:26-96 along y
+            if (it >= 3) fy = face_flux(sy_prev_p, pm2.h, pm2.z, sy.m, pm1.h, pm1.z, true, kc);
             if (it >= 4) {
-                // Output row o = k-2: its primitives are pm2.  x-sides need the
-                // neighbours' primitives, x-faces the right neighbour's side.
-                const int o = k - 2;
+                // x-sides need the neighbours' primitives, x-faces the right
+                // neighbour's side
                 const Prim xl{shfl_up1(pm2.h), shfl_up1(pm2.u), shfl_up1(pm2.v), shfl_up1(pm2.eta),
                               shfl_up1(pm2.z)};
                 const Prim xr{shfl_dn1(pm2.h), shfl_dn1(pm2.u), shfl_dn1(pm2.v), shfl_dn1(pm2.eta),
@@ -377,10 +398,16 @@ __device__ __forceinline__ void sweep_tile(const StepArgs& a, int bx, int by, in
                 const Sides sx = make_sides(xl, pm2, xr, kc, wsr);
                 const Side rm{shfl_dn1(sx.m.hlin), shfl_dn1(sx.m.eta), shfl_dn1(sx.m.bed),
                               shfl_dn1(sx.m.u), shfl_dn1(sx.m.v)};
-                const FaceFlux fx = face_flux(sx.p, pm2.h, pm2.z, rm, xr.h, xr.z, false, kc);
+                fx = face_flux(sx.p, pm2.h, pm2.z, rm, xr.h, xr.z, false, kc);
                 if (STAGE == 1 && lane >= 1 && lane < 2 + SW_OUT && c >= -1 && c < a.nx)
                     axb = max(axb, fx.speed_bits);
-                const FaceFlux fxl{shfl_up1(fx.fmass), 0.0f, shfl_up1(fx.fnorm_R), shfl_up1(fx.ftan), 0u};
+                fxl = FaceFlux{shfl_up1(fx.fmass), 0.0f, shfl_up1(fx.fnorm_R), shfl_up1(fx.ftan), 0u};
+            }
+        }
+        if (it >= 3) {
+            if (STAGE == 1 && out_lane && k - 1 >= 0 && k - 1 <= a.ny) ayb = max(ayb, fy.speed_bits);
+            if (it >= 4) {
+                const int o = k - 2;  // the output row, complete
                 const FaceFlux fyt{fy_m, 0.0f, fy_nR, fy_t, 0u};
                 if (out_lane) {
                     const float rain = forcing(a.rain, a.rain_mode, a.rain_batch, b, o, c, a.ny, a.nx);
@@ -398,13 +425,12 @@ __device__ __forceinline__ void sweep_tile(const StepArgs& a, int bx, int by, in
                             a.k2_out[oo + plane] = r.r1;
                             a.k2_out[oo + 2 * plane] = r.r2;
                         }
+                        const float nv = FRIC != 0 ? a.n[at1(a.nB == 1 ? 0 : b, o, c, a.ny, a.nx)] : 0.0f;
                         const State u = um2;
                         const State cand{u.h + dt * r.r0, u.hu + dt * r.r1, u.hv + dt * r.r2};
                         State upd = clean_and_limit(u, cand, kc, a.positivity != 0);
-                        if (FRIC != 0) {
-                            const float nv = a.n[at1(a.nB == 1 ? 0 : b, o, c, a.ny, a.nx)];
+                        if (FRIC != 0 && (CG || upd.h > kc.dry))  // dry cells have no momentum left
                             upd = FRIC == 1 ? manning(upd, nv, dt, kc) : roughness_friction(upd, nv, dt, kc);
-                        }
                         a.U_out[oo] = upd.h;
                         a.U_out[oo + plane] = upd.hu;
                         a.U_out[oo + 2 * plane] = upd.hv;
@@ -501,8 +527,8 @@ int g_sweep_rows = SW_ROWS;
 // chip's rate once warps queue (a large grid: the 4 halo rows want tall
 // tiles).  Against the best of twelve heights, measured from 40 x 40 to
 // 4096 x 4096 in both arithmetics, the height this picks is within 6 %; 64
-// rows everywhere took 467 us a step at 64 x 96 (29 us at one row), 516 at
-// 244 x 393 (45 at 1) and 789 at 4096^2 in the tolerance mode (754 at 32).
+// rows everywhere took 171 us a step at 64 x 96 in the tolerance mode (15 us at
+// one row), 172 at 244 x 393 (21 at two) and 789 at 4096^2 (754 at 32).
 int sweep_rows_for(int B, int ny, int nx) {
     if (g_sweep_rows != SW_ROWS) return g_sweep_rows;
     const double strips = (double)((nx + SW_OUT - 1) / SW_OUT) * B;
@@ -569,9 +595,9 @@ dim3 sweep_grid_of(const StepArgs& a) {
 // Kernel form of the IEEE stages.  The shared-memory tile evaluates a cell
 // per thread (no serial chain, fewer halo cells than short sweep tiles) and
 // is the faster form up to about 1.5 million cells; above that the row sweep
-// with tall tiles is (a step, tile / best sweep: 244 x 393 36 / 45 us,
-// 4 x 244 x 393 78 / 97, 1021 x 1019 168 / 189, 1200^2 221 / 235, 2048^2
-// 605 / 570, 4096^2 2341 / 1968).  SWE_STEP_KERNEL=tiled or =sweep fixes the
+// with tall tiles is (a step of an all-wet state, tile / best sweep: 244 x 393
+// 36 / 45 us, 4 x 244 x 393 78 / 97, 1021 x 1019 168 / 189, 1200^2 221 / 235,
+// 2048^2 605 / 570, 4096^2 2341 / 1968; both gain alike from dry land).  SWE_STEP_KERNEL=tiled or =sweep fixes the
 // form, read once per process.  Both give the same bits.
 constexpr long long kTiledMaxCells = 3ll << 19;
 

@@ -160,6 +160,17 @@ __device__ __forceinline__ float shfl_up1(float v) { return __shfl_up_sync(0xfff
 __device__ __forceinline__ float shfl_dn1(float v) { return __shfl_down_sync(0xffffffffu, v, 1); }
 __device__ __forceinline__ uint32_t warp_max_u32(uint32_t v) { return __reduce_max_sync(0xffffffffu, v); }
 
+// Whether no lane's cell holds any water (depth exactly zero, finite bed).
+// The faces between two such cells carry nothing: with a zero difference on
+// one side the limited depth increment is exactly zero, so both face depths
+// are zero, and with them the flux, both sources and the wave speed.  On a
+// flood plain, or the beach of the runup basin, a third to a half of the
+// warps' rows are such, and the sweep skips their sides and faces.
+__device__ __forceinline__ bool no_water(float h, float eta) { return h == 0.0f && fabsf(eta) < INFINITY; }
+__device__ __forceinline__ bool warp_no_water(float h, float eta) {
+    return __all_sync(0xffffffffu, no_water(h, eta));
+}
+
 // Stable time step of stage 2 from the stage-1 maxima (solver.py:620-632;
 // torch.minimum propagates a NaN stable dt); the first thread of the grid
 // records dt and its status bits.
