@@ -638,7 +638,7 @@ def run_ensemble(args, world, rank, local):
     torchrun each rank runs its own shard of the scenarios."""
     from diffswe2d_b200 import scenarios
     from diffswe2d_b200 import _native as nat
-    from diffswe2d_b200.autotune import tune
+    from diffswe2d_b200.autotune import tune, tuned_ensemble_rows
     from diffswe2d_b200.config import SWEConfig
     from diffswe2d_b200.ensemble import Ensemble
     dev = torch.device("cuda", local)
@@ -653,7 +653,7 @@ def run_ensemble(args, world, rank, local):
         members.append(sc)
     arith = args.ens_arithmetic
     tuning = tune(dev, arithmetic=arith)
-    ens = Ensemble(members, device=dev, arithmetic=arith)
+    ens = Ensemble(members, device=dev, arithmetic=arith, rows=tuned_ensemble_rows(dev, arith))
     ens.run()  # warm-up (also captures the graph)
     if world > 1:
         import torch.distributed as dist

@@ -40,8 +40,8 @@ class EnsembleResult:
 class Ensemble:
     """Scenarios (``diffswe2d_b200.scenarios.Scenario`` or compatible) on one GPU.
 
-    ``rows`` fixes the sweep tile height of every scenario; by default it is
-    the autotuner's ensemble value (``autotune.tuned_ensemble_rows``).
+    ``rows`` fixes the sweep tile height of every scenario; by default it
+    follows from their sizes (``autotune.ensemble_rows``).
     ``arithmetic`` selects the step kernels ("exact": IEEE operation for
     operation as the reference; "fast": the tolerance mode).  ``stall_ns``
     is the persistent kernel's idle limit (None: the library's 2 s): a launch
@@ -51,7 +51,7 @@ class Ensemble:
     def __init__(self, scenarios: Sequence, device="cuda", steps: Optional[int] = None,
                  rows: Optional[int] = None, track_hmax: bool = False, max_dt: float = 1.0e9,
                  arithmetic: str = "exact", stall_ns: Optional[int] = None):
-        from .autotune import tuned_ensemble_rows
+        from .autotune import ensemble_rows
         self.arith = nat.arithmetic_code(arithmetic)
         self.stall_ns = 0 if stall_ns is None else int(stall_ns)
         if self.stall_ns < 0:
@@ -60,6 +60,7 @@ class Ensemble:
         self.count = len(scenarios)
         if not 1 <= self.count <= 1024:
             raise ValueError("an ensemble holds 1 to 1024 scenarios")
+        r = int(rows) if rows is not None else ensemble_rows([tuple(sc.bed.shape) for sc in scenarios])
         self._keep = []  # tensors referenced by the device member table
         members = (nat.SweEnsembleMember * self.count)()
         fric = None
@@ -88,7 +89,6 @@ class Ensemble:
                 sw = torch.as_tensor(sc.bc_levels, dtype=torch.float32, device=dev).contiguous()
                 nser = st.numel()
             steps_m = int(sc.steps if steps is None else steps)
-            r = int(rows) if rows is not None else tuned_ensemble_rows(dev, arithmetic)
             mem = members[m]
             mem.bed, mem.n = bed.data_ptr(), n.data_ptr()
             mem.U_a, mem.U_b, mem.k1 = Ua.data_ptr(), Ub.data_ptr(), k1.data_ptr()
@@ -209,7 +209,7 @@ class GaugeEnsemble:
                  out_dt: float, gauges: Sequence, config: SWEConfig, dx: float, dy: Optional[float] = None,
                  rows: Optional[int] = None, max_steps: int = 1 << 30, max_dt_cap: float = 0.0,
                  arithmetic: str = "exact"):
-        from .autotune import tuned_ensemble_rows
+        from .autotune import ensemble_rows
         self.arith = nat.arithmetic_code(arithmetic)
         M, ny, nx = bed.shape
         if not 1 <= M <= 1024:
@@ -241,7 +241,7 @@ class GaugeEnsemble:
                                   device=dev)
         self.gauge_out = torch.zeros((M, self.n_out, max(self.ngauge, 1)), device=dev)
         self.friction = (1 + (0 if config.frictionmodel == "manning" else 1)) if config.apply_friction else 0
-        r = int(rows) if rows is not None else tuned_ensemble_rows(dev, arithmetic)
+        r = int(rows) if rows is not None else ensemble_rows([(ny, nx)] * M)
         p = nat.params(config, dx, dx if dy is None else dy, arithmetic)
         members = (nat.SweEnsembleMember * M)()
         for m in range(M):

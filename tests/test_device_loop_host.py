@@ -45,3 +45,11 @@ def test_level_blocks_one_cell_per_thread_up_to_1024():
     assert level_blocks(16, 16) == 1
     assert level_blocks(244, 393) == math.ceil(244 * 393 / 256)
     assert level_blocks(4096, 4096) == 1024
+
+
+def test_ensemble_rows_follow_the_members():
+    from diffswe2d_b200.autotune import ensemble_rows
+    assert ensemble_rows([(2, 2)]) == 1                       # one tile: the shortest chain
+    assert ensemble_rows([(122, 196)] * 8) <= 4               # few tiles: short ones
+    assert ensemble_rows([(122, 196)] * 64) in (8, 12, 16)
+    assert ensemble_rows([(1024, 1024)] * 1024) >= 32         # many: few halo rows
