@@ -7,6 +7,7 @@ contiguous float32 CUDA tensor, the call raises.
 from __future__ import annotations
 
 import ctypes
+import functools
 from pathlib import Path
 
 import torch
@@ -209,6 +210,7 @@ _SIGNATURES = {
     "swe_ensemble_reset_f32": [_P, _I, _P],
     "swe_ensemble_run_f32": [_P, _I, _I, _I, _I, ctypes.c_longlong, _P],
     "swe_ensemble_results_f32": [_P, _I, _P, _P, _P],
+    "swe_bed_f32": [_P, _P, _P, ctypes.c_longlong, _P, _P],
     "swe_tune_sweep_rows": [_I],
     "swe_sweep_rows": [],
     "swe_load_kernels": [],
@@ -274,23 +276,29 @@ def arithmetic_code(arithmetic: str) -> int:
     return ARITHMETIC[arithmetic]
 
 
+_SIDES = ("left", "right", "top", "bottom")
+
+
+@functools.lru_cache(maxsize=64)
+def _packed_params(numbers, codes, arithmetic) -> bytes:
+    return bytes(SweParams(*numbers, *codes, arithmetic, 0))
+
+
 def params(cfg, dx: float, dy: float, arithmetic: str = "exact") -> SweParams:
-    for side in ("left", "right", "top", "bottom"):
-        name = getattr(cfg, f"boundary_{side}")
+    bcs = (cfg.boundary_left, cfg.boundary_right, cfg.boundary_top, cfg.boundary_bottom)
+    for side, name in zip(_SIDES, bcs):
         if name not in BC_CODES:
             raise ValueError(f"Unsupported {side} boundary type {name!r}. "
                              f"Valid types are {sorted(BC_CODES)}.")
     # As in src/solver.py:654-661, every friction model name other than
     # "manning" selects the roughness-length law.
-    return SweParams(
-        float(cfg.gravity), float(cfg.dry_depth), float(cfg.epsilon), float(cfg.cfl),
-        float(cfg.limiter_theta), float(dx), float(dy), float(cfg.constant_value),
-        BC_CODES[cfg.boundary_left], BC_CODES[cfg.boundary_right],
-        BC_CODES[cfg.boundary_top], BC_CODES[cfg.boundary_bottom],
-        int(bool(cfg.water_slope_reset)), int(bool(cfg.positivity_limiter)),
-        int(bool(cfg.apply_friction)), 0 if cfg.frictionmodel == "manning" else 1,
-        arithmetic_code(arithmetic), 0,
-    )
+    return SweParams.from_buffer_copy(_packed_params(
+        (float(cfg.gravity), float(cfg.dry_depth), float(cfg.epsilon), float(cfg.cfl),
+         float(cfg.limiter_theta), float(dx), float(dy), float(cfg.constant_value)),
+        (BC_CODES[bcs[0]], BC_CODES[bcs[1]], BC_CODES[bcs[2]], BC_CODES[bcs[3]],
+         int(bool(cfg.water_slope_reset)), int(bool(cfg.positivity_limiter)),
+         int(bool(cfg.apply_friction)), 0 if cfg.frictionmodel == "manning" else 1),
+        arithmetic_code(arithmetic)))
 
 
 def require_cuda_f32(name: str, t: torch.Tensor) -> torch.Tensor:
@@ -304,12 +312,17 @@ def require_cuda_f32(name: str, t: torch.Tensor) -> torch.Tensor:
     return t.contiguous()
 
 
-def stream_handle(device: torch.device) -> ctypes.c_void_p:
-    return ctypes.c_void_p(torch.cuda.current_stream(device).cuda_stream)
+def stream_handle(device: torch.device) -> int:
+    """The current stream of the device (a cudaStream_t), as an address."""
+    if not torch.cuda.is_initialized():
+        torch.cuda.init()
+    index = device.index
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device() if index is None else index)
 
 
-def ptr(t) -> ctypes.c_void_p:
-    return ctypes.c_void_p(0 if t is None else t.data_ptr())
+def ptr(t) -> int:
+    """A tensor's device address (0, the null pointer, for None)."""
+    return 0 if t is None else t.data_ptr()
 
 
 def check(rc: int, what: str) -> None:

@@ -66,9 +66,8 @@ class AdjointStepper:
         if self.run:  # the partial sums of the frame's blocks
             self.level_blocks = min(self.level_blocks, -(-4 * (ny + nx) // 256))
         self.part = torch.empty((2, B * self.level_blocks), device=dev)
-        probe = torch.empty((B, 1, ny, nx), device=dev)
-        self.bed, self.n = model._fields(probe.expand(B, 3, ny, nx))
-        self.infil, self.imode, self.iB = model._forcing_arg(infiltration, probe)
+        self.bed, self.n = model._fields(self.lam_k)
+        self.infil, self.imode, self.iB = model._forcing_arg(infiltration, self.lam_k[:, 0:1])
         self.p = model._params()
         self.fric = bool(model.cfg.apply_friction)
         self.lib, self.dev = nat.lib(), dev
@@ -198,12 +197,13 @@ def adjoint_step(model, U, level, n, dt, lam_out, infiltration=None, ws=None, la
     lv, levelB = model._level_arg(level.detach(), B)
     if ws is None or ws.key != (B, ny, nx, str(dev), levelB, bool(bed_grad)):
         ws = AdjointStepper(model, B, ny, nx, dev, levelB, infiltration, bed_grad)
-    lam_U = torch.zeros_like(U) if lam_U is None else lam_U
+    overwrite = lam_U is None
+    lam_U = torch.empty_like(U) if overwrite else lam_U
     if ws.fric and lam_n is None:
         lam_n = torch.zeros_like(ws.n)
     if ws.bed_grad:
         ws.lam_bed.zero_()
-    part = ws(U, lv, dt, lam_out, lam_U, lam_n)
+    part = ws(U, lv, dt, lam_out, lam_U, lam_n, overwrite=overwrite)
     lam_bed = ws.bed_adjoint() if ws.bed_grad else None
     return lam_U, ws.level_adjoint(part), (lam_n if ws.fric else None), lam_bed
 
@@ -237,8 +237,7 @@ class _StepFunction(torch.autograd.Function):
 
 def step_with_adjoint(model, U, model_time, max_dt, infiltration=None, boundary_level=None):
     """SWE2D.step under autograd: returns (U_new, dt_float) like the reference."""
-    max_dt_f = float((max_dt.to(dtype=torch.float32) if torch.is_tensor(max_dt)
-                      else torch.tensor(float(max_dt), dtype=torch.float32)).item())
+    max_dt_f = model._max_dt_f32(max_dt)
     level = model._prepare_boundary_level(
         model.cfg.constant_level if boundary_level is None else boundary_level, U)
     level_vec = level.reshape(-1) if level.ndim > 0 else level.reshape(1)

@@ -304,6 +304,12 @@ bool batch_ok(int x, int B) { return x == 1 || x == B; }
 
 int launch_result() { return cudaGetLastError() == cudaSuccess ? SWE_OK : SWE_ECUDA; }
 
+__global__ void bed_kernel(const float* ref, const float* corr, const uint8_t* mask, float* bed, long long n) {
+    for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < n;
+         t += (long long)gridDim.x * blockDim.x)
+        bed[t] = ref[t] + corr[t] * (mask[t] ? 1.0f : 0.0f);
+}
+
 }  // namespace
 }  // namespace swe
 
@@ -416,4 +422,11 @@ extern "C" int swe_friction_f32(const float* U, const float* n, int nB, int B, i
     friction_kernel<<<blocks_for(B * plane), OPS_THREADS, 0, (cudaStream_t)stream>>>(
         U, n, nB, out, B, plane, dt, model, make_consts(*p));
     return launch_result();
+}
+
+extern "C" int swe_bed_f32(const float* reference, const float* correction, const uint8_t* mask,
+                           long long cells, float* bed, void* stream) {
+    if (!reference || !correction || !mask || !bed || cells < 1) return SWE_EARG;
+    bed_kernel<<<blocks_for(cells), OPS_THREADS, 0, (cudaStream_t)stream>>>(reference, correction, mask, bed, cells);
+    return cudaGetLastError() == cudaSuccess ? SWE_OK : SWE_ECUDA;
 }

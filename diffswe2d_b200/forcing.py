@@ -10,6 +10,7 @@ sees the reference's rain rates bit for bit.
 """
 from __future__ import annotations
 
+import numpy as np
 import torch
 import torch.nn as nn
 
@@ -31,6 +32,9 @@ class RainfallForcing(nn.Module):
         nt = self.times.numel()
         if nt == 1:
             return self.rates[0:1]
+        if (isinstance(time, float) and not self.times.requires_grad
+                and {self.times.dtype, self.rates.dtype} <= {torch.float32, torch.float64}):
+            return self._at_host_time(time, nt)
         t = torch.as_tensor(time, dtype=self.times.dtype, device=self.times.device)
         hi = torch.searchsorted(self.times, t).clamp(1, nt - 1)
         lo = hi - 1
@@ -40,3 +44,20 @@ class RainfallForcing(nn.Module):
         rate = torch.where(t <= self.times[0], self.rates[0], rate)
         rate = torch.where(t >= self.times[-1], self.rates[-1], rate)
         return rate.unsqueeze(0)
+
+    def _at_host_time(self, time: float, nt: int) -> torch.Tensor:
+        """``at`` for a time on the host: the bracket and the weight are found
+        there, in the series' own float type and operation by operation as
+        above, from one read of the times (the expression above waits for the
+        device at each index it takes from it)."""
+        times = self.times.detach().cpu().numpy()
+        t = times.dtype.type(time)
+        if t >= times[nt - 1]:
+            return self.rates[nt - 1:nt].clone()
+        if t <= times[0]:
+            return self.rates[0:1].clone()
+        hi = min(max(int(np.searchsorted(times, t)), 1), nt - 1)
+        lo = hi - 1
+        one = times.dtype.type(1.0)
+        w = (t - times[lo]) / np.maximum(times[hi] - times[lo], times.dtype.type(1.0e-12))
+        return (float(one - w) * self.rates[lo] + float(w) * self.rates[hi]).unsqueeze(0)

@@ -9,6 +9,7 @@ and dt), where the reference synchronises three times.
 """
 from __future__ import annotations
 
+import struct
 from numbers import Integral, Real
 from typing import Optional, Union
 
@@ -153,6 +154,8 @@ class SWE2D(nn.Module):
     def _prepare_boundary_level(level: ScalarOrTensor, reference: torch.Tensor) -> torch.Tensor:
         if torch.is_tensor(level):
             return level.to(dtype=reference.dtype, device=reference.device)
+        if isinstance(level, float):  # filled on the device: no host copy to wait for
+            return torch.full((), level, dtype=reference.dtype, device=reference.device)
         return reference.new_tensor(level)
 
     def _interpolate_dynamic_boundary(self, current_time: float,
@@ -221,9 +224,26 @@ class SWE2D(nn.Module):
             raise ValueError(f"ng cannot exceed either interior grid dimension. "
                              f"Received ng=2, ny={ny}, nx={nx}.")
 
+    def _bed_values(self):
+        """``bed`` without its gradient: one kernel where the correction is
+        not bounded by the tanh."""
+        ref, corr, mask = self.bed_reference, self.dem_correction_parameter, self.valid_mask
+        plain = (self.maximum_dem_correction is None and mask.dtype == torch.bool
+                 and ref.device == corr.device == mask.device and ref.is_cuda
+                 and ref.dtype == corr.dtype == torch.float32 and ref.shape == corr.shape == mask.shape
+                 and ref.is_contiguous() and corr.is_contiguous() and mask.is_contiguous()
+                 and type(self).bed is SWE2D.bed)
+        if not plain or ref.device.index != torch.cuda.current_device():
+            return nat.require_cuda_f32("bed", self.bed.detach())
+        bed = torch.empty_like(ref)
+        rc = nat.lib().swe_bed_f32(ref.data_ptr(), corr.data_ptr(), mask.data_ptr(), ref.numel(),
+                                   bed.data_ptr(), nat.stream_handle(ref.device))
+        nat.check(rc, "bed")
+        return bed
+
     def _fields(self, U):
         B = U.shape[0]
-        bed = nat.require_cuda_f32("bed", self.bed.detach())
+        bed = self._bed_values()
         if bed.shape[0] not in (1, B):
             raise ValueError(f"Field batch must be 1 or {B}, got {bed.shape[0]}.")
         n = nat.require_cuda_f32("roughness_length", self.roughness_length.detach())
@@ -294,9 +314,7 @@ class SWE2D(nn.Module):
             from .adjoint import step_with_adjoint
             return step_with_adjoint(self, U, model_time, max_dt, infiltration, boundary_level)
         U = nat.require_cuda_f32("U", U)
-        B, _, ny, nx = U.shape
-        max_dt_f = float((max_dt.to(dtype=torch.float32) if torch.is_tensor(max_dt)
-                          else torch.tensor(float(max_dt), dtype=torch.float32)).item())
+        max_dt_f = self._max_dt_f32(max_dt)
         level = self._prepare_boundary_level(
             self.cfg.constant_level if boundary_level is None else boundary_level, U)
         if self.rainfall is not None:
@@ -307,6 +325,20 @@ class SWE2D(nn.Module):
             U_new, status, dt = self._launch_step(U, level, max_dt_f, infiltration)
         self._raise_on_status(status, dt)
         return U_new, dt
+
+    @staticmethod
+    def _max_dt_f32(max_dt) -> float:
+        """max_dt rounded to float32, as the reference holds it."""
+        if torch.is_tensor(max_dt):
+            return float(max_dt.to(dtype=torch.float32).item())
+        with np.errstate(over="ignore"):
+            return float(np.float32(float(max_dt)))
+
+    @staticmethod
+    def _read_status(red):
+        """(status, dt) of a step: one read of the two words (waits for it)."""
+        status, bits = red[2:4].tolist()
+        return status & 0xFFFFFFFF, struct.unpack("f", struct.pack("i", bits))[0]
 
     def _needs_adjoint(self, U, boundary_level) -> bool:
         """A step is differentiated when autograd is on and the state, the
@@ -327,15 +359,12 @@ class SWE2D(nn.Module):
         U_out = torch.empty_like(U)
         scratch = torch.empty_like(U) if scratch is None else scratch
         red = torch.empty(nat.RED_WORDS, dtype=torch.int32, device=U.device) if red is None else red
-        p = self._params()
         rc = nat.lib().swe_step_f32(
-            nat.ptr(U), nat.ptr(bed), bed.shape[0], nat.ptr(n), n.shape[0], B, ny, nx, p,
-            nat.ptr(lv), levelB, max_dt_f, nat.ptr(infil), imode, iB, nat.ptr(scratch),
-            nat.ptr(red), nat.ptr(U_out), nat.stream_handle(U.device))
+            U.data_ptr(), bed.data_ptr(), bed.shape[0], n.data_ptr(), n.shape[0], B, ny, nx,
+            self._params(), lv.data_ptr(), levelB, max_dt_f, nat.ptr(infil), imode, iB,
+            scratch.data_ptr(), red.data_ptr(), U_out.data_ptr(), nat.stream_handle(U.device))
         nat.check(rc, "step")
-        host = red[2:4].cpu()
-        status = int(host[0].item()) & 0xFFFFFFFF
-        dt = float(host[1:2].view(torch.float32).item())
+        status, dt = self._read_status(red)
         return U_out, status, dt
 
     def _host_dt(self, red_host: torch.Tensor, max_dt_f: float) -> float:
@@ -381,10 +410,9 @@ class SWE2D(nn.Module):
         if not np.isfinite(dt) or not dt > 0.0:
             return U_out, nat.S_NONFINITE_DT if not np.isfinite(dt) else nat.S_NONPOSITIVE_DT, dt
         keep = stage(2, self.rainfall.at(time_float + 0.5 * dt))
-        host = red[2:4].cpu()
+        status, dt = self._read_status(red)
         del keep
-        status = int(host[0].item()) & 0xFFFFFFFF
-        return U_out, status, float(host[1:2].view(torch.float32).item())
+        return U_out, status, dt
 
     @staticmethod
     def _raise_on_status(status: int, dt: float) -> None:

@@ -482,6 +482,12 @@ int swe_ensemble_results_f32(const void* workspace, int count, swe_ensemble_resu
  * on first launch); call once before capturing launches in a CUDA graph. */
 int swe_load_kernels(void);
 
+/* The bed of a model, reference + correction * mask (mask: one byte per cell,
+ * 0 or 1), product and sum rounded separately (src/solver.py:134-147 without
+ * the tanh bound). */
+int swe_bed_f32(const float* reference, const float* correction, const uint8_t* mask,
+                long long cells, float* bed, void* stream);
+
 /* Output rows per tile of the single-grid sweep kernels (process-wide
  * tuning knob; set it between launches, not during them).  At its default,
  * 64, each launch takes the height that suits its grid, at most 64. */

@@ -53,3 +53,19 @@ def test_ensemble_rows_follow_the_members():
     assert ensemble_rows([(122, 196)] * 8) <= 4               # few tiles: short ones
     assert ensemble_rows([(122, 196)] * 64) in (8, 12, 16)
     assert ensemble_rows([(1024, 1024)] * 1024) >= 32         # many: few halo rows
+
+
+def test_rainfall_at_a_host_time_equals_the_tensor_expression():
+    import pytest
+    import torch
+    from diffswe2d_b200 import RainfallForcing
+    g = torch.Generator().manual_seed(1)
+    for dtype in (torch.float32, torch.float64):
+        times = torch.tensor([0.0, 1.5, 3.7, 10.0], dtype=dtype)
+        f = RainfallForcing(times, torch.rand((4, 1, 5, 6), generator=g) * 1e-5)
+        for t in (-1.0, 0.0, 0.3, 1.5, 2.2, 3.7, 9.999, 10.0, 11.0):
+            assert torch.equal(f.at(t), f.at(torch.tensor(t, dtype=dtype)))
+    f.at(0.0).zero_()  # a result of its own, not a view of the series
+    assert float(f.rates[0].sum()) > 0
+    with pytest.raises(ValueError):
+        RainfallForcing(times.flip(0), f.rates)

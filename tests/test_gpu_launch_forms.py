@@ -39,3 +39,16 @@ def test_sweep_and_tile_forms_agree(ny, nx, friction):
     for b in (0, B // 2, B - 1):
         assert torch.equal(ks[b], k[0])
         assert torch.equal(Vs[b], V[0])
+
+
+def test_bed_kernel_equals_the_bed_property():
+    """Shared and batched beds, masked and NaN-free corrections, and the
+    tanh-bounded form (which stays a PyTorch expression)."""
+    g = torch.Generator().manual_seed(2)
+    for shape, bound in (((1, 1, 7, 9), None), ((3, 1, 65, 129), None), ((1, 1, 7, 9), 0.5)):
+        z = torch.rand(shape, generator=g).to(DEV)
+        mask = (torch.rand(shape, generator=g) < 0.5).to(DEV)
+        m = SWE2D(z, torch.full_like(z, 0.02), 0.5, 0.7, maximum_dem_correction=bound, valid_mask=mask)
+        with torch.no_grad():
+            m.dem_correction_parameter.copy_(torch.randn(shape, generator=g))
+        assert torch.equal(m._bed_values(), m.bed.detach())
