@@ -74,13 +74,13 @@ SWE_HD void incr_bwd(const Incr& r, float lam, float theta, float& lqm, float& l
 //   FastMath:  the hardware approximations of the tolerance-mode step
 //              (swe_approx.cuh), for runs made with SWE_ARITH_FAST.
 // div(a, b, y) is a / b with y = rcp(b) shared by the quotients of one
-// denominator; pow(x, t) is x^t for positive normal x.
+// denominator; pow2(x, t1, t2) gives x^t1 and x^t2 for positive normal x.
 struct ExactMath {
     static SWE_HD float rcp(float b) { return shared_rcp(b); }
     static SWE_HD float div(float a, float b, float y) { return quot(a, b, y); }
     static SWE_HD float sqrt(float x) { return root(x); }
     static SWE_HD float inv(float b) { return recip(b); }
-    static SWE_HD float pow(float x, float t) { return pow_pos(x, t); }
+    static SWE_HD void pow2(float x, float t1, float t2, float& p1, float& p2) { pow_pos2(x, t1, t2, p1, p2); }
     static SWE_HD float ln(float x) { return (float)::log((double)x); }
 };
 
@@ -90,14 +90,21 @@ struct FastMath {
     static __device__ __forceinline__ float div(float a, float, float y) { return a * y; }
     static __device__ __forceinline__ float sqrt(float x) { return sqrta(x); }
     static __device__ __forceinline__ float inv(float b) { return rcpa(b); }
-    static __device__ __forceinline__ float pow(float x, float t) { return ex2a(t * lg2a(x)); }
+    static __device__ __forceinline__ void pow2(float x, float t1, float t2, float& p1, float& p2) {
+        const float l = lg2a(x);
+        p1 = ex2a(t1 * l);
+        p2 = ex2a(t2 * l);
+    }
     static __device__ __forceinline__ float ln(float x) { return 0.69314718f * lg2a(x); }
 #else
     static inline float rcp(float b) { return 1.0f / b; }
     static inline float div(float a, float b, float) { return a / b; }
     static inline float sqrt(float x) { return ::sqrtf(x); }
     static inline float inv(float b) { return 1.0f / b; }
-    static inline float pow(float x, float t) { return ::powf(x, t); }
+    static inline void pow2(float x, float t1, float t2, float& p1, float& p2) {
+        p1 = ::powf(x, t1);
+        p2 = ::powf(x, t2);
+    }
     static inline float ln(float x) { return ::logf(x); }
 #endif
 };

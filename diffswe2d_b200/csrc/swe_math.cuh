@@ -480,12 +480,14 @@ SWE_HD double u2d(uint64_t x) {
 // the same float as a correctly rounded double pow except for x^t within
 // that distance of a float rounding midpoint.  swe_selftest_arith_f32
 // (which = 4) compares it with CUDA's pow for every float x in a range.
-SWE_HD float pow_pos(float x, float t) {
+constexpr double kLn2Hi = 0x1.62e42feep-1;              // 32 significant bits
+constexpr double kLn2Lo = 0x1.a39ef35793c76p-33;        // ln 2 - kLn2Hi
+struct LnDouble {
+    double hi, lo;
+};
+SWE_HD bool pow_ln_ok(float x) { return f2u(x) - 0x00800000u < 0x7f000000u; }  // positive normal
+SWE_HD LnDouble pow_ln(float x) {
     const uint32_t xb = f2u(x);
-    if (xb - 0x00800000u >= 0x7f000000u) return (float)pow((double)x, (double)t);
-    constexpr double kLn2Hi = 0x1.62e42feep-1;              // 32 significant bits
-    constexpr double kLn2Lo = 0x1.a39ef35793c76p-33;        // ln 2 - kLn2Hi
-    constexpr double kInvLn2 = 0x1.71547652b82fep+0;        // 1 / ln 2
     int e = (int)(xb >> 23) - 127;
     uint32_t mb = (xb & 0x007fffffu) | 0x3f800000u;         // m in [1, 2)
     if (mb > 0x3fb504f3u) {                                 // m > sqrt(2): halve it
@@ -517,11 +519,15 @@ SWE_HD float pow_pos(float x, float t) {
     const double L_hi = p + a_hi;
     const double bb = L_hi - p;
     const double L_lo = ((p - (L_hi - bb)) + (a_hi - bb)) + fma(E, kLn2Lo, a_lo);
+    return LnDouble{L_hi, L_lo};
+}
+SWE_HD float pow_exp(float x, float t, const LnDouble& L) {
+    constexpr double kInvLn2 = 0x1.71547652b82fep+0;        // 1 / ln 2
     // y = t ln x = y_hi + y_lo
     const double td = (double)t;
-    const double y_hi = td * L_hi;
+    const double y_hi = td * L.hi;
     if (!(fabs(y_hi) <= 700.0)) return (float)pow((double)x, (double)t);
-    const double y_lo = fma(td, L_hi, -y_hi) + td * L_lo;
+    const double y_lo = fma(td, L.hi, -y_hi) + td * L.lo;
     const double n = rint(y_hi * kInvLn2);
     const double r = fma(-n, kLn2Hi, y_hi) + fma(-n, kLn2Lo, y_lo);
     double c = 1.0 / 6227020800.0;                          // 1/13!
@@ -539,6 +545,20 @@ SWE_HD float pow_pos(float x, float t) {
     const double er = 1.0 + fma(r * r, c, r);               // exp(r)
     const double scale = u2d((uint64_t)((int)n + 1023) << 52);
     return (float)(er * scale);
+}
+SWE_HD float pow_pos(float x, float t) {
+    return pow_ln_ok(x) ? pow_exp(x, t, pow_ln(x)) : (float)pow((double)x, (double)t);
+}
+// x^t1 and x^t2 from one logarithm.
+SWE_HD void pow_pos2(float x, float t1, float t2, float& p1, float& p2) {
+    if (!pow_ln_ok(x)) {
+        p1 = (float)pow((double)x, (double)t1);
+        p2 = (float)pow((double)x, (double)t2);
+        return;
+    }
+    const LnDouble l = pow_ln(x);
+    p1 = pow_exp(x, t1, l);
+    p2 = pow_exp(x, t2, l);
 }
 
 // x ** (float)(1/3) rounded to float (friction.py:66): the double power

@@ -545,3 +545,35 @@ def test_spatial_adjoint_of_a_rolled_periodic_grid(ny, nx, dj, di):
                                 "exact")
     assert float((roll(a) - c).abs().max()) <= 1e-5 * float(a.abs().max())
     assert float((roll(ab) - cb).abs().max()) <= 1e-5 * float(ab.abs().max())
+
+
+# tiles of 32 x 16 cells: a patch inside one, over seams and over corners of
+# the grid, a single cell, and nothing at all
+@pytest.mark.parametrize("patch", [(20, 30, 36, 60), (14, 18, 30, 34), (0, 9, 0, 40), (44, 67, 90, 101), (31, 32, 63, 64),
+                                   (0, 0, 0, 0)])
+@pytest.mark.parametrize("arithmetic", ["exact", "fast"])
+def test_step_adjoint_of_a_patch_of_cotangents(patch, arithmetic):
+    """A step's adjoint reaches four cells: cotangents that are zero outside
+    a patch give exactly zero further away, and inside, further than that
+    from the patch's edge, the bits that cotangents everywhere give."""
+    from diffswe2d_b200.adjoint import adjoint_step
+    ny, nx, reach = 67, 101, 4
+    g = torch.Generator().manual_seed(sum(patch))
+    z = (torch.rand((ny, nx), generator=g) * 0.1 - 0.2 + torch.linspace(0.0, 0.4, nx)).to(DEV)
+    h = torch.clamp(0.1 - z.cpu(), min=0.0)[None, None]
+    U = torch.cat([h, h * torch.randn((1, 2, ny, nx), generator=g)], 1).to(DEV)
+    dense = torch.randn(U.shape, generator=g).to(DEV)
+    cfg = SWEConfig(boundary_left="water_level", boundary_right="wall", boundary_top="wall", boundary_bottom="absorbing")
+    m = SWE2D(z, torch.full((ny, nx), 0.02, device=DEV), 0.5, 0.7, config=cfg, train_dem=False,
+              arithmetic=arithmetic)
+    level = torch.tensor([0.1], device=DEV)
+    run = lambda lam: adjoint_step(m, U, level, m.roughness_length, 0.01, lam.contiguous(), bed_grad=True)  # noqa: E731
+    mask = torch.zeros((ny, nx), device=DEV)
+    mask[patch[0]:patch[1], patch[2]:patch[3]] = 1.0
+    grow = lambda q: torch.nn.functional.max_pool2d(q[None, None], 2 * reach + 1, 1, reach)[0, 0]  # noqa: E731
+    near, inner = grow(mask) > 0, grow(1.0 - mask) == 0
+    full, part = run(dense), run(dense * mask)
+    for k in (0, 2, 3):  # the state, the roughness, the bed
+        a, b = full[k].reshape(-1, ny, nx), part[k].reshape(-1, ny, nx)
+        assert bool((b[:, ~near] == 0.0).all())
+        assert torch.equal(a[:, inner], b[:, inner])
