@@ -8,31 +8,13 @@
 // reference's: double-precision elapsed/remaining time, float32 max_dt and
 // float32 interpolation of the boundary series.
 #include <cuda_runtime.h>
-#include <float.h>
 #include <stdint.h>
 
+#include "swe_clock.cuh"
 #include "swe_common.cuh"
 
 namespace swe {
 namespace {
-
-// SWE2D._interpolate_dynamic_boundary (src/solver.py:391-415) in float32:
-// index = searchsorted(times, t, right=False) clamped to [1, n-1].
-__device__ float interpolate_level(const float* times, const float* levels, int n, float t) {
-    if (n == 1) return levels[0];
-    int lo = 0, hi = n;
-    while (lo < hi) {  // first index with times[i] >= t
-        const int mid = (lo + hi) >> 1;
-        if (times[mid] < t) lo = mid + 1;
-        else hi = mid;
-    }
-    const int idx = min(max(lo, 1), n - 1);
-    const float t0 = times[idx - 1], t1 = times[idx];
-    const float w0 = levels[idx - 1], w1 = levels[idx];
-    const float span = t1 - t0;
-    const float weight = __fdiv_rn(t - t0, fmaxf(span, FLT_EPSILON));
-    return w0 + weight * (w1 - w0);
-}
 
 __global__ void clock_kernel(swe_clock* c, uint32_t* red, const float* series_t,
                              const float* series_w, int nseries, float* level_out, const float* U,
@@ -46,58 +28,13 @@ __global__ void clock_kernel(swe_clock* c, uint32_t* red, const float* series_t,
         swe_clock cl = *c;
         const uint32_t red_status = red[2], red_dt = red[3];
         s_record_row = -1;
-        if (cl.active) {
-            // The step that just ran (solver.py:627-632, :765-768).
-            const uint32_t st = red_status;
-            const float dt = __uint_as_float(red_dt);
-            if (st & (SWE_S_NONFINITE_STATE | SWE_S_NONFINITE_DT | SWE_S_NONPOSITIVE_DT)) {
-                cl.state = SWE_CLOCK_FAILED;
-                cl.dt_status = st;
-                cl.last_dt = dt;
-                cl.active = 0;
-            } else {
-                double elapsed = cl.elapsed + (double)dt;
-                if (elapsed > cl.duration && elapsed - cl.duration <= cl.tolerance) elapsed = cl.duration;
-                cl.elapsed = elapsed;
-                cl.last_dt = dt;
-                cl.steps += 1;
-                if (gauges && gauge_rows > 0) {
-                    const int row = (cl.steps - 1) % gauge_rows;
-                    gauges[(size_t)row * (2 + ngauge)] = cl.start + elapsed;
-                    gauges[(size_t)row * (2 + ngauge) + 1] = (double)dt;
-                    s_record_row = row;
-                }
-            }
+        if (clock_finish_step(cl, red_status, __uint_as_float(red_dt)) && gauges && gauge_rows > 0) {
+            const int row = (cl.steps - 1) % gauge_rows;
+            gauges[(size_t)row * (2 + ngauge)] = cl.start + cl.elapsed;
+            gauges[(size_t)row * (2 + ngauge) + 1] = (double)cl.last_dt;
+            s_record_row = row;
         }
-        if (cl.state == SWE_CLOCK_RUNNING) {
-            // The next step (solver.py:741-760).
-            // The loop runs out of iterations before it checks the remaining
-            // time again, so max_steps is tested first.
-            const double remaining = cl.duration - cl.elapsed;
-            if (cl.steps >= cl.max_steps) {
-                cl.state = SWE_CLOCK_MAXSTEPS;
-                cl.active = 0;
-            } else if (remaining <= cl.tolerance) {
-                cl.state = SWE_CLOCK_DONE;
-                cl.active = 0;
-            } else {
-                double step_max_dt = remaining;
-                if (cl.max_dt_cap > 0.0 && cl.max_dt_cap < remaining) step_max_dt = cl.max_dt_cap;
-                cl.max_dt = (float)step_max_dt;
-                const double current = cl.start + cl.elapsed;
-                if (nseries > 0) {
-                    const float lev = interpolate_level(series_t, series_w, nseries, (float)current);
-                    cl.level = lev;
-                    level_out[0] = lev;
-                }
-                red[0] = 0u;
-                red[1] = 0u;
-                red[2] = 0u;
-                cl.active = 1;
-            }
-        } else {
-            cl.active = 0;
-        }
+        clock_set_up(cl, series_t, series_w, nseries, level_out, red);
         *c = cl;
     }
     __syncthreads();

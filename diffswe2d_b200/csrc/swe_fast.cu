@@ -423,7 +423,8 @@ __device__ __forceinline__ void fast_tile(const StepArgs& a, int bx, int by, int
 template <int STAGE, int FRIC>
 __global__ void __launch_bounds__(SW_WARPS * 32, 8) fast_kernel(const StepArgs a) {
     chain_start();
-    fast_tile<STAGE, FRIC, false>(a, blockIdx.x, blockIdx.y, blockIdx.z, a.rows);
+    if (clock_row<STAGE>(a)) return;
+    fast_tile<STAGE, FRIC, false>(a, blockIdx.x, tile_row<STAGE>(a), blockIdx.z, a.rows);
 }
 
 struct FastTile {
@@ -447,6 +448,7 @@ int fast_launch_stages(int stage, const StepArgs& a, dim3 grid, cudaStream_t s) 
     cudaError_t e = cudaSuccess;
     if (stage & 1) e = launch_chained(fast_kernel<1, 0>, grid, threads, s, a);
     if ((stage & 2) && e == cudaSuccess) {
+        if (a.next_clk != nullptr) grid.y += 1;
         if (!a.friction) e = launch_chained(fast_kernel<2, 0>, grid, threads, s, a);
         else if (a.friction_model == 0) e = launch_chained(fast_kernel<2, 1>, grid, threads, s, a);
         else e = launch_chained(fast_kernel<2, 2>, grid, threads, s, a);

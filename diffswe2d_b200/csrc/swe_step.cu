@@ -133,10 +133,11 @@ __global__ void __launch_bounds__(NT) stage_kernel(const StepArgs a) {
     __shared__ FaceFlux s_fx[TY][TX + 1], s_fy[TY + 1][TX];
 
     chain_start();
+    if (clock_row<STAGE>(a)) return;
     const SweConsts& kc = a.kc;
     const int tid = threadIdx.x;
     const int b = blockIdx.z;
-    const int i0 = blockIdx.x * TX, j0 = blockIdx.y * TY;
+    const int i0 = blockIdx.x * TX, j0 = tile_row<STAGE>(a) * TY;
 
     if (a.clk != nullptr && !a.clk->active) {
         // A step after the end of the call: the state is carried over unchanged.
@@ -160,10 +161,8 @@ __global__ void __launch_bounds__(NT) stage_kernel(const StepArgs a) {
         const float max_dt = a.clk != nullptr ? a.clk->max_dt : a.max_dt;
         dt = st != st ? st : fminf(st, max_dt);
         hdt = 0.5f * dt;
-        if (tid == 0 && blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0) {
-            uint32_t st_bits = 0;
-            if (!isfinite(dt)) st_bits |= SWE_S_NONFINITE_DT;
-            else if (!(dt > 0.0f)) st_bits |= SWE_S_NONPOSITIVE_DT;
+        if (tid == 0 && i0 == 0 && j0 == 0 && b == 0) {
+            const uint32_t st_bits = dt_status(dt);
             if (st_bits) atomicOr(&a.red[2], st_bits);
             a.red[3] = f2u(dt);
         }
@@ -465,7 +464,8 @@ __device__ __forceinline__ void sweep_tile(const StepArgs& a, int bx, int by, in
 template <int STAGE, int FRIC>
 __global__ void __launch_bounds__(SW_WARPS * 32, 8) sweep_kernel(const StepArgs a) {
     chain_start();
-    sweep_tile<STAGE, FRIC, false>(a, blockIdx.x, blockIdx.y, blockIdx.z, a.rows);
+    if (clock_row<STAGE>(a)) return;
+    sweep_tile<STAGE, FRIC, false>(a, blockIdx.x, tile_row<STAGE>(a), blockIdx.z, a.rows);
 }
 
 
@@ -645,11 +645,22 @@ extern "C" int swe_spatial_operator_f32(const float* U, const float* bed, int B,
 namespace swe {
 namespace {
 
+// Where stage 2 leaves the clock of the following step.
+struct NextClock {
+    swe_clock* clock;
+    uint32_t* red;
+    float* level;
+    const float* series_t;
+    const float* series_w;
+    int nseries;
+};
+
 int launch_step(int stage, const float* U, const float* bed, int bedB, const float* n, int nB, int B,
                 int ny, int nx, const swe_params* p, const float* level, int levelB, float max_dt,
                 const swe_clock* clk, const float* rain, int rain_mode, int rain_batch,
                 const float* infil, int infil_mode, int infil_batch, float* scratch_k, uint32_t* red,
-                float* U_out, float* hmax, void* stream, float* k2_out = nullptr) {
+                float* U_out, float* hmax, void* stream, float* k2_out = nullptr,
+                const NextClock* next = nullptr) {
     StepArgs a{};
     if (stage != 1 && stage != 2 && stage != 3) return SWE_EARG;
     if (!fill_common(a, U, bed, B, bedB, ny, nx, p, level, levelB)) return SWE_EARG;
@@ -672,11 +683,20 @@ int launch_step(int stage, const float* U, const float* bed, int bedB, const flo
     a.clk = clk;
     a.hmax = hmax;
     a.k2_out = k2_out;
+    if (next != nullptr) {
+        a.next_clk = next->clock;
+        a.next_red = next->red;
+        a.next_level = next->level;
+        a.series_t = next->series_t;
+        a.series_w = next->series_w;
+        a.nseries = next->nseries;
+    }
     cudaStream_t s = (cudaStream_t)stream;
     const bool fast = p->arithmetic == SWE_ARITH_FAST;
     const bool tiled = !fast && use_tiled_kernels(a);
-    const dim3 g = tiled ? grid_of(a) : sweep_grid_of(a);
-    // A clocked step's reduction words are cleared by swe_clock_f32.
+    dim3 g = tiled ? grid_of(a) : sweep_grid_of(a);
+    if (next != nullptr && g.y >= 65535u) return SWE_EARG;  // no room for the clock's row
+    // A clocked step's reduction words are cleared when the clock is advanced.
     if ((stage & 1) && !clk && cudaMemsetAsync(red, 0, SWE_RED_WORDS * sizeof(uint32_t), s) != cudaSuccess)
         return SWE_ECUDA;
     if (fast) return fast_launch_stages(stage, a, g, s);
@@ -687,6 +707,7 @@ int launch_step(int stage, const float* U, const float* bed, int bedB, const flo
         else e = launch_chained(sweep_kernel<1, 0>, g, th, s, a);
     }
     if ((stage & 2) && e == cudaSuccess) {
+        if (next != nullptr) g.y += 1;
         if (tiled) {
             e = launch_chained(stage_kernel<2>, g, dim3(NT), s, a);
         } else if (!a.friction) {
@@ -736,6 +757,21 @@ extern "C" int swe_step_clocked_f32(int stage, const float* U, const float* bed,
     return launch_step(stage, U, bed, bedB, n, nB, B, ny, nx, p, level, levelB, 0.0f, clock, nullptr,
                        SWE_FORCING_NONE, 1, infil, infil_mode, infil_batch, scratch_k, red, U_out, hmax,
                        stream);
+}
+
+extern "C" int swe_step_clocked_next_f32(const float* U, const float* bed, int bedB, const float* n, int nB, int B,
+                                         int ny, int nx, const swe_params* p, const float* level, int levelB,
+                                         const swe_clock* clock, const float* infil, int infil_mode,
+                                         int infil_batch, float* scratch_k, uint32_t* red, float* U_out,
+                                         float* hmax, swe_clock* next_clock, uint32_t* next_red,
+                                         const float* series_t, const float* series_w, int nseries,
+                                         float* next_level, void* stream) {
+    if (!clock || !next_clock || next_clock == clock || !next_red || next_red == red || nseries < 0) return SWE_EARG;
+    if (nseries > 0 && (!series_t || !series_w || !next_level || next_level == level)) return SWE_EARG;
+    const NextClock next{next_clock, next_red, next_level, series_t, series_w, nseries};
+    return launch_step(3, U, bed, bedB, n, nB, B, ny, nx, p, level, levelB, 0.0f, clock, nullptr,
+                       SWE_FORCING_NONE, 1, infil, infil_mode, infil_batch, scratch_k, red, U_out, hmax,
+                       stream, nullptr, &next);
 }
 
 extern "C" int swe_step_clocked_k2_f32(int stage, const float* U, const float* bed, int bedB,

@@ -607,11 +607,15 @@ class _DeviceLoop:
         self.chunk = int(chunk)
         self.bufs = [torch.empty((B, 3, ny, nx), device=dev), torch.empty((B, 3, ny, nx), device=dev)]
         self.scratch = torch.empty((B, 3, ny, nx), device=dev)
-        self.red = torch.zeros(nat.RED_WORDS, dtype=torch.int32, device=dev)
+        # Two sets of clock, reduction words and level: each step's second
+        # stage leaves the next step's in the other set.  With gauges to
+        # record after every step a clock kernel follows it instead, on the
+        # first set (so does a grid too high for another row of tiles).
+        self.red = torch.zeros((2, nat.RED_WORDS), dtype=torch.int32, device=dev)
         self.hmax = torch.empty((B, ny, nx), device=dev)
         self.bed = torch.empty(bed_shape, device=dev)
         self.n = torch.empty(n_shape, device=dev)
-        self.lv = torch.zeros(levelB, device=dev)
+        self.lv = torch.zeros((2, levelB), device=dev)
         self.nseries = 0 if series is None else series[0].numel()
         self.series_t = None if series is None else torch.empty(self.nseries, device=dev)
         self.series_w = None if series is None else torch.empty(self.nseries, device=dev)
@@ -622,7 +626,8 @@ class _DeviceLoop:
                       if cells else None)
         self.gbuf = (torch.zeros((self.chunk, 2 + self.ncells), dtype=torch.float64, device=dev)
                      if cells else None)
-        self.clock = torch.zeros(72, dtype=torch.uint8, device=dev)
+        self.clock = torch.zeros((2, 72), dtype=torch.uint8, device=dev)
+        self.chained_clock = not cells and ny < 65535
         self.clock_host = torch.zeros(72, dtype=torch.uint8).pin_memory()
         self.params = params
         self.arithmetic = model.arithmetic
@@ -643,14 +648,23 @@ class _DeviceLoop:
             nat.stream_handle(self.dev))
         nat.check(rc, "forward clock")
 
-    def _step(self, src, dst):
-        rc = nat.lib().swe_step_clocked_f32(
-            3, nat.ptr(src), nat.ptr(self.bed), self.bed.shape[0], nat.ptr(self.n), self.n.shape[0],
-            self.B, self.ny, self.nx, self.params, nat.ptr(self.lv), self.levelB,
-            nat.ptr(self.clock), nat.ptr(self.infil), self.imode, self.iB, nat.ptr(self.scratch),
-            nat.ptr(self.red), nat.ptr(dst), nat.ptr(self.hmax), nat.stream_handle(self.dev))
-        nat.check(rc, "forward step")
-        self._clock_tick(dst)
+    def _step(self, s):
+        """Step s of a graph, bufs[s % 2] to the other, and the clock after it."""
+        src, dst = self.bufs[s % 2], self.bufs[1 - s % 2]
+        cur = s % 2 if self.chained_clock else 0
+        args = (nat.ptr(src), nat.ptr(self.bed), self.bed.shape[0], nat.ptr(self.n), self.n.shape[0],
+                self.B, self.ny, self.nx, self.params, nat.ptr(self.lv[cur]), self.levelB,
+                nat.ptr(self.clock[cur]), nat.ptr(self.infil), self.imode, self.iB, nat.ptr(self.scratch),
+                nat.ptr(self.red[cur]), nat.ptr(dst), nat.ptr(self.hmax))
+        if self.chained_clock:
+            rc = nat.lib().swe_step_clocked_next_f32(
+                *args, nat.ptr(self.clock[1 - cur]), nat.ptr(self.red[1 - cur]), nat.ptr(self.series_t),
+                nat.ptr(self.series_w), self.nseries, nat.ptr(self.lv[1 - cur]), nat.stream_handle(self.dev))
+            nat.check(rc, "forward step")
+        else:
+            rc = nat.lib().swe_step_clocked_f32(3, *args, nat.stream_handle(self.dev))
+            nat.check(rc, "forward step")
+            self._clock_tick(dst)
 
     def run(self, U0, bed, n, lv, series, infil, clock):
         """Yields (state buffer, clock) after each replay until the call ends."""
@@ -659,14 +673,14 @@ class _DeviceLoop:
         self.bed.copy_(bed)
         self.n.copy_(n)
         if lv is not None:
-            self.lv.copy_(lv.reshape(-1))
+            self.lv.copy_(lv.reshape(1, -1).expand_as(self.lv))
         if series is not None:
             self.series_t.copy_(series[0])
             self.series_w.copy_(series[1])
         if infil is not None:
             self.infil.copy_(infil)
         self.clock_host.copy_(torch.frombuffer(bytearray(bytes(clock)), dtype=torch.uint8))
-        self.clock.copy_(self.clock_host, non_blocking=True)
+        self.clock[0].copy_(self.clock_host, non_blocking=True)
         self._clock_tick(self.bufs[0])  # sets up the first step
         if not self.graphs:
             from .autotune import sweep_rows, tuned_rows_for_shape
@@ -678,7 +692,7 @@ class _DeviceLoop:
                     graph = torch.cuda.CUDAGraph()
                     with torch.cuda.graph(graph):
                         for s in range(n):
-                            self._step(self.bufs[s % 2], self.bufs[1 - s % 2])
+                            self._step(s)
                     self.graphs[n] = graph
         def size_for(left):
             return replay_length(self.sizes, left)
@@ -686,7 +700,7 @@ class _DeviceLoop:
         n = size_for(clock.duration / self.dt_hint) if self.dt_hint > 0 else self.chunk
         while True:
             self.graphs[n].replay()
-            c = nat.SweClock.from_buffer_copy(self.clock.cpu().numpy().tobytes())
+            c = nat.SweClock.from_buffer_copy(self.clock[0].cpu().numpy().tobytes())
             if c.steps > 0 and c.elapsed > 0:
                 self.dt_hint = float(c.elapsed) / c.steps
             yield self.bufs[0], c

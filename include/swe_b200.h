@@ -286,6 +286,22 @@ int swe_step_clocked_f32(int stage, const float* U, const float* bed, int bedB, 
                          float* hmax, void* stream);
 
 /*
+ * Both stages of swe_step_clocked_f32 and, while stage 2 runs, what
+ * swe_clock_f32 (without gauges) does after them, into a second set: the
+ * clock after this step into next_clock, the boundary level of the next step
+ * into next_level[0] (nseries > 0), and next_red cleared if there is a next
+ * step.  The next step takes next_clock, next_red and next_level, and leaves
+ * its own in this step's.  The two sets may not be the same; the grid has at
+ * most 65534 rows of tiles.
+ */
+int swe_step_clocked_next_f32(const float* U, const float* bed, int bedB, const float* n, int nB, int B,
+                              int ny, int nx, const swe_params* p, const float* level, int levelB,
+                              const swe_clock* clock, const float* infil, int infil_mode, int infil_batch,
+                              float* scratch_k, uint32_t* red, float* U_out, float* hmax,
+                              swe_clock* next_clock, uint32_t* next_red, const float* series_t,
+                              const float* series_w, int nseries, float* next_level, void* stream);
+
+/*
  * swe_step_clocked_f32 (stage 2 or 3) that also writes stage 2's tendency
  * k2 = rhs(P) at the predictor P (solver.py:641) into k2_out [B,3,ny,nx],
  * as the step computes it, for an adjoint pass that then need not

@@ -52,3 +52,50 @@ def test_bed_kernel_equals_the_bed_property():
         with torch.no_grad():
             m.dem_correction_parameter.copy_(torch.randn(shape, generator=g))
         assert torch.equal(m._bed_values(), m.bed.detach())
+
+
+# one tile, several, the row sweeps (the last grid also in the IEEE mode)
+@pytest.mark.parametrize("ny,nx", [(2, 2), (9, 40), (65, 129), (1250, 1260)])
+@pytest.mark.parametrize("arithmetic", ["exact", "fast"])
+@pytest.mark.parametrize("ends", ["duration", "cap", "max_steps"])
+@pytest.mark.parametrize("calm", [False, True])
+def test_clock_advanced_by_the_step_equals_the_clock_kernel(ny, nx, arithmetic, ends, calm):
+    """A run with a gauge has a clock kernel between two steps, one without
+    advances the clock inside the second stage: the same steps, bits, number
+    of steps and errors (the rough states of some sizes go non-finite)."""
+    if ny > 1000 and ends != "duration":
+        pytest.skip("covered by the smaller grids")
+    z, U = _site(ny, nx, ny * 1000 + nx)
+    if calm:
+        U = torch.cat([torch.clamp(0.1 - z, min=0.0)[None], 0.01 * U[1:] * (z < 0.05)])
+    cfg = SWEConfig(boundary_left="water_level", boundary_right="wall", boundary_top="wall", boundary_bottom="absorbing")
+    kw = {"duration": {}, "cap": dict(max_dt_cap=4e-4), "max_steps": dict(max_steps=5)}[ends]
+    out = []
+    for gauges in ({}, {"g": (1, 1)}):
+        m = SWE2D(z, torch.full_like(z, 0.02), 0.05, 0.07, config=cfg, train_dem=False, arithmetic=arithmetic)
+        t = torch.linspace(0.0, 0.05, 33, device=DEV)
+        m.set_dynamic_boundary(t, 0.1 + 0.05 * torch.sin(200.0 * t))
+        m.gauge_indices, m.track_gauges = gauges, bool(gauges)
+        with torch.no_grad():
+            for t_end in (0.01, 0.05):  # the second finds another call's clock and level in the buffers
+                try:
+                    V, hmax = m(U[None], t_end=t_end, **kw)
+                    out.append((m.last_forward_steps, V, hmax))
+                except (FloatingPointError, RuntimeError) as err:
+                    assert not calm or ends == "max_steps"
+                    out.append((str(err),))
+    for a, b in ((out[0], out[2]), (out[1], out[3])):
+        assert a[0] == b[0]
+        assert all(torch.equal(p, q) for p, q in zip(a[1:], b[1:]))
+
+
+def test_clocked_step_refuses_a_shared_set():
+    from diffswe2d_b200 import _native as nat
+    z, U = _site(9, 40, 1)
+    m = SWE2D(z, torch.full_like(z, 0.02), 0.5, 0.7, train_dem=False)
+    buf = torch.zeros((4, 256), device=DEV)
+    p = lambda k: nat.ptr(buf[k])  # noqa: E731
+    args = [nat.ptr(U), nat.ptr(z), 1, nat.ptr(z), 1, 1, 9, 40, m._params(), p(0), 1, p(1), None, 0, 1, nat.ptr(U),
+            p(2), nat.ptr(U), None]
+    rc = nat.lib().swe_step_clocked_next_f32(*args, p(1), p(3), None, None, 0, None, nat.stream_handle(torch.device(DEV, 0)))
+    assert rc == nat.SWE_EARG
