@@ -48,7 +48,7 @@ def _cache_file() -> Path:
 
 
 #: generation of the step kernels: choices timed with other kernels are not used
-KERNELS = 2
+KERNELS = 3
 
 
 def _device_key(device) -> str:
