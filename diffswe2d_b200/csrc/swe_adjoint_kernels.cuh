@@ -33,7 +33,9 @@ constexpr int ADJ_TX = 32;  // tile columns
 // Blocks per SM the tile kernel is compiled for (80 registers, no spills).
 // Measured with 16-row tiles at 4 x 244 x 393, stage 2 / stage 1: three
 // 58.5 / 52.0 us, two 69 / 60; with 8-row tiles (37 KB instead of 65) at
-// three, four and five blocks 67 / 59, 64 / 57 and 66 / 59.
+// three, four and five blocks 67 / 59, 64 / 57 and 66 / 59, all with every
+// cell evaluated; where zero cotangents are skipped 8 rows and four blocks
+// come out level (44 / 39 against 45 / 39).
 #ifndef SWE_ADJ_TILE_MINB
 #define SWE_ADJ_TILE_MINB 3
 #endif
