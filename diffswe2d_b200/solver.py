@@ -628,6 +628,7 @@ class _DeviceLoop:
                      if cells else None)
         self.clock = torch.zeros((2, 72), dtype=torch.uint8, device=dev)
         self.chained_clock = not cells and ny < 65535
+        self.calls = None
         self.clock_host = torch.zeros(72, dtype=torch.uint8).pin_memory()
         self.params = params
         self.arithmetic = model.arithmetic
@@ -650,21 +651,25 @@ class _DeviceLoop:
 
     def _step(self, s):
         """Step s of a graph, bufs[s % 2] to the other, and the clock after it."""
-        src, dst = self.bufs[s % 2], self.bufs[1 - s % 2]
-        cur = s % 2 if self.chained_clock else 0
-        args = (nat.ptr(src), nat.ptr(self.bed), self.bed.shape[0], nat.ptr(self.n), self.n.shape[0],
+        if self.calls is None:  # the arguments of an even and an odd step, once for the graphs
+            self.calls = [self._step_args(0), self._step_args(1)]
+        st = nat.stream_handle(self.dev)
+        if self.chained_clock:
+            nat.check(nat.lib().swe_step_clocked_next_f32(*self.calls[s % 2], st), "forward step")
+        else:
+            nat.check(nat.lib().swe_step_clocked_f32(3, *self.calls[s % 2], st), "forward step")
+            self._clock_tick(self.bufs[1 - s % 2])
+
+    def _step_args(self, odd):
+        cur = odd if self.chained_clock else 0
+        args = (nat.ptr(self.bufs[odd]), nat.ptr(self.bed), self.bed.shape[0], nat.ptr(self.n), self.n.shape[0],
                 self.B, self.ny, self.nx, self.params, nat.ptr(self.lv[cur]), self.levelB,
                 nat.ptr(self.clock[cur]), nat.ptr(self.infil), self.imode, self.iB, nat.ptr(self.scratch),
-                nat.ptr(self.red[cur]), nat.ptr(dst), nat.ptr(self.hmax))
+                nat.ptr(self.red[cur]), nat.ptr(self.bufs[1 - odd]), nat.ptr(self.hmax))
         if self.chained_clock:
-            rc = nat.lib().swe_step_clocked_next_f32(
-                *args, nat.ptr(self.clock[1 - cur]), nat.ptr(self.red[1 - cur]), nat.ptr(self.series_t),
-                nat.ptr(self.series_w), self.nseries, nat.ptr(self.lv[1 - cur]), nat.stream_handle(self.dev))
-            nat.check(rc, "forward step")
-        else:
-            rc = nat.lib().swe_step_clocked_f32(3, *args, nat.stream_handle(self.dev))
-            nat.check(rc, "forward step")
-            self._clock_tick(dst)
+            args += (nat.ptr(self.clock[1 - cur]), nat.ptr(self.red[1 - cur]), nat.ptr(self.series_t),
+                     nat.ptr(self.series_w), self.nseries, nat.ptr(self.lv[1 - cur]))
+        return args
 
     def run(self, U0, bed, n, lv, series, infil, clock):
         """Yields (state buffer, clock) after each replay until the call ends."""
