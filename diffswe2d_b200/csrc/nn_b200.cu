@@ -396,11 +396,11 @@ __global__ void __launch_bounds__(NT, 1) gemm_kernel(const GemmArgs g) {
         const uint32_t sA = base + st * stage_bytes, sB = sA + tile_bytes(BM);
         const uint32_t full = full0 + 8 * st, freed = free0 + 8 * st;
         for (int kb = st; kb < nkb; kb += S) {
-            if (kb >= S && !mbar_wait(freed, (uint32_t)(((kb >> log_s) - 1) & 1), g.wait_ns)) {
-                s_ok = 0;
-                break;
-            }
-            if (!s_ok) break;
+            // one decision for the warp: each lane probes and reads the clock by
+            // itself, and at the limit they may disagree
+            const bool freed_ok = kb < S || mbar_wait(freed, (uint32_t)(((kb >> log_s) - 1) & 1), g.wait_ns);
+            if (!freed_ok) s_ok = 0;
+            if (!__all_sync(0xffffffffu, freed_ok && s_ok)) break;
             const int k0 = kbeg + kb * BK;
             stage_tile<A_MN>(sA, g.A, m0, BM, k0, kend, part, parts);
             stage_tile<B_MN>(sB, g.B, n0, bn, k0, kend, part, parts);

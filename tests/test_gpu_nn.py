@@ -325,3 +325,26 @@ def test_network_pass_equals_elementary_kernels(nb):
     for i in range(6):
         assert torch.equal(net.weight_grad(i), dW[i])
         assert bool(((net.bias_grad(i).double() - db[i][0]).abs() <= 600 * 2.0 ** -24 * db[i][1] + 1e-30).all())
+
+
+@pytest.mark.parametrize("wait_ns", [1, 300, 1000, 3000, 20000])
+def test_gemm_wait_limit_that_runs_out_midway(wait_ns):
+    """Limits about as long as the waits: some CTAs, and some lanes of a
+    warp, give up where others do not.  The launch returns, a word of 0 means
+    a correct product and 1 that a wait gave up, and the next call with the
+    normal limit is correct.  70 K blocks in up to eight stages."""
+    rng = np.random.default_rng(6)
+    M, N, K = 1024, 96, 4480
+    A, B = _bf16_dev(rng.normal(size=(M, K))), _bf16_dev(rng.normal(size=(N, K)))
+    full, _, _ = _gemm(A, B, M, N, K, K, K)
+    out = torch.empty((M, N), device=DEV)
+    z, s = ctypes.c_void_p(0), nat.stream_handle(torch.device(DEV))
+    for _ in range(20):
+        err = torch.zeros(1, dtype=torch.int32, device=DEV)
+        nat.check(nat.lib().nn_gemm_bf16(nat.ptr(A), K, nat.ptr(B), K, M, N, K, z, 0, nat.ptr(out), z, z, N, 1,
+                                         z, wait_ns, nat.ptr(err), s), "gemm")
+        code = int(err.item())
+        assert code in (0, 1)
+        assert code == 1 or np.array_equal(out.cpu().numpy(), full)
+    again, _, _ = _gemm(A, B, M, N, K, K, K)
+    assert np.array_equal(again, full)
