@@ -477,8 +477,8 @@ class SWE2D(nn.Module):
                            f"requested duration={duration:.8f} s.")
 
     # ------------------------------------------------ device-driven forward
-    #: steps per CUDA-graph replay of the device-driven loop (even: the state
-    #: ping-pongs between two buffers and ends each chunk in the first)
+    #: steps per CUDA-graph replay of the device-driven loop (the next even
+    #: number is used: see ``even_chunk``)
     steps_per_chunk = 32
 
     def _device_loop_ok(self, U0, callback, boundary_level, max_dt_cap) -> bool:
@@ -501,9 +501,10 @@ class SWE2D(nn.Module):
         """forward() with the time loop on the device (src/solver.py:680-779).
 
         Each chunk of ``steps_per_chunk`` steps is one replay of a CUDA graph
-        of [stage 1, stage 2, clock] launches; the host reads the 72-byte
-        clock once per chunk.  The graph and its buffers are captured once per
-        shape and configuration (``_DeviceLoop``) and reused by later calls.
+        of [stage 1, stage 2] launches (stage 2 advances the clock; with gauges
+        a clock launch follows each step); the host reads the 72-byte clock
+        once per chunk.  The graph and its buffers are captured once per shape
+        and configuration (``_DeviceLoop``) and reused by later calls.
         Results are those of the host loop bit for bit.
         """
         self._check_state(U0)
@@ -530,14 +531,15 @@ class SWE2D(nn.Module):
                 raise ValueError(f"gauge cell {(iy, ix)} outside the {ny}x{nx} grid")
             cells.append((int(iy), int(ix)))
         p = self._params()
+        chunk = even_chunk(self.steps_per_chunk)
         key = (B, ny, nx, str(dev), bed.shape[0], n.shape[0], levelB,
                None if series is None else series[0].numel(), tuple(cells), imode, iB,
-               None if infil is None else tuple(infil.shape), self.steps_per_chunk, bytes(p))
+               None if infil is None else tuple(infil.shape), chunk, bytes(p))
         loops = self.__dict__.setdefault("_device_loops", {})
         loop = loops.get(key)
         if loop is None:
             loop = _DeviceLoop(self, key, B, ny, nx, dev, bed.shape, n.shape, levelB, series, cells,
-                               infil, imode, iB, p, self.steps_per_chunk)
+                               infil, imode, iB, p, chunk)
             loops[key] = loop
         cap = self._scalar_float(max_dt_cap, "max_dt_cap") if max_dt_cap is not None else 0.0
         clock = nat.SweClock(duration, absolute_start, max(1e-12, 1e-12 * abs(duration)), cap, 0.0,
@@ -579,6 +581,16 @@ class SWE2D(nn.Module):
             bed = float(current_bed[0, 0, iy, ix].detach().cpu())
             self.ts_h[name].append(depth)
             self.ts_z[name].append(depth + bed)
+
+
+def even_chunk(chunk: int) -> int:
+    """The even number of steps that a chunk length stands for: the state and
+    the clock alternate between two buffers, and a replay has to leave both
+    in the first."""
+    n = int(chunk)
+    if n < 1:
+        raise ValueError(f"steps_per_chunk must be positive, got {chunk!r}.")
+    return n + n % 2
 
 
 def replay_lengths(chunk: int):

@@ -69,3 +69,13 @@ def test_rainfall_at_a_host_time_equals_the_tensor_expression():
     assert float(f.rates[0].sum()) > 0
     with pytest.raises(ValueError):
         RainfallForcing(times.flip(0), f.rates)
+
+
+def test_chunks_of_an_odd_length_are_rounded_up():
+    import pytest
+    from diffswe2d_b200.solver import even_chunk
+    assert [even_chunk(c) for c in (1, 2, 3, 31, 32, 32.0)] == [2, 2, 4, 32, 32, 32]
+    assert all(n % 2 == 0 for c in range(1, 40) for n in replay_lengths(even_chunk(c)))
+    for bad in (0, -2):
+        with pytest.raises(ValueError):
+            even_chunk(bad)

@@ -99,3 +99,20 @@ def test_clocked_step_refuses_a_shared_set():
             p(2), nat.ptr(U), None]
     rc = nat.lib().swe_step_clocked_next_f32(*args, p(1), p(3), None, None, 0, None, nat.stream_handle(torch.device(DEV, 0)))
     assert rc == nat.SWE_EARG
+
+
+@pytest.mark.parametrize("gauges", [{}, {"g": (1, 1)}])
+def test_odd_chunks_give_the_steps_of_even_ones(gauges):
+    z, U = _site(37, 53, 3)
+    U = torch.cat([torch.clamp(0.1 - z, min=0.0)[None], 0.01 * U[1:] * (z < 0.05)])
+    out = []
+    for chunk in (32, 1, 3):
+        m = SWE2D(z, torch.full_like(z, 0.02), 0.05, 0.07, train_dem=False)
+        m.steps_per_chunk = chunk
+        m.gauge_indices, m.track_gauges = gauges, bool(gauges)
+        with torch.no_grad():
+            V, hmax = m(U[None], t_end=0.1, boundary_level=0.1)
+        out.append((m.last_forward_steps, list(m.ts_time), V, hmax))
+    assert out[0][0] > 3
+    for b in out[1:]:
+        assert b[:2] == out[0][:2] and torch.equal(b[2], out[0][2]) and torch.equal(b[3], out[0][3])
