@@ -909,8 +909,10 @@ __global__ void __launch_bounds__(ADJ_THREADS) adj_edge_kernel(const AdjArgs a) 
             if (!touches || (code == SWE_BC_CONSTANT && !BEDG)) continue;
             // a band holds the records of its own side's ghosts, and in stage 2
             // of those at the ends of its two lines
-            if (bs >= 0 && (bs == side || (PRED && (bs < 2) == yax))) {
-                band_sum(band, yax == (bs >= 2), far, e, yax ? i : j, g, n, l);
+            if (level_side(a, side)) {
+                band_sum(LevelBand(a, b, side), true, (side & 1) != 0, 0, yax ? i : j, g, n, l);
+            } else if (PRED && bs >= 0 && (bs < 2) == yax) {
+                band_sum(band, false, far, e, yax ? i : j, g, n, l);
             } else {
                 const float* gl = yax ? a.gy + 4 * (((size_t)b * 4 + (q - 4)) * nx + i)
                                       : a.gx + 4 * (((size_t)b * 4 + q) * ny + j);

@@ -577,3 +577,40 @@ def test_step_adjoint_of_a_patch_of_cotangents(patch, arithmetic):
         a, b = full[k].reshape(-1, ny, nx), part[k].reshape(-1, ny, nx)
         assert bool((b[:, ~near] == 0.0).all())
         assert torch.equal(a[:, inner], b[:, inner])
+
+
+def _member_level_adjoints(z, U, lam, sides, level):
+    """Level adjoint of every batch member of one tendency ([B])."""
+    from diffswe2d_b200.adjoint import AdjointStepper
+    cfg = SWEConfig(**dict(zip(("boundary_left", "boundary_right", "boundary_top", "boundary_bottom"), sides)))
+    B, _, ny, nx = U.shape
+    m = SWE2D(z, torch.full_like(z, 0.02), 0.5, 0.7, config=cfg, train_dem=False)
+    st = AdjointStepper(m, B, ny, nx, torch.device(DEV), B)
+    st._spatial(U.contiguous(), level, lam.contiguous(), torch.zeros_like(U), st.part[1], "adjoint")
+    return st.part[1].reshape(B, -1).sum(1)
+
+
+def _member_states(B, ny, nx, seed):
+    g = torch.Generator().manual_seed(seed)
+    z = torch.rand((B, 1, ny, nx), generator=g) * 0.1 - 0.3
+    h = 0.05 - z + 0.02 * torch.randn(z.shape, generator=g)
+    U = torch.cat([h, 0.3 * h * torch.randn((B, 2, ny, nx), generator=g)], 1)
+    return z.to(DEV), U.to(DEV), 0.05 + 0.02 * torch.randn(B, generator=g).to(DEV)
+
+
+@pytest.mark.parametrize("kinds", [("water_level", "absorbing"), ("absorbing", "water_level"),
+                                   ("water_level", "water_level")])
+def test_level_adjoint_at_a_corner_of_two_level_sides(kinds):
+    """A cotangent in cell (0, 1) alone reaches the left ghosts of row 0 and
+    the top ghosts of column 1: with both sides on the level its adjoint is
+    the rounded sum of what the two give with a wall in the other's place,
+    bit for bit, because each side's ghosts are evaluated face by face."""
+    z, U, level = _member_states(256, 33, 40, 5)
+    lam = torch.zeros_like(U)
+    lam[:, :, 0, 1] = torch.randn((256, 3), generator=torch.Generator().manual_seed(6)).to(DEV)
+    left, top = kinds
+    a = _member_level_adjoints(z, U, lam, (left, "wall", "wall", "wall"), level)
+    b = _member_level_adjoints(z, U, lam, ("wall", "wall", top, "wall"), level)
+    both = _member_level_adjoints(z, U, lam, (left, "wall", top, "wall"), level)
+    assert int((a != 0).sum()) > 16 and int((b != 0).sum()) > 16
+    assert torch.equal(both, a + b)
