@@ -220,11 +220,11 @@ __device__ State padded_state(const AdjArgs& a, int b, int j, int i, float scale
 
 // ------------------------------------------------------------ level bands
 // Along a side whose ghosts depend on the level, the adjoints of its ghosts
-// are summed from face records (swe_adjoint.cuh, namespace line): of the
-// faces normal to the side, d = 0, 1 lines away from it.  In stage 2 also
-// those of the two lines of cells next to it, which stage 1's ghosts take
-// their cotangents from: normal faces to d = 3 and the faces along each line
-// of cells, e = 0, 1.  A record holds the face's contributions to its
+// and of the two lines of cells next to it are summed from face records
+// (swe_adjoint.cuh, namespace line): of the faces normal to the side, d = 0
+// to 3 lines away from it, and of the faces along each line of cells, e = 0,
+// 1.  (The cells because a second call's ghosts take their cotangents from
+// what this one makes of them.)  A record holds the face's contributions to its
 // four cells, 4 x (U0, U1, U2, Z).  Grids too small for the scratch buffers
 // (either side below BAND_MIN cells) do without.
 constexpr int BAND_MIN = 32;
@@ -284,12 +284,11 @@ __device__ void band_face(const AdjArgs& a, int b, bool diry, int f, int row, fl
 }
 
 // Faces of all bands of a batch member.
-__host__ __device__ inline long long side_items(const AdjArgs& a, int side, bool pred) {
-    const int n = side < 2 ? a.ny : a.nx;
-    return level_side(a, side) ? (pred ? band_faces(n) : 2LL * n) : 0;
+__host__ __device__ inline long long side_items(const AdjArgs& a, int side) {
+    return level_side(a, side) ? band_faces(side < 2 ? a.ny : a.nx) : 0;
 }
-__host__ __device__ inline long long band_items(const AdjArgs& a, bool pred) {
-    return side_items(a, 0, pred) + side_items(a, 1, pred) + side_items(a, 2, pred) + side_items(a, 3, pred);
+__host__ __device__ inline long long band_items(const AdjArgs& a) {
+    return side_items(a, 0) + side_items(a, 1) + side_items(a, 2) + side_items(a, 3);
 }
 
 // The bands' faces, one per thread.  (In the tile kernel's grid their code
@@ -302,7 +301,7 @@ __global__ void __launch_bounds__(64) adj_band_kernel(const AdjArgs a) {
     if (PRED) scale = 0.5f * (a.dt_dev != nullptr ? *a.dt_dev : a.dt);
     long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     int side = 0;
-    while (side < 4 && t >= side_items(a, side, PRED)) t -= side_items(a, side++, PRED);
+    while (side < 4 && t >= side_items(a, side)) t -= side_items(a, side++);
     if (side == 4) return;
     const int n = side < 2 ? a.ny : a.nx, m = side < 2 ? a.nx : a.ny;  // along, across
     const LevelBand band(a, b, side);
@@ -883,7 +882,7 @@ __global__ void __launch_bounds__(ADJ_THREADS) adj_edge_kernel(const AdjArgs a) 
         const int e = bs < 2 ? (far ? nx - 1 - i : i) : (far ? ny - 1 - j : j);
         float lam[4], lz = 0.0f, l[4];
         float* fr = a.frame + (size_t)b * 4 * plane + (size_t)j * nx + i;
-        if (bs < 0 || !PRED) {
+        if (bs < 0) {
             lam[0] = fr[0];
             lam[1] = fr[plane];
             lam[2] = fr[2 * plane];
@@ -907,11 +906,11 @@ __global__ void __launch_bounds__(ADJ_THREADS) adj_edge_kernel(const AdjArgs a) 
             const bool touches = code == SWE_BC_PERIODIC ? pos == periodic
                                                          : pos == edge || (code == SWE_BC_WALL && pos == mirror);
             if (!touches || (code == SWE_BC_CONSTANT && !BEDG)) continue;
-            // a band holds the records of its own side's ghosts, and in stage 2
-            // of those at the ends of its two lines
+            // a band holds the records of its own side's ghosts and of those
+            // at the ends of its two lines
             if (level_side(a, side)) {
                 band_sum(LevelBand(a, b, side), true, (side & 1) != 0, 0, yax ? i : j, g, n, l);
-            } else if (PRED && bs >= 0 && (bs < 2) == yax) {
+            } else if (bs >= 0 && (bs < 2) == yax) {
                 band_sum(band, false, far, e, yax ? i : j, g, n, l);
             } else {
                 const float* gl = yax ? a.gy + 4 * (((size_t)b * 4 + (q - 4)) * nx + i)
@@ -1145,7 +1144,7 @@ template <bool BEDG, bool PRED, class M>
 cudaError_t launch_adj_forms(AdjArgs a, cudaStream_t s) {
     const dim3 th(ADJ_THREADS);
     const dim3 ge((unsigned)((frame_cells(a.ny, a.nx) + ADJ_THREADS - 1) / ADJ_THREADS), a.B);
-    const long long items = band_items(a, PRED);
+    const long long items = band_items(a);
     cudaError_t e = cudaSuccess;
     if (items > 0)
         e = launch_chained(adj_band_kernel<BEDG, PRED, M>, dim3((unsigned)((items + 63) / 64), a.B), dim3(64), s, a);

@@ -614,3 +614,38 @@ def test_level_adjoint_at_a_corner_of_two_level_sides(kinds):
     both = _member_level_adjoints(z, U, lam, (left, "wall", top, "wall"), level)
     assert int((a != 0).sum()) > 16 and int((b != 0).sum()) > 16
     assert torch.equal(both, a + b)
+
+
+@pytest.mark.parametrize("ny,nx", [(33, 40), (50, 67)])
+@pytest.mark.parametrize("bed_grad", [False, True])
+def test_stage2_entry_equals_spatial_then_predictor_with_face_records(ny, nx, bed_grad):
+    """The two-call form of test_stage2_entry_equals_spatial_then_predictor
+    on grids that keep face records along their level sides: bit for bit."""
+    from diffswe2d_b200.adjoint import AdjointStepper
+    z, U, level = _member_states(2, ny, nx, ny)
+    cfg = SWEConfig(boundary_left="water_level", boundary_top="absorbing", boundary_right="wall",
+                    boundary_bottom="absorbing")
+    m = SWE2D(z, torch.full_like(z, 0.02), 0.5, 0.7, config=cfg, train_dem=False)
+    st = AdjointStepper(m, 2, ny, nx, torch.device(DEV), 2, bed_grad=bed_grad)
+    k1, P, dt = torch.empty_like(U), torch.empty_like(U), 0.02
+    st._tendency(U, level, k1)
+    st._pointwise(2, U, k1, dt, None, None, None, P)
+    g = torch.Generator().manual_seed(3)
+    lam, base = torch.randn(U.shape, generator=g).to(DEV), torch.randn(U.shape, generator=g).to(DEV)
+    out = []
+    for fused in (True, False):
+        lamU, lamP = base.clone(), torch.zeros_like(U)
+        if bed_grad:
+            st.lam_bed.zero_()
+        if fused:
+            st.lam_k.copy_(lam)
+            st._stage2(P, U, k1, level, dt, lamU)
+            lk1 = st.lam_k1.clone()
+        else:
+            lk1 = torch.empty_like(U)
+            st._spatial(P, level, lam, lamP, st.part[0], "spatial")
+            st.lam_k = lk1  # where _pointwise writes the adjoint of k1
+            st._pointwise(1, U, k1, dt, lamP, lamU, None, None)
+        out.append([lamU, lk1, st.part[0].clone()] + ([st.lam_bed.clone()] if bed_grad else []))
+    for a, b in zip(*out):
+        assert float(a.abs().max()) > 0 and torch.equal(a, b)
