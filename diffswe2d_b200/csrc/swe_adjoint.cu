@@ -54,6 +54,7 @@ int adj_args(AdjArgs& a, const float* S, const float* bed, int bedB, int B, int 
     a.kc = make_consts(*p);
     a.positivity = p->positivity_limiter;
     a.level_blocks = level_blocks;
+    a.bands = bands;
     if (bands && ny >= BAND_MIN && nx >= BAND_MIN) {
         a.bandx = scratch_cx + (size_t)16 * B * ny;
         a.bandy = a.frame + (size_t)4 * B * ny * nx;

@@ -50,7 +50,8 @@ struct AdjArgs {
     float* gy;           // adjoints of the y ghosts [B][top, bottom][1st, 2nd][nx][4]
     float* frame;        // adjoints of the frame's cells before the folds [B][4][ny][nx] (the
                          // fourth plane: the bed's, then the cell's share of the level's)
-    float* bandx;        // face records along the level's x sides (LevelBand), else null
+    int bands;           // along level sides, sums face by face (level bands, below)
+    float* bandx;        // face records along the level's x sides, or null: no records
     float* bandy;        // the same along its y sides
     float* lS;           // adjoint of S, accumulated (+=)
     float* llevel_part;  // partial level adjoints [B][level_blocks]
@@ -226,14 +227,15 @@ __device__ State padded_state(const AdjArgs& a, int b, int j, int i, float scale
 // 1.  (The cells because a second call's ghosts take their cotangents from
 // what this one makes of them.)  A record holds the face's contributions to its
 // four cells, 4 x (U0, U1, U2, Z).  Grids too small for the scratch buffers
-// (either side below BAND_MIN cells) do without.
+// (either side below BAND_MIN cells) keep none: there every face is evaluated
+// where it is summed (FLY below), the same values in the same order.
 constexpr int BAND_MIN = 32;
 constexpr int BAND_REC = 16;
 
 __host__ __device__ inline long long band_faces(int n) { return 4LL * n + 2LL * (n + 1); }
 __host__ __device__ inline long long band_floats(int B, int n) { return 2LL * B * band_faces(n) * BAND_REC; }
 __host__ __device__ inline bool level_side(const AdjArgs& a, int side) {
-    return a.bandx != nullptr && (a.bc[side] == SWE_BC_WATER_LEVEL || a.bc[side] == SWE_BC_ABSORBING);
+    return a.bands && (a.bc[side] == SWE_BC_WATER_LEVEL || a.bc[side] == SWE_BC_ABSORBING);
 }
 
 struct LevelBand {
@@ -285,7 +287,7 @@ __device__ void band_face(const AdjArgs& a, int b, bool diry, int f, int row, fl
 
 // Faces of all bands of a batch member.
 __host__ __device__ inline long long side_items(const AdjArgs& a, int side) {
-    return level_side(a, side) ? band_faces(side < 2 ? a.ny : a.nx) : 0;
+    return a.bandx != nullptr && level_side(a, side) ? band_faces(side < 2 ? a.ny : a.nx) : 0;
 }
 __host__ __device__ inline long long band_items(const AdjArgs& a) {
     return side_items(a, 0) + side_items(a, 1) + side_items(a, 2) + side_items(a, 3);
@@ -332,6 +334,26 @@ __device__ __noinline__ void band_sum(const LevelBand& band, bool normal, bool f
     }
 #pragma unroll
     for (int c = 0; c < 4; ++c) l[c] = (((0.0f + v[0][c]) + v[1][c]) + v[2][c]) + v[3][c];
+}
+
+// The same sum with the faces evaluated here: along x of row `line`, or along
+// y of column `line`.
+template <bool BEDG, bool PRED, class M>
+__device__ __noinline__ void face_sum(const AdjArgs& a, int b, bool diry, int line, int pos, int n, float scale,
+                                      float l[4]) {
+#pragma unroll
+    for (int c = 0; c < 4; ++c) l[c] = 0.0f;
+#pragma unroll 1
+    for (int q = 0; q < 4; ++q) {
+        const int f = pos - 1 + q;
+        if (f < 0 || f > n) continue;
+        float r[BAND_REC];
+        band_face<BEDG, PRED, M>(a, b, diry, f, line, scale, r);
+#pragma unroll
+        for (int s = 0; s < 4; ++s)  // (a constant index keeps the record in registers)
+            if (s == 3 - q)
+                for (int c = 0; c < 4; ++c) l[c] += r[4 * s + c];
+    }
 }
 
 // Floats per cell of the sides' and adjoints' slots (see adj_tile_kernel).
@@ -857,8 +879,8 @@ __device__ __forceinline__ void frame_cell(int ny, int nx, long long t, int& j, 
 
 // Finishes the frame, a cell per thread.  A few warps run through it once,
 // so its time is that of its instruction fetches and load chains: one copy
-// of each part, no ghost read in vain.
-template <bool BEDG, bool PRED, class M>
+// of each part, no ghost read in vain.  FLY: level bands without records.
+template <bool BEDG, bool PRED, bool FLY, class M>
 __global__ void __launch_bounds__(ADJ_THREADS) adj_edge_kernel(const AdjArgs a) {
     chain_start();
     const int ny = a.ny, nx = a.nx, b = blockIdx.y;
@@ -888,8 +910,13 @@ __global__ void __launch_bounds__(ADJ_THREADS) adj_edge_kernel(const AdjArgs a) 
             lam[2] = fr[2 * plane];
             if (BEDG) lz = fr[3 * plane];
         } else {
-            band_sum(band, bs < 2, far, e, j, i, nx, lam);
-            band_sum(band, bs >= 2, far, e, i, j, ny, l);
+            if (FLY) {
+                face_sum<BEDG, PRED, M>(a, b, false, j, i, nx, scale, lam);
+                face_sum<BEDG, PRED, M>(a, b, true, i, j, ny, scale, l);
+            } else {
+                band_sum(band, bs < 2, far, e, j, i, nx, lam);
+                band_sum(band, bs >= 2, far, e, i, j, ny, l);
+            }
             lam[0] += l[0];
             lam[1] += l[1];
             lam[2] += l[2];
@@ -908,7 +935,9 @@ __global__ void __launch_bounds__(ADJ_THREADS) adj_edge_kernel(const AdjArgs a) 
             if (!touches || (code == SWE_BC_CONSTANT && !BEDG)) continue;
             // a band holds the records of its own side's ghosts and of those
             // at the ends of its two lines
-            if (level_side(a, side)) {
+            if (FLY && (level_side(a, side) || (bs >= 0 && (bs < 2) == yax))) {
+                face_sum<BEDG, PRED, M>(a, b, yax, yax ? i : j, g, n, scale, l);
+            } else if (level_side(a, side)) {
                 band_sum(LevelBand(a, b, side), true, (side & 1) != 0, 0, yax ? i : j, g, n, l);
             } else if (bs >= 0 && (bs < 2) == yax) {
                 band_sum(band, false, far, e, yax ? i : j, g, n, l);
@@ -1145,12 +1174,15 @@ cudaError_t launch_adj_forms(AdjArgs a, cudaStream_t s) {
     const dim3 th(ADJ_THREADS);
     const dim3 ge((unsigned)((frame_cells(a.ny, a.nx) + ADJ_THREADS - 1) / ADJ_THREADS), a.B);
     const long long items = band_items(a);
+    const bool level = level_side(a, 0) || level_side(a, 1) || level_side(a, 2) || level_side(a, 3);
     cudaError_t e = cudaSuccess;
     if (items > 0)
         e = launch_chained(adj_band_kernel<BEDG, PRED, M>, dim3((unsigned)((items + 63) / 64), a.B), dim3(64), s, a);
-    a.direct_level = items == 0 && a.level_blocks >= (int)ge.x;
+    a.direct_level = !level && a.level_blocks >= (int)ge.x;
     if (e == cudaSuccess) e = launch_tiles<BEDG, PRED, M, 16>(a, s);
-    if (e == cudaSuccess) e = launch_chained(adj_edge_kernel<BEDG, PRED, M>, ge, th, s, a);
+    if (e == cudaSuccess)
+        e = level && items == 0 ? launch_chained(adj_edge_kernel<BEDG, PRED, true, M>, ge, th, s, a)
+                                : launch_chained(adj_edge_kernel<BEDG, PRED, false, M>, ge, th, s, a);
     if (e == cudaSuccess && !a.direct_level)
         e = launch_chained(adj_level_kernel, dim3(a.level_blocks, a.B), th, s, a.frame, a.llevel_part, a.ny, a.nx);
     return e;

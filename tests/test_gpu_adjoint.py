@@ -649,3 +649,27 @@ def test_stage2_entry_equals_spatial_then_predictor_with_face_records(ny, nx, be
         out.append([lamU, lk1, st.part[0].clone()] + ([st.lam_bed.clone()] if bed_grad else []))
     for a, b in zip(*out):
         assert float(a.abs().max()) > 0 and torch.equal(a, b)
+
+
+@pytest.mark.parametrize("ny", [12, 20, 31])
+@pytest.mark.parametrize("kinds", [("water_level", "absorbing"), ("wall", "water_level"), ("absorbing", "wall")])
+def test_level_adjoint_of_a_small_grid(ny, kinds):
+    """A step's level adjoint for cotangents in the first two rows does not
+    depend on the rows far below: the same bits on a grid of fewer than 32
+    rows, which keeps no face records, as on the grid continued to 40."""
+    from diffswe2d_b200.adjoint import AdjointStepper
+    B, nx = 16, 40
+    z, U, level = _member_states(B, 40, nx, ny)
+    lam = torch.zeros_like(U)
+    lam[:, :, :2] = torch.randn((B, 3, 2, nx), generator=torch.Generator().manual_seed(7)).to(DEV)
+    cfg = SWEConfig(boundary_left=kinds[0], boundary_top=kinds[1], boundary_right="wall", boundary_bottom="wall")
+    out = []
+    for rows in (40, ny):
+        cut = lambda q: q[:, :, :rows].contiguous()  # noqa: E731
+        m = SWE2D(cut(z), torch.full_like(cut(z), 0.02), 0.5, 0.7, config=cfg, train_dem=False)
+        st = AdjointStepper(m, B, rows, nx, torch.device(DEV), B)
+        V = cut(U)
+        part = st(V, level, 0.01, cut(lam), torch.zeros_like(V), torch.zeros((B, 1, rows, nx), device=DEV))
+        out.append(part.reshape(2, B, -1).sum(2))
+    assert int((out[0] != 0).sum()) > B
+    assert torch.equal(out[0], out[1])
