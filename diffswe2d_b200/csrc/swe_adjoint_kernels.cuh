@@ -635,7 +635,21 @@ __global__ void __launch_bounds__(ADJ_THREADS, SWE_ADJ_TILE_MINB) adj_tile_kerne
         s_p[4 * RY * RX + w] = p.z;
     }
     const bool tame = !__syncthreads_or(wild);
-    if (!__syncthreads_or(!idle) && tame) {
+    bool quiet = !__syncthreads_or(!idle) && tame;
+    if (PRED && quiet) {  // the predictor's adjoint takes U and U + dt/2 k1, of which dry cells show nothing
+        bool odd = false;
+        for (int w = tid; w < TY * TX; w += ADJ_THREADS) {
+            const int ty = w / TX, tx = w % TX, j = j0 + ty, i = i0 + tx;
+            if (j >= ny || i >= nx || s_p[(ty + 3) * RX + tx + 3] > kc.dry) continue;
+            const size_t o = a3(b, 0, j, i, ny, nx);
+            for (int c = 0; c < 3; ++c) {
+                const float u = a.U[o + c * plane];
+                odd |= !(fabsf(u) <= kTame && fabsf(u + scale * a.k1[o + c * plane]) <= kTame);
+            }
+        }
+        quiet = !__syncthreads_or(odd);
+    }
+    if (quiet) {
         zero_tile<PRED>(a, b, j0, i0, TY);
         return;
     }

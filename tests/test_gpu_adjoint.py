@@ -673,3 +673,36 @@ def test_level_adjoint_of_a_small_grid(ny, kinds):
         out.append(part.reshape(2, B, -1).sum(2))
     assert int((out[0] != 0).sum()) > B
     assert torch.equal(out[0], out[1])
+
+
+@pytest.mark.parametrize("run", [False, True])
+@pytest.mark.parametrize("field,value,h", [("k1", -np.inf, 0.3), ("U", np.nan, 0.0), ("U", np.inf, 0.0)])
+def test_predictor_adjoint_of_a_non_finite_cell_beside_zero_cotangents(run, field, value, h):
+    """The clean-up makes a cell of a -inf tendency, or of a dry cell's
+    non-finite momentum, dry: the state that the spatial adjoint sees is
+    finite.  Its predictor adjoint is the same NaN (or number) whether the
+    tile's cotangents are all zero or one of them, far away, is not."""
+    from diffswe2d_b200.adjoint import AdjointStepper
+    ny, nx = 16, 64
+    z = torch.full((1, 1, ny, nx), -0.3, device=DEV)
+    U = torch.zeros((1, 3, ny, nx), device=DEV)
+    U[:, 0] = 0.3
+    k1 = torch.zeros_like(U)
+    U[0, 0, 8, 8] = h
+    if field == "k1":
+        k1[0, 0, 8, 8] = value
+    else:
+        U[0, 1, 8, 8] = value
+        k1[0, 0, 8, 8] = -1.0
+    m = SWE2D(z, torch.full_like(z, 0.02), 0.5, 0.7, train_dem=False)
+    st = AdjointStepper(m, 1, ny, nx, torch.device(DEV), 1, run=run)
+    level, P, out = torch.zeros(1, device=DEV), torch.empty_like(U), []
+    st._pointwise(2, U, k1, 0.01, None, None, None, P)
+    for far in (0.0, 1.0):
+        lamU = torch.zeros_like(U)
+        st.lam_k.zero_()
+        st.lam_k[0, 0, 8, 28] = far
+        st._stage2(P, U, k1, level, 0.01, lamU)
+        out.append(torch.cat([lamU[..., 8, 8], st.lam_k1[..., 8, 8]]))
+    assert bool(out[1].isnan().any())
+    assert torch.equal(out[0].nan_to_num(7.0), out[1].nan_to_num(7.0))
