@@ -693,7 +693,10 @@ __global__ void im2col8_kernel(const float* __restrict__ x, int Nb, int Lin, int
     *reinterpret_cast<uint4*>(cols + (size_t)row * ldcols + c0) = q;
 }
 
-constexpr int ADJ_ROWS = 128;  // rows per block of the kernel below
+constexpr int ADJ_ROWS = 128, ADJ_COLS = 1024;  // rows and channels per block of the kernel below
+dim3 adjoint_rows_grid(int rows, int C) {
+    return dim3((rows + ADJ_ROWS - 1) / ADJ_ROWS, (C + ADJ_COLS - 1) / ADJ_COLS);
+}
 
 // Adjoint of a layer's activation over [rows, C], four channels per thread:
 // the adjoint of the activation is src itself (k == 0) or gathered from the
@@ -702,16 +705,19 @@ constexpr int ADJ_ROWS = 128;  // rows per block of the kernel below
 // block's rows (the bias gradient's partial sums).  One pass in place of
 // col2im, activation adjoint, transpose and column sums, with three fp32
 // arrays written and read back (first convolution of 256 records: 120 us in
-// four kernels, 12 us here; memory bound, 32 MB).
+// four kernels, 12 us here; memory bound, 32 MB).  A block's 256 threads
+// share the rows of up to 1,024 channels (blockIdx.y: which); where C / 4
+// does not divide 256 the threads past the last whole row idle.
 __global__ void __launch_bounds__(256) adjoint_rows_kernel(const float* __restrict__ src, int ld, int rows, int C,
                                                            int Lin, int k, int stride, int pad, int Lout,
                                                            const float* __restrict__ pre, uint16_t* d_bf16,
                                                            float* colpart) {
     __shared__ float4 s_sum[256];
-    const int tpr = C / 4, rpp = 256 / tpr;  // threads per row, rows per pass
-    const int t = threadIdx.x, g = t / tpr, c = (t - g * tpr) * 4;
+    const int c0 = blockIdx.y * ADJ_COLS;
+    const int tpr = min(C - c0, ADJ_COLS) / 4, rpp = 256 / tpr;  // threads per row, rows per pass
+    const int t = threadIdx.x, g = t / tpr, c = c0 + (t - g * tpr) * 4;
     float4 sum = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    const int row0 = blockIdx.x * ADJ_ROWS, row1 = min(rows, row0 + ADJ_ROWS);
+    const int row0 = blockIdx.x * ADJ_ROWS, row1 = g < rpp ? min(rows, row0 + ADJ_ROWS) : 0;
     for (int r = row0 + g; r < row1; r += rpp) {
         float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         if (k == 0) {
@@ -849,9 +855,8 @@ bool valid_layers(const nn_layer* L, int n, int nb) {
         } else if (l.kpad != l.cin || l.cin != (L[i - 1].conv ? L[i - 1].cout * L[i - 1].lout : L[i - 1].cout)) {
             return false;
         }
-        // rows of 16-byte chunks, whole four-channel groups, 32-bit indices
+        // rows of 16-byte chunks, 32-bit indices
         if (i + 1 < n && l.cout % 16) return false;
-        if (i + 1 < n && L[i + 1].conv && (l.cout > 1024 || 256 % (l.cout / 4))) return false;
         if ((long long)rows_of(l, nb) * (l.kpad > l.cout ? l.kpad : l.cout) >= (1ll << 31)) return false;
     }
     return true;
@@ -999,7 +1004,7 @@ extern "C" int nn_net_backward(const nn_layer* layers, int nlayers, const uint16
         return SWE_EARG;
     const nn_layer* L = layers;
     const int n = nlayers;
-    if (L[n - 1].cout % 16 || L[n - 1].cout > 1024 || 256 % (L[n - 1].cout / 4)) return SWE_EARG;
+    if (L[n - 1].cout % 16) return SWE_EARG;
     if (((uintptr_t)workspace & 255u) || ((uintptr_t)params_bf16 & 15u) || ((uintptr_t)dout & 15u)) return SWE_EARG;
     cudaStream_t s = (cudaStream_t)stream;
     const NetBuffers b = carve(workspace, L, n, nb, true);
@@ -1013,7 +1018,7 @@ extern "C" int nn_net_backward(const nn_layer* layers, int nlayers, const uint16
         ba.n[i] = L[i].cout;
         columns += L[i].cout;
     }
-    adjoint_rows_kernel<<<(nb + ADJ_ROWS - 1) / ADJ_ROWS, 256, 0, s>>>(
+    adjoint_rows_kernel<<<adjoint_rows_grid(nb, L[n - 1].cout), 256, 0, s>>>(
         dout, L[n - 1].cout, nb, L[n - 1].cout, 0, 0, 0, 0, 0, nullptr, b.d[n - 1], b.colpart[n - 1]);
     for (int i = n - 1; i >= 0; --i) {
         const nn_layer& l = L[i];
@@ -1049,7 +1054,7 @@ extern "C" int nn_net_backward(const nn_layer* layers, int nlayers, const uint16
             rc = launch_gemm<false, true>(g, 1, nullptr, s);
             if (rc != SWE_OK) return rc;
             const int prows = nb * l.lin;
-            adjoint_rows_kernel<<<(prows + ADJ_ROWS - 1) / ADJ_ROWS, 256, 0, s>>>(
+            adjoint_rows_kernel<<<adjoint_rows_grid(prows, l.cin), 256, 0, s>>>(
                 b.dcols, l.kpad, prows, l.cin, l.lin, l.k, l.stride, l.pad, l.lout, b.pre[i - 1], b.d[i - 1],
                 b.colpart[i - 1]);
         }

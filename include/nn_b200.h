@@ -114,9 +114,8 @@ int nn_adam_bf16(float* params, const float* grads, float* m, float* v, long lon
  * [cout, kpad] (column kk*cin + ci of a convolution) and bias [cout] lie at
  * offsets w (a multiple of 8) and b of the flat parameter vector; kpad is
  * k*cin (dense: cin) rounded up to 16 for the first layer, equal to it for
- * the others.  cout of every layer but the last is a multiple of 16, that of
- * a convolution before another one (and, for training, of the last layer)
- * also a divisor of 1024.  At most 8 layers; others are refused (SWE_EARG,
+ * the others.  cout of every layer but the last (and, for training, of the
+ * last) is a multiple of 16.  At most 8 layers; others are refused (SWE_EARG,
  * workspace -1).
  */
 typedef struct {

@@ -348,3 +348,22 @@ def test_gemm_wait_limit_that_runs_out_midway(wait_ns):
         assert code == 1 or np.array_equal(out.cpu().numpy(), full)
     again, _, _ = _gemm(A, B, M, N, K, K, K)
     assert np.array_equal(again, full)
+
+
+@pytest.mark.parametrize("controls", [16, 48, 80, 1040])
+def test_backward_of_any_number_of_controls(controls):
+    """Numbers of controls that divide a block's threads evenly, do not, and
+    need a second block of channels."""
+    nb = 3
+    net = WarmStartNet(DEV, seed=1, controls=controls)
+    g = torch.Generator(device=DEV).manual_seed(controls)
+    x = torch.randn((nb, 6, 1125), device=DEV, generator=g) * 0.008
+    dout = torch.randn((nb, controls), device=DEV, generator=g)
+    out = net.forward(x).clone()
+    net.backward(dout)
+    net.check_errors()
+    ref, dW, db = _composed_pass(net, x, dout)
+    assert torch.equal(out, ref)
+    for i in range(6):
+        assert torch.equal(net.weight_grad(i), dW[i])
+        assert bool(((net.bias_grad(i).double() - db[i][0]).abs() <= 600 * 2.0 ** -24 * db[i][1] + 1e-30).all())
