@@ -720,8 +720,9 @@ __global__ void __launch_bounds__(256) adjoint_rows_kernel(const float* __restri
     const int row0 = blockIdx.x * ADJ_ROWS, row1 = g < rpp ? min(rows, row0 + ADJ_ROWS) : 0;
     for (int r = row0 + g; r < row1; r += rpp) {
         float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        if (k == 0) {
-            v = *reinterpret_cast<const float4*>(src + (size_t)r * ld + c);
+        if (k == 0) {  // (the caller's array: any alignment)
+            const float* q = src + (size_t)r * ld + c;
+            v = make_float4(q[0], q[1], q[2], q[3]);
         } else {
             const int n = r / Lin, l = r - n * Lin;
             for (int kk = (l + pad) % stride; kk < k; kk += stride) {  // kk = l + pad - lo * stride
@@ -1005,7 +1006,7 @@ extern "C" int nn_net_backward(const nn_layer* layers, int nlayers, const uint16
     const nn_layer* L = layers;
     const int n = nlayers;
     if (L[n - 1].cout % 16) return SWE_EARG;
-    if (((uintptr_t)workspace & 255u) || ((uintptr_t)params_bf16 & 15u) || ((uintptr_t)dout & 15u)) return SWE_EARG;
+    if (((uintptr_t)workspace & 255u) || ((uintptr_t)params_bf16 & 15u)) return SWE_EARG;
     cudaStream_t s = (cudaStream_t)stream;
     const NetBuffers b = carve(workspace, L, n, nb, true);
     BiasArgs ba{};

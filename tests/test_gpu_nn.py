@@ -367,3 +367,16 @@ def test_backward_of_any_number_of_controls(controls):
     for i in range(6):
         assert torch.equal(net.weight_grad(i), dW[i])
         assert bool(((net.bias_grad(i).double() - db[i][0]).abs() <= 600 * 2.0 ** -24 * db[i][1] + 1e-30).all())
+
+
+def test_backward_of_a_cotangent_at_any_address():
+    net, nb = WarmStartNet(DEV, seed=1), 5
+    g = torch.Generator(device=DEV).manual_seed(2)
+    net.forward(torch.randn((nb, 6, 1125), device=DEV, generator=g) * 0.008)
+    buf = torch.randn(3 + nb * 16, device=DEV, generator=g)
+    grads = []
+    for dout in (buf[3:].view(nb, 16).clone(), buf[3:].view(nb, 16)):
+        net.backward(dout)
+        grads.append(net.grads.clone())
+    net.check_errors()
+    assert torch.equal(grads[0], grads[1])
