@@ -856,9 +856,10 @@ bool valid_layers(const nn_layer* L, int n, int nb) {
         } else if (l.kpad != l.cin || l.cin != (L[i - 1].conv ? L[i - 1].cout * L[i - 1].lout : L[i - 1].cout)) {
             return false;
         }
-        // rows of 16-byte chunks, 32-bit indices
+        // rows of 16-byte chunks; 32-bit row numbers and places within a record
         if (i + 1 < n && l.cout % 16) return false;
-        if ((long long)rows_of(l, nb) * (l.kpad > l.cout ? l.kpad : l.cout) >= (1ll << 31)) return false;
+        const long long per = l.conv ? l.lout : 1;
+        if (nb * per > (1ll << 30) || per * std::max(l.kpad, l.cout) >= (1ll << 31)) return false;
     }
     return true;
 }
@@ -970,10 +971,14 @@ extern "C" int nn_net_forward(const nn_layer* layers, int nlayers, const float* 
     const NetBuffers b = carve(workspace, L, nlayers, nb, false);
     {
         const nn_layer& l = L[0];  // x is [nb, cin, lin]
-        const long long total = (long long)nb * l.lout * (l.kpad / 8);
-        im2col8_kernel<<<(unsigned)((total + 255) / 256), 256, 0, s>>>(x, nb, l.lin, l.cin, l.cin * l.lin, 1, l.lin,
-                                                                       l.k, l.stride, l.pad, l.lout, in_scale,
-                                                                       b.cols, l.kpad);
+        const long long per = (long long)l.lout * (l.kpad / 8);  // the kernel's indices are 32-bit
+        const int step = (int)std::max(1ll, std::min((long long)nb, (1ll << 31) / per));
+        for (int n0 = 0; n0 < nb; n0 += step) {
+            const int count = std::min(step, nb - n0);
+            im2col8_kernel<<<(unsigned)((count * per + 255) / 256), 256, 0, s>>>(
+                x + (size_t)n0 * l.cin * l.lin, count, l.lin, l.cin, l.cin * l.lin, 1, l.lin, l.k, l.stride, l.pad,
+                l.lout, in_scale, b.cols + (size_t)n0 * l.lout * l.kpad, l.kpad);
+        }
     }
     for (int i = 0; i < nlayers; ++i) {
         const nn_layer& l = L[i];

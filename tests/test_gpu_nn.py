@@ -380,3 +380,19 @@ def test_backward_of_a_cotangent_at_any_address():
         grads.append(net.grads.clone())
     net.check_errors()
     assert torch.equal(grads[0], grads[1])
+
+
+def test_forward_of_a_very_large_batch():
+    """More than 2^31 elements in the first layer's patches (about 35 GB of
+    workspace): the same outputs as the records by themselves."""
+    nb = 121_001
+    net = WarmStartNet(DEV, seed=3)
+    g = torch.Generator(device=DEV).manual_seed(3)
+    few = torch.randn((1001, 6, 1125), device=DEV, generator=g) * 0.008
+    ref = net.forward(few).clone()
+    x = few.repeat(-(-nb // 1001), 1, 1)[:nb].contiguous()
+    out = net.forward(x)
+    net.check_errors()
+    assert torch.equal(out, ref.repeat(-(-nb // 1001), 1)[:nb])
+    del net, out, x
+    torch.cuda.empty_cache()
