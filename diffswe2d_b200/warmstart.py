@@ -134,7 +134,8 @@ class WarmStartNet:
             t.conv, t.cin, t.cout, t.kpad, t.w, t.b = int(conv), L.cin, L.cout, kp, w, b
             if conv:
                 t.k, t.stride, t.pad, t.lin, t.lout = L.k, L.stride, L.pad, L.lin, L.lout
-        self._cap = 0  # the largest batch that the workspace and the outputs hold
+        self._cap = 0      # the largest batch that the workspace holds
+        self._nb = None    # the last batch
 
     # ----------------------------------------------------------- helpers
     def weight(self, i):
@@ -162,29 +163,30 @@ class WarmStartNet:
                   "nn cast")
 
     def _buffers(self, nb: int):
-        """Workspace and outputs, for the largest batch seen."""
-        if nb <= self._cap:
-            return
-        nbytes = nat.lib().nn_net_workspace_bytes(self._table, len(self.layers), nb, 1)
-        if nbytes < 0:
-            raise ValueError(f"the network's shapes are not supported for a batch of {nb}")
-        self._ws = torch.empty(int(nbytes), dtype=torch.uint8, device=self.dev)
-        self._out = torch.empty((nb, self.controls), device=self.dev)
-        self._dpred = torch.empty_like(self._out)
-        self.loss = torch.zeros(1, device=self.dev)
-        self._cap = nb
+        """Workspace for the largest batch seen, and outputs: those of a batch
+        of another size than the last are tensors of their own."""
+        if nb > self._cap:
+            nbytes = nat.lib().nn_net_workspace_bytes(self._table, len(self.layers), nb, 1)
+            if nbytes < 0:
+                raise ValueError(f"the network's shapes are not supported for a batch of {nb}")
+            self._ws = torch.empty(int(nbytes), dtype=torch.uint8, device=self.dev)
+            self._cap = nb
+        if nb != self._nb:
+            self.out = torch.empty((nb, self.controls), device=self.dev)
+            self.dpred = torch.empty_like(self.out)
+            self.loss = torch.zeros(1, device=self.dev)
+            self._nb = nb
 
     # ----------------------------------------------------------- forward
     def forward(self, x: torch.Tensor) -> torch.Tensor:
         """x: gauge eta [Nb, gauges, samples] fp32 (metres) -> normalised
-        controls [Nb, controls] fp32 (a view of an internal buffer)."""
+        controls [Nb, controls] fp32 (an internal buffer that the next call
+        with as many records overwrites)."""
         x = nat.require_cuda_f32("x", x)
         nb, G, T = x.shape
         if G != self.gauges or T != self.samples:
             raise ValueError(f"expected [N, {self.gauges}, {self.samples}] gauge series, got {tuple(x.shape)}")
         self._buffers(nb)
-        self._nb = nb
-        self.out, self.dpred = self._out[:nb], self._dpred[:nb]
         rc = nat.lib().nn_net_forward(self._table, len(self.layers), nat.ptr(self.params),
                                       nat.ptr(self.params_bf16), nat.ptr(x), INPUT_SCALE, nb,
                                       nat.ptr(self._ws), nat.ptr(self.out), self.wait_ns,

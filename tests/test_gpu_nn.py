@@ -396,3 +396,18 @@ def test_forward_of_a_very_large_batch():
     assert torch.equal(out, ref.repeat(-(-nb // 1001), 1)[:nb])
     del net, out, x
     torch.cuda.empty_cache()
+
+
+def test_outputs_of_another_batch_size_are_kept():
+    """A result is overwritten by the next call with as many records, not by
+    one with more or fewer."""
+    net = WarmStartNet(DEV, seed=4)
+    g = torch.Generator(device=DEV).manual_seed(4)
+    x = torch.randn((9, 6, 1125), device=DEV, generator=g) * 0.008
+    y = torch.randn((9, 16), device=DEV, generator=g)
+    held = []
+    for nb in (9, 4, 7, 9):
+        loss = net.loss_and_grad(x[:nb].contiguous(), y[:nb].contiguous())
+        held.append((net.out, net.out.clone(), loss, loss.clone()))
+    net.check_errors()
+    assert all(torch.equal(a, b) and torch.equal(c, d) for a, b, c, d in held)
