@@ -154,7 +154,8 @@ class SWE2D(nn.Module):
     def _prepare_boundary_level(level: ScalarOrTensor, reference: torch.Tensor) -> torch.Tensor:
         if torch.is_tensor(level):
             return level.to(dtype=reference.dtype, device=reference.device)
-        if isinstance(level, float):  # filled on the device: no host copy to wait for
+        if isinstance(level, float) and reference.dtype == torch.float32 and -3e38 < level < 3e38:
+            # filled on the device: no host copy to wait for (full() refuses what rounds to infinity)
             return torch.full((), level, dtype=reference.dtype, device=reference.device)
         return reference.new_tensor(level)
 

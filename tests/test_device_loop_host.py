@@ -79,3 +79,13 @@ def test_chunks_of_an_odd_length_are_rounded_up():
     for bad in (0, -2):
         with pytest.raises(ValueError):
             even_chunk(bad)
+
+
+def test_boundary_levels_from_the_host_as_new_tensor_gives_them():
+    import torch
+    from diffswe2d_b200 import SWE2D
+    for dtype in (torch.float32, torch.float64, torch.float16):
+        U = torch.zeros((1, 3, 2, 2), dtype=dtype)
+        for v in (0.1, 1e-46, -0.0, 3.4028235e38, -3.4028235677973366e38, 1e300, math.inf, -math.inf, math.nan, 7):
+            a, b = SWE2D._prepare_boundary_level(v, U), U.new_tensor(v)
+            assert a.dtype == b.dtype and a.shape == b.shape and torch.equal(a.nan_to_num(3.0), b.nan_to_num(3.0))
