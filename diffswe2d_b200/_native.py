@@ -215,6 +215,7 @@ _SIGNATURES = {
     "swe_bed_f32": [_P, _P, _P, ctypes.c_longlong, _P, _P],
     "swe_tune_sweep_rows": [_I],
     "swe_sweep_rows": [],
+    "swe_launch_rows": [_I, _I, _I, _I],
     "swe_load_kernels": [],
     # include/nn_b200.h
     "nn_gemm_bf16": [_P, _I, _P, _I, _I, _I, _I, _P, _I, _P, _P, _P, _I, _I, _P, ctypes.c_longlong,

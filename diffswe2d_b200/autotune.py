@@ -35,8 +35,9 @@ import torch
 from . import _native as nat
 
 SIZE_CLASSES = ((0, 1 << 16), (1 << 16, 1 << 18), (1 << 18, 1 << 20), (1 << 20, 1 << 62))
-ROW_CHOICES = (4, 8, 16, 32, 64, 128)
-DEFAULT_ROWS = (16, 32, 64, 64)
+#: heights that are timed; 0: the library's own choice for the grid
+ROW_CHOICES = (0, 4, 8, 16, 32, 64, 128)
+DEFAULT_ROWS = (0, 0, 0, 0)
 CHUNK_CHOICES = (8, 16, 32, 64)
 
 _tuned: Dict[str, dict] = {}
@@ -47,8 +48,9 @@ def _cache_file() -> Path:
     return Path(base) / "diffswe2d_b200" / "autotune.json"
 
 
-#: generation of the step kernels: choices timed with other kernels are not used
-KERNELS = 3
+#: generation of the step kernels and of what their heights mean: choices of
+#: other generations are not used
+KERNELS = 4
 
 
 def _device_key(device) -> str:
@@ -92,7 +94,8 @@ def _mode_key(name: str, arithmetic: str) -> str:
 
 
 def tuned_rows(cells: int, device="cuda", arithmetic: str = "exact") -> int:
-    """Tile height for a grid of `cells` cells (the default if not tuned)."""
+    """Tile height for a grid of `cells` cells (0, the library's choice, if
+    not tuned)."""
     k = size_class(cells)
     rows = _load(device).get(_mode_key("rows", arithmetic))
     return int(rows[k]) if rows else DEFAULT_ROWS[k]
@@ -153,7 +156,7 @@ def tune(device="cuda", steps: int = 8, force: bool = False, arithmetic: str = "
             if best_ms is None or ms < best_ms:
                 best, best_ms = r, ms
         rows_choice.append(best)
-    nat.check(nat.lib().swe_tune_sweep_rows(64), "tune rows")
+    nat.check(nat.lib().swe_tune_sweep_rows(0), "tune rows")
     entry[rkey] = rows_choice
     if not entry.get("chunk") or force:
         entry["chunk"] = _tune_chunk(device)

@@ -517,10 +517,11 @@ __global__ void ensemble_init_kernel(EnsCtl* ctl, int count, EnsGlobal* g) {
 }
 
 // Output rows per sweep tile for the single-grid kernels (tuning knob set by
-// swe_tune_sweep_rows; the ensemble carries one value per scenario).
-int g_sweep_rows = SW_ROWS;
+// swe_tune_sweep_rows, 0: sweep_rows_for's choice; the ensemble carries one
+// value per scenario).
+int g_sweep_rows = 0;
 
-// Tile height of a launch while the knob is at its default.  A warp walks
+// Tile height of a launch while the knob is 0.  A warp walks
 // r + 4 rows one after another, so a stage takes about
 // (r + 4) (1 + W(r) / 2500) row times, W(r) the launch's warps: the first
 // term is one warp's chain (a small grid: short tiles), the second the
@@ -530,7 +531,7 @@ int g_sweep_rows = SW_ROWS;
 // rows everywhere took 171 us a step at 64 x 96 in the tolerance mode (15 us at
 // one row), 172 at 244 x 393 (21 at two) and 789 at 4096^2 (754 at 32).
 int sweep_rows_for(int B, int ny, int nx) {
-    if (g_sweep_rows != SW_ROWS) return g_sweep_rows;
+    if (g_sweep_rows != 0) return g_sweep_rows;
     const double strips = (double)((nx + SW_OUT - 1) / SW_OUT) * B;
     int best = SW_ROWS;
     double best_cost = INFINITY;
@@ -1021,12 +1022,21 @@ extern "C" int swe_ensemble_results_f32(const void* workspace, int count, swe_en
 }
 
 extern "C" int swe_tune_sweep_rows(int rows) {
-    if (rows < 1 || rows > 4096) return SWE_EARG;
+    if (rows < 0 || rows > 4096) return SWE_EARG;
     g_sweep_rows = rows;
     return SWE_OK;
 }
 
 extern "C" int swe_sweep_rows(void) { return g_sweep_rows; }
+
+extern "C" int swe_launch_rows(int B, int ny, int nx, int arithmetic) {
+    if (B < 1 || ny < 2 || nx < 2) return -1;
+    StepArgs a{};
+    a.B = B;
+    a.ny = ny;
+    a.nx = nx;
+    return arithmetic != SWE_ARITH_FAST && use_tiled_kernels(a) ? 0 : sweep_rows_for(B, ny, nx);
+}
 
 extern "C" int swe_load_kernels(void) {
     // Touching each kernel loads its module now (CUDA lazy loading), so that

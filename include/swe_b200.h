@@ -505,13 +505,17 @@ int swe_bed_f32(const float* reference, const float* correction, const uint8_t* 
                 long long cells, float* bed, void* stream);
 
 /* Output rows per tile of the single-grid sweep kernels (process-wide
- * tuning knob; set it between launches, not during them).  At its default,
- * 64, each launch takes the height that suits its grid, at most 64. */
+ * tuning knob; set it between launches, not during them): 1 to 4096, or 0,
+ * the default: each launch takes the height that suits its grid, at most 64. */
 int swe_tune_sweep_rows(int rows);
 
 /* The current value of that knob (CUDA graphs keep the value they were
  * captured with). */
 int swe_sweep_rows(void);
+
+/* The height that a launch on such a grid takes now; 0 if it is not made of
+ * sweeps (smaller IEEE grids take shared-memory tiles), -1 for no grid. */
+int swe_launch_rows(int B, int ny, int nx, int arithmetic);
 
 /*
  * swe_step_noalloc_f32 -- one step like swe_step_f32, for callers that must

@@ -86,3 +86,25 @@ def test_cpu_tensor_fails_loudly():
     U = torch.zeros(1, 3, 8, 8)
     with pytest.raises(NativeLibraryError):
         m.step(U, 0.0, 1.0)
+
+
+def test_every_tile_height_can_be_fixed_and_0_is_automatic():
+    """64 rows are 64 rows, on any grid that is swept; 0, the default, leaves
+    the height to the launch."""
+    from diffswe2d_b200 import _native as nat
+    lib = nat.lib()
+    prev = lib.swe_sweep_rows()
+    try:
+        for rows in (1, 64, 4096):
+            assert lib.swe_tune_sweep_rows(rows) == nat.SWE_OK
+            assert lib.swe_launch_rows(1, 244, 393, nat.ARITHMETIC["fast"]) == rows
+            assert lib.swe_launch_rows(1, 4096, 4096, nat.ARITHMETIC["exact"]) == rows
+            assert lib.swe_launch_rows(1, 244, 393, nat.ARITHMETIC["exact"]) == 0  # shared-memory tiles
+        assert lib.swe_tune_sweep_rows(0) == nat.SWE_OK and lib.swe_sweep_rows() == 0
+        small, large = (lib.swe_launch_rows(1, n, n, nat.ARITHMETIC["fast"]) for n in (96, 4096))
+        assert 1 <= small < 16 <= large <= 64
+        for rows in (-1, 4097):
+            assert lib.swe_tune_sweep_rows(rows) == nat.SWE_EARG and lib.swe_sweep_rows() == 0
+    finally:
+        lib.swe_tune_sweep_rows(prev)
+    assert prev == 0
