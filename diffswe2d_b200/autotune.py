@@ -101,6 +101,12 @@ def tuned_rows(cells: int, device="cuda", arithmetic: str = "exact") -> int:
     return int(rows[k]) if rows else DEFAULT_ROWS[k]
 
 
+def _swept(batch: int, ny: int, nx: int, arithmetic: str) -> bool:
+    """Whether steps on such states are row sweeps (smaller IEEE grids take
+    shared-memory tiles, which have no height to choose)."""
+    return nat.lib().swe_launch_rows(batch, ny, nx, nat.arithmetic_code(arithmetic)) != 0
+
+
 def _time_steps(side_y: int, side_x: int, rows: int, device, steps: int, batch: int = 1,
                 arithmetic: str = "exact") -> float:
     """ms per step of the single-grid step kernels on a runup-recipe grid
@@ -149,8 +155,8 @@ def tune(device="cuda", steps: int = 8, force: bool = False, arithmetic: str = "
     reps = ((96, 160), (384, 512), (1024, 960), (2048, 2048))
     rows_choice, timing = [], {}
     for k, (ny, nx) in enumerate(reps):
-        best, best_ms = None, None
-        for r in ROW_CHOICES:
+        best, best_ms = 0, None
+        for r in ROW_CHOICES if _swept(1, ny, nx, arithmetic) else ():
             ms = _time_steps(ny, nx, r, device, steps, arithmetic=arithmetic)
             timing[f"{ny}x{nx}/rows{r}"] = ms
             if best_ms is None or ms < best_ms:
@@ -246,7 +252,10 @@ def _tune_chunk(device) -> int:
 def tuned_rows_for_shape(batch: int, ny: int, nx: int, device="cuda", steps: int = 6,
                          arithmetic: str = "exact") -> int:
     """Tile height for a time loop over [batch, 3, ny, nx] states: timed on
-    that shape (runup recipe) the first time it is asked for, then cached."""
+    that shape (runup recipe) the first time it is asked for, then cached
+    (0 where the steps are not swept)."""
+    if not _swept(batch, ny, nx, arithmetic):
+        return 0
     entry = _load(device)
     key = f"{batch}x{ny}x{nx}" if arithmetic == "exact" else f"{arithmetic}/{batch}x{ny}x{nx}"
     shapes = entry.setdefault("shapes", {})

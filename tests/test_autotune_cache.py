@@ -35,3 +35,25 @@ def test_defaults_without_cache(tmp_path, monkeypatch):
     assert autotune.tuned_rows(100, "cuda") == autotune.DEFAULT_ROWS[0]
     assert autotune.tuned_ensemble_rows("cuda", "fast") == 16
     assert autotune.checkpoint_tuning("cuda") == {}
+
+
+def test_heights_are_timed_only_where_steps_are_swept(tmp_path, monkeypatch):
+    """IEEE grids that take shared-memory tiles have no height: nothing is
+    timed or stored for them."""
+    monkeypatch.setenv("XDG_CACHE_HOME", str(tmp_path))
+    monkeypatch.setattr(autotune, "_device_key", lambda device: "TestGPU/148")
+    monkeypatch.setattr(autotune, "_tuned", {})
+    timed = []
+    monkeypatch.setattr(autotune, "_time_steps",
+                        lambda ny, nx, r, *a, **k: timed.append((ny, nx, r)) or 1.0 + abs(r - 32))
+    assert autotune.tuned_rows_for_shape(1, 244, 393) == 0 and not timed
+    assert autotune._load("cuda").get("shapes", {}) == {}
+    assert autotune.tuned_rows_for_shape(1, 244, 393, arithmetic="fast") == 32
+    assert [r for _, _, r in timed] == list(autotune.ROW_CHOICES)
+    timed.clear()
+    assert autotune.tuned_rows_for_shape(17, 244, 393) == 32 and timed  # 1.63 million cells
+    timed.clear()
+    monkeypatch.setattr(autotune, "_tune_chunk", lambda device: 32)
+    monkeypatch.setattr(autotune, "_tune_ensemble_rows", lambda device, arithmetic: 16)
+    assert autotune.tune()["rows"] == [0, 0, 0, 32]
+    assert {(ny, nx) for ny, nx, _ in timed} == {(2048, 2048)}
