@@ -782,13 +782,14 @@ def run_inversion(args, world, rank, local):
 def run_adjoint(args, world, rank, local):
     """The step adjoint alone at the inversion's shape (--inv-cases runup
     cases of --inv-grid, --inv-arithmetic): time per adjoint step as the
-    gauge run's backward pass runs it (predictor and k2 re-evaluated, k1
-    kept; corrector, stage-2 and stage-1 spatial adjoints), on a state after
-    0.3 s of inflow.  The timed loop is bracketed by cudaProfilerStart/Stop
+    gauge run's backward pass runs it (k1 and k2 kept; corrector, stage-2
+    and stage-1 spatial adjoints), on a state after 0.3 s of inflow with a
+    cotangent in every cell.  The timed loop is bracketed by cudaProfilerStart/Stop
     (for `ncu --profile-from-start off`).  A step of the metric is one
     adjoint step."""
     from diffswe2d_b200.adjoint import AdjointStepper
     from diffswe2d_b200.autotune import sweep_rows, tuned_rows_for_shape
+    from diffswe2d_b200.gauge_run import ADJOINT_KERNELS_PER_STEP
     from diffswe2d_b200.inversion import make_runup_problem
     dev = torch.device("cuda", local)
     torch.cuda.set_device(dev)
@@ -800,27 +801,29 @@ def run_adjoint(args, world, rank, local):
     B = args.inv_cases
     with torch.no_grad():
         U, _ = m(problem.U0.clone(), t_end=0.3, boundary_level=torch.tensor(0.02, device=dev))
-    stp = AdjointStepper(m, B, gy, gx, dev, 1)
+    stp = AdjointStepper(m, B, gy, gx, dev, 1, run=True)
     lv = torch.tensor([0.01], device=dev)
     gen = torch.Generator(device="cpu").manual_seed(0)
     lam_out = (torch.randn(U.shape, generator=gen) * 1e-3).to(dev)
     lam_U = torch.zeros_like(U)
     lam_n = torch.zeros_like(stp.n)
     dt = torch.tensor([1e-3], device=dev)
-    K1 = torch.empty_like(U)
+    K1, K2, P = (torch.empty_like(U) for _ in range(3))
     rows = tuned_rows_for_shape(B, gy, gx, dev, arithmetic=args.inv_arithmetic)
     clk = Clocks(local)
     with sweep_rows(rows):
         stp._tendency(U, lv, K1)
+        stp._pointwise(2, U, K1, dt, None, None, None, P)
+        stp._tendency(P, lv, K2)
         for _ in range(max(args.warmup, 1)):
-            stp(U, lv, dt, lam_out, lam_U, lam_n, K1=K1)
+            stp(U, lv, dt, lam_out, lam_U, lam_n, K1=K1, K2=K2, overwrite=True)
         torch.cuda.synchronize(dev)
         e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
         torch.cuda.profiler.start()
         with clk:
             e0.record()
             for _ in range(args.steps):
-                stp(U, lv, dt, lam_out, lam_U, lam_n, K1=K1)
+                stp(U, lv, dt, lam_out, lam_U, lam_n, K1=K1, K2=K2, overwrite=True)
             e1.record()
             torch.cuda.synchronize(dev)
         torch.cuda.profiler.stop()
@@ -832,11 +835,12 @@ def run_adjoint(args, world, rank, local):
         "data": "synthetic",
         "config": {"workload": f"runup_adjoint_{gy}x{gx}", "cases": B, "dx": gdx, "tile_rows": rows,
                    "arithmetic": args.inv_arithmetic,
-                   "per_step": "predictor + k2 re-evaluation, corrector adjoint, stage-2 spatial + "
-                               "predictor adjoint, stage-1 spatial adjoint (k1 kept)"},
+                   "per_step": "corrector adjoint, stage-2 spatial + predictor adjoint, stage-1 "
+                               "spatial adjoint (k1 and k2 kept)"},
         "adjoint_mcell_per_s": B * gy * gx / us,
         "gradient_finite": bool(torch.isfinite(lam_U).all()),
-        "gpu_launches": 7 * args.steps, "clocks": clk.summary(),
+        # those of a run's step without its cursor's two
+        "gpu_launches": (ADJOINT_KERNELS_PER_STEP - 2) * args.steps, "clocks": clk.summary(),
     }
     if rank == 0:
         print(json.dumps(line), flush=True)
