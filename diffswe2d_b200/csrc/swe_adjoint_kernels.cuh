@@ -294,7 +294,7 @@ __host__ __device__ inline long long band_items(const AdjArgs& a) {
 }
 
 // The bands' faces, one per thread.  (In the tile kernel's grid their code
-// cost every tile 8 to 25 %; here 10.5 and 8.4 us at 2 x 244 x 393.)
+// cost every tile 8 to 25 %; here 10.6 and 8.7 us at 2 x 244 x 393.)
 template <bool BEDG, bool PRED, class M>
 __global__ void __launch_bounds__(64) adj_band_kernel(const AdjArgs a) {
     chain_start();
@@ -336,23 +336,28 @@ __device__ __noinline__ void band_sum(const LevelBand& band, bool normal, bool f
     for (int c = 0; c < 4; ++c) l[c] = (((0.0f + v[0][c]) + v[1][c]) + v[2][c]) + v[3][c];
 }
 
-// The same sum with the faces evaluated here: along x of row `line`, or along
-// y of column `line`.
+// The same sum with the faces evaluated here, one by each of four lanes that
+// share a cell (q: this lane's): along x of row `line`, or along y of column
+// `line`.  (A cell's lane evaluating all four takes the edge kernel 74 and 81
+// us in the two stages at 2 x 24 x 30, four lanes 38 and 43; tile sums 6.)
 template <bool BEDG, bool PRED, class M>
 __device__ __noinline__ void face_sum(const AdjArgs& a, int b, bool diry, int line, int pos, int n, float scale,
-                                      float l[4]) {
-#pragma unroll
-    for (int c = 0; c < 4; ++c) l[c] = 0.0f;
-#pragma unroll 1
-    for (int q = 0; q < 4; ++q) {
-        const int f = pos - 1 + q;
-        if (f < 0 || f > n) continue;
+                                      int q, float l[4]) {
+    const int f = pos - 1 + q, lane = threadIdx.x & 31;
+    float v[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+    if (f >= 0 && f <= n) {
         float r[BAND_REC];
         band_face<BEDG, PRED, M>(a, b, diry, f, line, scale, r);
 #pragma unroll
         for (int s = 0; s < 4; ++s)  // (a constant index keeps the record in registers)
             if (s == 3 - q)
-                for (int c = 0; c < 4; ++c) l[c] += r[4 * s + c];
+                for (int c = 0; c < 4; ++c) v[c] = r[4 * s + c];
+    }
+    const unsigned group = 0xfu << (lane & 28);
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+        l[c] = 0.0f;
+        for (int k = 0; k < 4; ++k) l[c] += __shfl_sync(group, v[c], (lane & 28) + k);
     }
 }
 
@@ -893,7 +898,8 @@ __device__ __forceinline__ void frame_cell(int ny, int nx, long long t, int& j, 
 
 // Finishes the frame, a cell per thread.  A few warps run through it once,
 // so its time is that of its instruction fetches and load chains: one copy
-// of each part, no ghost read in vain.  FLY: level bands without records.
+// of each part, no ghost read in vain.  FLY: level bands without records,
+// four lanes per cell.
 template <bool BEDG, bool PRED, bool FLY, class M>
 __global__ void __launch_bounds__(ADJ_THREADS) adj_edge_kernel(const AdjArgs a) {
     chain_start();
@@ -901,7 +907,9 @@ __global__ void __launch_bounds__(ADJ_THREADS) adj_edge_kernel(const AdjArgs a) 
     const size_t plane = (size_t)ny * nx;
     float scale = 0.0f;
     if (PRED) scale = 0.5f * (a.dt_dev != nullptr ? *a.dt_dev : a.dt);
-    const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    const int face = FLY ? (int)(t & 3) : 0;
+    if (FLY) t >>= 2;
     float level = 0.0f;
     if (t < frame_cells(ny, nx)) {
         int j, i;
@@ -925,8 +933,8 @@ __global__ void __launch_bounds__(ADJ_THREADS) adj_edge_kernel(const AdjArgs a) 
             if (BEDG) lz = fr[3 * plane];
         } else {
             if (FLY) {
-                face_sum<BEDG, PRED, M>(a, b, false, j, i, nx, scale, lam);
-                face_sum<BEDG, PRED, M>(a, b, true, i, j, ny, scale, l);
+                face_sum<BEDG, PRED, M>(a, b, false, j, i, nx, scale, face, lam);
+                face_sum<BEDG, PRED, M>(a, b, true, i, j, ny, scale, face, l);
             } else {
                 band_sum(band, bs < 2, far, e, j, i, nx, lam);
                 band_sum(band, bs >= 2, far, e, i, j, ny, l);
@@ -950,7 +958,7 @@ __global__ void __launch_bounds__(ADJ_THREADS) adj_edge_kernel(const AdjArgs a) 
             // a band holds the records of its own side's ghosts and of those
             // at the ends of its two lines
             if (FLY && (level_side(a, side) || (bs >= 0 && (bs < 2) == yax))) {
-                face_sum<BEDG, PRED, M>(a, b, yax, yax ? i : j, g, n, scale, l);
+                face_sum<BEDG, PRED, M>(a, b, yax, yax ? i : j, g, n, scale, face, l);
             } else if (level_side(a, side)) {
                 band_sum(LevelBand(a, b, side), true, (side & 1) != 0, 0, yax ? i : j, g, n, l);
             } else if (bs >= 0 && (bs < 2) == yax) {
@@ -962,9 +970,11 @@ __global__ void __launch_bounds__(ADJ_THREADS) adj_edge_kernel(const AdjArgs a) 
             }
             fold_ghost<BEDG, PRED, M>(a, b, side, g, l, j, i, scale, lam, llev, lz);
         }
-        finish_cell<PRED, M>(a, a3(b, 0, j, i, ny, nx), plane, lam, scale);
-        if (BEDG) a.lbed[(size_t)b * plane + (size_t)j * nx + i] += lz;
-        fr[3 * plane] = level = llev;
+        if (face == 0) {
+            finish_cell<PRED, M>(a, a3(b, 0, j, i, ny, nx), plane, lam, scale);
+            if (BEDG) a.lbed[(size_t)b * plane + (size_t)j * nx + i] += lz;
+            fr[3 * plane] = level = llev;
+        }
     }
     if (a.direct_level) {
         const float sum = block_sum(level);
@@ -1187,6 +1197,7 @@ template <bool BEDG, bool PRED, class M>
 cudaError_t launch_adj_forms(AdjArgs a, cudaStream_t s) {
     const dim3 th(ADJ_THREADS);
     const dim3 ge((unsigned)((frame_cells(a.ny, a.nx) + ADJ_THREADS - 1) / ADJ_THREADS), a.B);
+    const dim3 gf((unsigned)((4 * frame_cells(a.ny, a.nx) + ADJ_THREADS - 1) / ADJ_THREADS), a.B);
     const long long items = band_items(a);
     const bool level = level_side(a, 0) || level_side(a, 1) || level_side(a, 2) || level_side(a, 3);
     cudaError_t e = cudaSuccess;
@@ -1195,7 +1206,7 @@ cudaError_t launch_adj_forms(AdjArgs a, cudaStream_t s) {
     a.direct_level = !level && a.level_blocks >= (int)ge.x;
     if (e == cudaSuccess) e = launch_tiles<BEDG, PRED, M, 16>(a, s);
     if (e == cudaSuccess)
-        e = level && items == 0 ? launch_chained(adj_edge_kernel<BEDG, PRED, true, M>, ge, th, s, a)
+        e = level && items == 0 ? launch_chained(adj_edge_kernel<BEDG, PRED, true, M>, gf, th, s, a)
                                 : launch_chained(adj_edge_kernel<BEDG, PRED, false, M>, ge, th, s, a);
     if (e == cudaSuccess && !a.direct_level)
         e = launch_chained(adj_level_kernel, dim3(a.level_blocks, a.B), th, s, a.frame, a.llevel_part, a.ny, a.nx);
