@@ -52,6 +52,11 @@ constexpr unsigned long long DRAIN_LIMIT_NS = 2000000000ull;  // 2 s
 // tiles, four of the widest.
 constexpr int SMEM_ALIGN = 1024;
 constexpr int SMEM_MAX = STAGES_MAX * (tile_bytes(BM) + tile_bytes(64));
+// At least a quarter of an SM's shared memory (228 KB), so that no more than
+// three CTAs of a launch share an SM whatever their registers allow: their
+// allocations (at most 128 of its 512 tensor-memory columns each) never wait.
+constexpr int SMEM_MIN = 57 * 1024;
+static_assert(4 * SMEM_MIN >= 228 * 1024 && 3 * BN_MAX <= 512, "");
 static_assert(SMEM_MAX + SMEM_ALIGN + 1024 <= 227 * 1024 && 4 * (tile_bytes(BM) + tile_bytes(BN_MAX)) <= SMEM_MAX, "");
 
 // A GEMM operand in memory: lines of `cols` contiguous elements.  K-major: a
@@ -826,7 +831,7 @@ int launch_gemm(GemmArgs g, int ksplit, float* workspace, cudaStream_t s) {
     g.stages = 1;  // a power of two, no more than the K blocks need
     while (g.stages < per && g.stages < (bn == BN_MAX ? 4 : STAGES_MAX)) g.stages *= 2;
     const dim3 grid((g.M + BM - 1) / BM, (g.N + bn - 1) / bn, zs);
-    gemm_kernel<A_MN, B_MN><<<grid, NT, g.stages * stage + SMEM_ALIGN, s>>>(g);
+    gemm_kernel<A_MN, B_MN><<<grid, NT, std::max(g.stages * stage + SMEM_ALIGN, SMEM_MIN), s>>>(g);
     if (zs > 1) splitk_epilogue_kernel<<<grid_for((long long)g.M * g.N, 256), 256, 0, s>>>(g, zs);
     return cudaGetLastError() == cudaSuccess ? SWE_OK : SWE_ECUDA;
 }
