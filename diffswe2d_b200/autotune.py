@@ -1,14 +1,18 @@
 """Autotuner for the step kernels' launch shape.
 
-Two knobs are tuned by timing them on the GPU in use:
+Tuned by timing on the GPU in use:
 
 * the sweep tile height (output rows per warp strip) per grid-size class --
   taller tiles recompute fewer halo rows, shorter ones give more tiles to
   fill the 148 SMs on small grids and a shorter serial chain per warp; used
-  by the single-grid kernels (``swe_tune_sweep_rows``); one throughput-tuned
-  value for the persistent ensemble kernel (``tuned_ensemble_rows``); and per
-  exact (batch, ny, nx) shape for the captured time loops of gauge runs and
-  ``SWE2D.forward`` (``tuned_rows_for_shape``);
+  by the single-grid kernels (``swe_tune_sweep_rows``, through ``apply``);
+  and per exact (batch, ny, nx) shape for the captured time loops of gauge
+  runs and ``SWE2D.forward`` (``tuned_rows_for_shape``).  Nothing is timed
+  where the steps are not swept (IEEE grids up to 1.5 million cells take
+  shared-memory tiles); untuned launches choose by a rule of their own.  One
+  value for the persistent ensemble kernel is timed too
+  (``tuned_ensemble_rows``); ensembles take it only as their ``rows``
+  argument, else ``ensemble_rows`` of their members;
 * the number of steps per CUDA-graph replay of ``SWE2D.forward``'s device
   loop -- more steps per replay mean fewer host reads, more no-op steps at
   the end of a call;

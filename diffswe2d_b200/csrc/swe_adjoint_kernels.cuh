@@ -14,8 +14,8 @@
 // add_ghost_cells, src/boundary.py:150-413) and finishes the two-cell frame
 // along the sides; adj_level_kernel sums the level's adjoint.  Stage 2 goes on through the predictor's adjoint in both.
 // No float atomics: results are deterministic.  On request the ghosts that
-// depend on the level are done face by face instead (level bands, below),
-// in two more launches.
+// depend on the level and the cells next to them are done face by face
+// instead (level bands, below), in two more launches.
 #pragma once
 
 #include <cuda_runtime.h>

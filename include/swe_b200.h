@@ -376,9 +376,10 @@ int swe_adj_stage2_f32(const float* P, const float* U, const float* k1, const fl
  * The two calls above for the steps of a long run: the stage-2 form makes P
  * from U and k1 itself (as mode 2 of swe_adj_pointwise_f32 does), and the
  * ghosts that depend on the level are not done face by face.  (The calls
- * above evaluate them in autograd's own order of operations, because one
- * step's level adjoint is a sum of both signs over a side and may nearly
- * cancel; that costs two more launches.)  lam_bed may be null.
+ * above evaluate them, and the two lines of cells next to them, in autograd's
+ * own order of operations, because one step's level adjoint is a sum of both
+ * signs over a side and may nearly cancel; that costs two more launches.)
+ * lam_bed may be null.
  */
 int swe_adj_spatial_run_f32(const float* S, const float* bed, int bedB, int B, int ny, int nx,
                             const swe_params* p, const float* level, int levelB,
