@@ -278,7 +278,7 @@ class _ChunkFunction(torch.autograd.Function):
         lam_n = torch.zeros_like(n) if model.cfg.apply_friction else None
         B, _, ny, nx = U0.shape
         ws = AdjointStepper(model, B, ny, nx, U0.device, model._level_arg(level_vec, B)[1],
-                            bed_grad=need_bed, run=True)
+                            bed_grad=need_bed, run=len(states) > 1)  # a chunk of one step is a single step
         lv = model._level_arg(level_vec.detach(), B)[0]
         for U_s, dt_s in zip(reversed(states), reversed(dts)):
             lam_out, lam = lam, torch.zeros_like(lam)

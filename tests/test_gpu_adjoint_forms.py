@@ -161,3 +161,23 @@ def test_forward_with_a_level_per_member(arithmetic):
         W, hm = m(U, t_end=1.5, boundary_level=level, callback=lambda *a: None)
     assert steps == m.last_forward_steps and steps > 3
     assert torch.equal(V, W) and torch.equal(hmax, hm)
+
+
+@pytest.mark.parametrize("ny,nx", [(20, 25), (50, 67)])
+def test_a_chunk_of_one_step_is_a_single_step(ny, nx):
+    """forward_checkpointed over one step gives the gradients of step(), the
+    level's included, bit for bit."""
+    from diffswe2d_b200.adjoint import forward_checkpointed
+    m, U, lam, level = _problem(8, ny, nx, "level")
+    grads = []
+    for chunk in (False, True):
+        V, lv = U.clone().requires_grad_(True), level.clone().requires_grad_(True)
+        if chunk:
+            W = forward_checkpointed(m, V, 1e-3, boundary_level=lv)
+            assert m.last_forward_steps == 1
+        else:
+            W, dt = m.step(V, 0.0, 1e-3, boundary_level=lv)
+        (W * lam).sum().backward()
+        grads.append((W.detach(), V.grad, lv.grad))
+    for a, b in zip(*grads):
+        assert torch.equal(a, b)
